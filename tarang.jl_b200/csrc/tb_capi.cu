@@ -141,74 +141,16 @@ std::vector<double2> pass_twiddles(const FftPlan& fp) {
   return t;
 }
 
-// In-place (DIF/DIT) twiddles: per pass s, exp(-2 pi i j / L_s) for j < L_s / R_s,
-// L_s = n / (R_0 ... R_{s-1}) (the layout fftg::fft_ip_dif / fft_ip_dit read)
-std::vector<double2> ip_twiddles(const FftPlan& fp) {
-  std::vector<double2> t;
-  const long double pi = 3.141592653589793238462643383279502884L;
-  int L = fp.n;
-  for (int s = 0; s < fp.nstages; ++s) {
-    const int m = L / fp.radix[s];
-    for (int j = 0; j < m; ++j) {
-      const long double a = -2.0L * pi * (long double)j / (long double)L;
-      t.push_back(make_double2((double)cosl(a), (double)sinl(a)));
-    }
-    L = m;
+// The in-place plan's twiddles (rplan_twiddles) as complex entries of type C.
+template <class C>
+std::vector<C> rplan_table(const RPlan& rp) {
+  const std::vector<double> w = rplan_twiddles(rp);
+  std::vector<C> t(w.size() / 2);
+  for (size_t i = 0; i < t.size(); ++i) {
+    t[i].x = (decltype(t[i].x))w[2 * i];
+    t[i].y = (decltype(t[i].y))w[2 * i + 1];
   }
   return t;
-}
-
-// Shared-memory wavefronts of the in-place passes of plan fp (fftg::pass_ip:
-// item = thread + k * blockDim over NA arrays Ms = n apart, a warp = 32
-// consecutive items, lane element base + r m at the XOR-swizzled index
-// fidx), summed over the DIF inverse (4 arrays) and DIT forward (2 arrays)
-// transforms of the x-products kernel.  Elements of esz bytes: 16 (double2,
-// four 8-lane phases over 8 bank quads) or 8 (float2, two 16-lane phases
-// over 16 bank pairs); a phase costs as many wavefronts as the most distinct
-// addresses on one bank group.
-long long ip_wavefronts(const FftPlan& fp, int esz) {
-  const int n = fp.n, lanes = esz == 16 ? 8 : 16, banks = esz == 16 ? 8 : 16;
-  auto swz = [](int i) { return i ^ ((i >> 3) & 7); };
-  long long wf = 0;
-  for (int t = 0; t < 2; ++t) {
-    const int NA = t == 0 ? 4 : 2;
-    int L = n;
-    for (int s = 0; s < fp.nstages; ++s) {
-      const int R = fp.radix[s], m = L / R, nb = n / R, total = NA * nb;
-      for (int w0 = 0; w0 < total; w0 += 32)
-        for (int r = 0; r < R; ++r)
-          for (int ph = w0; ph < w0 + 32 && ph < total; ph += lanes) {
-            std::vector<std::vector<int>> grp(banks);
-            int worst = 0;
-            for (int item = ph; item < ph + lanes && item < total; ++item) {
-              const int arr = item / nb, b = item - arr * nb, base = (b / m) * L + b % m;
-              const int addr = arr * n + swz(base + r * m);
-              auto& g = grp[addr % banks];
-              if (std::find(g.begin(), g.end(), addr) == g.end()) g.push_back(addr);
-              worst = std::max(worst, (int)g.size());
-            }
-            wf += worst;
-          }
-      L = m;
-    }
-  }
-  return wf;
-}
-
-// The order of fp's passes with the fewest in-place wavefronts (ties keep the
-// earlier order in lexicographic sequence, starting from fp's own).
-FftPlan best_ip_order(const FftPlan& fp, int esz) {
-  FftPlan best = fp, cand = fp;
-  long long bw = ip_wavefronts(fp, esz);
-  std::sort(cand.radix, cand.radix + cand.nstages);
-  do {
-    const long long w = ip_wavefronts(cand, esz);
-    if (w < bw) {
-      bw = w;
-      best = cand;
-    }
-  } while (std::next_permutation(cand.radix, cand.radix + cand.nstages));
-  return best;
 }
 
 std::vector<double2> twiddles(int n) {
@@ -412,7 +354,8 @@ void enqueue_rhs_mixed(tb_plan* P, const double2* Xin, double2* out3, bool c2row
   }
   xa.ptw = P->ptwM32.as<float2>();
   xa.nptw = (int)(P->ptwM32.bytes / sizeof(float2));
-  xa.fp = P->xrows == 3 ? P->fpMip : P->fpM;  // the in-place kernels run their own pass order
+  xa.fp = P->fpM;
+  xa.rp = P->rpM;  // the in-place form's own passes
   xa.Nx = P->Nx;
   xa.Nk = P->Nkm;
   xa.ld = P->Nk;
@@ -421,10 +364,9 @@ void enqueue_rhs_mixed(tb_plan* P, const double2* Xin, double2* out3, bool c2row
   xa.Nz = N;
   xa.k0 = (float)P->k0;
   xa.iptw = P->iptwM32.as<float2>();
-  xa.niptw = (int)(P->iptwM32.bytes / sizeof(float2));
   timed(P, "x_fft_products", [&] {
     if (P->xrows == 3)
-      launch_xprod32_ip(xa, P->st);  // transforms in place (DIF / DIT)
+      launch_xprod32_r(xa, P->st);  // transforms in place (DIF / DIT)
     else if (P->xrows == 2)
       launch_xprod32_b(xa, P->st);  // transforms batched through shared passes
     else
@@ -486,7 +428,8 @@ void enqueue_rhs(tb_plan* P, const double2* Xin, double2* out3, bool c2rows, boo
   }
   xa.ptw = P->ptwM.as<double2>();
   xa.nptw = (int)(P->ptwM.bytes / sizeof(double2));
-  xa.fp = P->xrows == 3 ? P->fpMip : P->fpM;  // the in-place kernels run their own pass order
+  xa.fp = P->fpM;
+  xa.rp = P->rpM;  // the in-place form's own passes
   xa.Nx = P->Nx;
   xa.Nk = P->Nkm;
   xa.ld = P->Nk;
@@ -495,10 +438,9 @@ void enqueue_rhs(tb_plan* P, const double2* Xin, double2* out3, bool c2rows, boo
   xa.Nz = N;
   xa.k0 = P->k0;
   xa.iptw = P->iptwM.as<double2>();
-  xa.niptw = (int)(P->iptwM.bytes / sizeof(double2));
   timed(P, "x_fft_products", [&] {
     if (P->xrows == 3)
-      launch_xprod_ip(xa, P->st);  // transforms in place (DIF / DIT)
+      launch_xprod_r(xa, P->st);  // transforms in place (DIF / DIT)
     else if (P->xrows == 2)
       launch_xprod_b(xa, P->st);  // transforms batched through shared passes
     else
@@ -852,9 +794,9 @@ static bool xprod2d_form_fits(const tb_plan* P, int form) {
   if (form == 1) return true;
   if (P->mixed)
     return form == 2 ? xprod32_b_fits(P->M, (int)(P->ptwM32.bytes / sizeof(float2)))
-                     : xprod32_ip_fits(P->M, (int)(P->iptwM32.bytes / sizeof(float2)));
+                     : xprod32_r_fits(P->rpM);
   return form == 2 ? xprod_b_fits(P->M, (int)(P->ptwM.bytes / sizeof(double2)))
-                   : xprod_ip_fits(P->M, (int)(P->iptwM.bytes / sizeof(double2)));
+                   : xprod_r_fits(P->rpM);
 }
 
 bool tb::plan_tau_parts_ok(const tb_plan* P, int parts) {
@@ -1268,8 +1210,8 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
     upload(P->twM, twiddles(P->M));
     upload(P->ptwM, pass_twiddles(P->fpM));
     P->mixed = desc->precision == TB_PREC_MIXED;
-    P->fpMip = best_ip_order(P->fpM, P->mixed ? 8 : 16);
-    upload(P->iptwM, ip_twiddles(P->fpMip));
+    TB_REQUIRE(make_rplan(P->M, P->mixed ? 8 : 16, &P->rpM), TB_ENOTSUPPORTED, "Nx must be of the form 2^a 3^b");
+    if (!P->mixed) upload(P->iptwM, rplan_table<double2>(P->rpM));
     upload(P->twN, twiddles(P->Nx));
     if (P->mixed) {
       auto f32 = [](const std::vector<double>& v) {
@@ -1289,10 +1231,7 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
       std::vector<float2> pt32(pt.size());
       for (size_t i = 0; i < pt.size(); ++i) pt32[i] = make_float2((float)pt[i].x, (float)pt[i].y);
       upload(P->ptwM32, pt32);
-      const std::vector<double2> it = ip_twiddles(P->fpMip);
-      std::vector<float2> it32(it.size());
-      for (size_t i = 0; i < it.size(); ++i) it32[i] = make_float2((float)it[i].x, (float)it[i].y);
-      upload(P->iptwM32, it32);
+      upload(P->iptwM32, rplan_table<float2>(P->rpM));
       TB_REQUIRE(xprod32_smem_bytes(P->M, (int)pt32.size()) <= 227 * 1024, TB_ENOTSUPPORTED,
                  "Nx too large for the FP32 x kernel");
       // TF32 operand images of the eight transform matrices for the 2D

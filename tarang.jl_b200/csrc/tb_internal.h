@@ -130,4 +130,18 @@ struct FftPlan {
 };
 bool make_fft_plan(int n, FftPlan* out);
 
+// Plan of the in-place passes of tb_fftr.cuh: radices R[s] (at most 16, the last
+// at most 8), butterfly strides m[s], magic divisors of m[s] (dm) and of the
+// butterfly count n / R[s] (db), twiddle offsets of the passes in the table.
+struct RPlan {
+  static constexpr int kMax = 12;
+  int n = 0, np = 0, ntw = 0;
+  int R[kMax], m[kMax], tw[kMax];
+  unsigned dm[kMax], db[kMax];
+};
+// n = 2^a 3^b; element_bytes 8 (float2) or 16 (double2) selects the bank model.
+bool make_rplan(int n, int element_bytes, RPlan* out);
+// Twiddles of the plan's passes, (cos, sin) pairs, in the layout the passes read.
+std::vector<double> rplan_twiddles(const RPlan& p);
+
 }  // namespace tb

@@ -15,6 +15,7 @@
 // by the pin tau_p = 0, which leaves every other unknown unchanged.
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <tuple>
 
 #include "tb_internal.h"
@@ -405,6 +406,98 @@ bool make_fft_plan(int n, FftPlan* out) {
   p.nstages = ns;
   *out = p;
   return true;
+}
+
+namespace {
+
+// Shared-memory wavefronts per access of one in-place pass: the lanes of a
+// phase (8 of 16 bytes, 16 of 8 bytes) read entry r of consecutive butterflies
+// (block L, stride m = L / R) at the XOR-swizzled index; a phase takes as many
+// wavefronts as the most distinct entries on one bank group.  The pattern
+// repeats, so the first blocks stand for all.
+double pass_wavefronts(int n, int L, int R, int lanes) {
+  const int m = L / R, nb = n / R, shift = lanes == 8 ? 3 : 4;
+  const int phases = std::min((nb + lanes - 1) / lanes, 24);
+  int waves = 0;
+  for (int ph = 0; ph < phases; ++ph)
+    for (int r = 0; r < R; ++r) {
+      int count[16] = {0}, worst = 1;
+      for (int b = ph * lanes; b < std::min((ph + 1) * lanes, nb); ++b) {
+        const int i = (b / m) * L + b % m + r * m;
+        worst = std::max(worst, ++count[(i ^ (i >> shift)) & (lanes - 1)]);
+      }
+      waves += worst;
+    }
+  return (double)waves / (phases * R);
+}
+
+}  // namespace
+
+bool make_rplan(int n, int element_bytes, RPlan* out) {
+  int rest = n;
+  while (rest % 2 == 0) rest /= 2;
+  while (rest % 3 == 0) rest /= 3;
+  if (n < 2 || rest != 1) return false;
+  const int lanes = element_bytes == 16 ? 8 : 16;
+  // a pass costs its wavefronts (one read and one write of the array) plus
+  // about 45 for its barrier and latency (measured between 192 and 1536 points)
+  const double per_pass = 45.0;
+  const int radices[] = {16, 12, 9, 8, 6, 4, 3, 2};
+  std::map<std::pair<int, int>, double> memo;
+  std::vector<int> seq, best;
+  double best_cost = 1e300;
+  std::function<void(int, double)> search = [&](int L, double cost) {
+    if (cost >= best_cost) return;
+    if (L == 1) {
+      best_cost = cost;
+      best = seq;
+      return;
+    }
+    for (int R : radices) {
+      if (L % R || (L == R && (R > 8))) continue;  // the last pass runs fused, in registers: at most 8
+      auto it = memo.find({L, R});
+      if (it == memo.end()) it = memo.emplace(std::make_pair(L, R), pass_wavefronts(n, L, R, lanes)).first;
+      seq.push_back(R);
+      if ((int)seq.size() < RPlan::kMax) search(L / R, cost + 2.0 * n / lanes * it->second + per_pass);
+      seq.pop_back();
+    }
+  };
+  search(n, 0.0);
+  if (best.empty()) return false;
+  auto magic = [](int d) { return d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); };
+  RPlan p;
+  p.n = n;
+  p.np = (int)best.size();
+  int L = n, off = 0;
+  for (int s = 0; s < p.np; ++s) {
+    p.R[s] = best[s];
+    p.m[s] = L / best[s];
+    p.dm[s] = magic(p.m[s]);
+    p.db[s] = magic(n / best[s]);
+    p.tw[s] = off;
+    if (p.m[s] > 1) off += p.m[s] * (best[s] > 8 ? 2 : 1);
+    L = p.m[s];
+  }
+  p.ntw = off;
+  *out = p;
+  return true;
+}
+
+std::vector<double> rplan_twiddles(const RPlan& p) {
+  std::vector<double> t;
+  t.reserve(2 * (size_t)p.ntw);
+  const long double pi = 3.141592653589793238462643383279502884L;
+  for (int s = 0; s < p.np; ++s) {
+    const int m = p.m[s], L = m * p.R[s];
+    if (m == 1) continue;
+    for (int e = 1; e <= (p.R[s] > 8 ? 4 : 1); e += 3)
+      for (int j = 0; j < m; ++j) {
+        const long double a = -2.0L * pi * (long double)(e * j) / (long double)L;
+        t.push_back((double)cosl(a));
+        t.push_back((double)sinl(a));
+      }
+  }
+  return t;
 }
 
 }  // namespace tb

@@ -146,6 +146,7 @@ struct tb_plan {
   using TauLayout = tb::TauLayout;
   using TauSystem = tb::TauSystem;
   using FftPlan = tb::FftPlan;
+  using RPlan = tb::RPlan;
   tb_context* ctx = nullptr;
   tb_problem_desc d{};
   int Nx = 0, Nz = 0, Nk = 0, M = 0;
@@ -189,9 +190,7 @@ struct tb_plan {
   DevBuf bEv, bOv, bEd, bOd, fE, fO, sfE, sfO;
   int Hz = 0, Ke = 0, Ko = 0;  // Hz = ceil(Nz/2)
   FftPlan fpM{}, fpN{};
-  // the padded length's passes in the order of the in-place x-products kernels
-  // (x-products form 3; the order with the fewest shared-memory bank conflicts)
-  FftPlan fpMip{};
+  RPlan rpM{};  // the padded length's in-place passes (x-products form 3)
   // tau systems
   TauSystem sys[2];
   int nsys = 1;

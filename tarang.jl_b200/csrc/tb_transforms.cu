@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "tb_fft.cuh"
+#include "tb_fftr.cuh"
 #include "tb_kernels.cuh"
 
 namespace tb {
@@ -905,12 +906,7 @@ cudaError_t set_transform_smem_limits(int bytes) {
     return e;
   if ((e = cudaFuncSetAttribute(k_xprod_b<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess)
     return e;
-  if ((e = cudaFuncSetAttribute(fftg::k_xprod_ip<256, double2, XProdArgs>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                bytes)) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(fftg::k_xprod_ip<512, double2, XProdArgs>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                bytes)) != cudaSuccess)
-    return e;
+  if ((e = fftr::xprod_r_set_limits<double2, XProdArgs>(bytes)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(k_x_rfft, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(k_x_irfft, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_x_dealias_mul, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -934,16 +930,9 @@ size_t xprod_b_smem_bytes(int M, int nptw) {
 
 bool xprod_b_fits(int M, int nptw) { return xprod_b_smem_bytes(M, nptw) <= 227 * 1024; }
 
-bool xprod_ip_fits(int M, int niptw) { return fftg::xprod_ip_smem_bytes<double2>(M, niptw) <= 227 * 1024; }
+bool xprod_r_fits(const RPlan& rp) { return fftr::xprod_r_smem_bytes<double2>(rp.n, rp.ntw) <= 227 * 1024; }
 
-void launch_xprod_ip(const XProdArgs& a, cudaStream_t st) {
-  const size_t smem = fftg::xprod_ip_smem_bytes<double2>(a.M, a.niptw);
-  const dim3 grid(a.Nz, a.instances > 0 ? a.instances : 1);
-  if (2 * smem <= 227 * 1024)  // two CTAs of 256 threads per SM while both fit
-    fftg::k_xprod_ip<256, double2, XProdArgs><<<grid, 256, smem, st>>>(a);
-  else
-    fftg::k_xprod_ip<512, double2, XProdArgs><<<grid, 512, smem, st>>>(a);
-}
+void launch_xprod_r(const XProdArgs& a, cudaStream_t st) { fftr::launch_xprod_r_t<double2>(a, st); }
 
 void launch_xprod_b(const XProdArgs& a, cudaStream_t st) {
   const size_t smem = xprod_b_smem_bytes(a.M, a.nptw);

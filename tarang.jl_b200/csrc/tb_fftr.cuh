@@ -370,15 +370,13 @@ inline size_t xprod_r_smem_bytes(int M, int ntw) {
   return (4 * (size_t)rpad<C>(M) + (size_t)ntw) * sizeof(C);
 }
 
-// 128 threads up to 384 points (a pass has at most a few butterflies a
-// thread), 256 above while two CTAs share an SM, else one CTA of 512.
+// 256 threads while two CTAs share an SM (128 threads measured 1 to 2 us slower
+// from 384 points on and no faster below), else one CTA of 512.
 template <class C, class Args>
 inline void launch_xprod_r_t(const Args& a, cudaStream_t st) {
   const size_t smem = xprod_r_smem_bytes<C>(a.M, a.rp.ntw);
   const dim3 grid(a.Nz, a.instances > 0 ? a.instances : 1);
-  if (a.M <= 384)
-    k_xprod_r<128, 4, C, Args><<<grid, 128, smem, st>>>(a);
-  else if (2 * smem <= 227 * 1024)
+  if (2 * smem <= 227 * 1024)
     k_xprod_r<256, 2, C, Args><<<grid, 256, smem, st>>>(a);
   else
     k_xprod_r<512, 1, C, Args><<<grid, 512, smem, st>>>(a);
@@ -386,9 +384,7 @@ inline void launch_xprod_r_t(const Args& a, cudaStream_t st) {
 
 template <class C, class Args>
 inline cudaError_t xprod_r_set_limits(int bytes) {
-  cudaError_t e = cudaFuncSetAttribute(k_xprod_r<128, 4, C, Args>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_xprod_r<256, 2, C, Args>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaError_t e = cudaFuncSetAttribute(k_xprod_r<256, 2, C, Args>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_xprod_r<512, 1, C, Args>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }

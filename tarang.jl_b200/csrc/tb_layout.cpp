@@ -439,9 +439,13 @@ bool make_rplan(int n, int element_bytes, RPlan* out) {
   while (rest % 3 == 0) rest /= 3;
   if (n < 2 || rest != 1) return false;
   const int lanes = element_bytes == 16 ? 8 : 16;
-  // a pass costs its wavefronts (one read and one write of the array) plus
-  // about 45 for its barrier and latency (measured between 192 and 1536 points)
-  const double per_pass = 45.0;
+  // A pass costs its wavefronts (one read and one write of the array) plus its
+  // barrier and the serial chain of a butterfly, which grows with the radix.
+  // The charge decides between equal pass counts: balanced radices win
+  // (event-timed FP64 rows: 192 points 6, 4, 8 9.6 us against 12, 8, 2 10.7;
+  // 1152 points 12, 12, 8 18.9 against 16, 9, 8 20.1), while 1536 points stay
+  // at three passes (16, 12, 8 23.0 us, the best four-pass order 25.0).
+  auto per_pass = [](int R) { return 25.0 + 4.0 * R; };
   const int radices[] = {16, 12, 9, 8, 6, 4, 3, 2};
   std::map<std::pair<int, int>, double> memo;
   std::vector<int> seq, best;
@@ -458,7 +462,7 @@ bool make_rplan(int n, int element_bytes, RPlan* out) {
       auto it = memo.find({L, R});
       if (it == memo.end()) it = memo.emplace(std::make_pair(L, R), pass_wavefronts(n, L, R, lanes)).first;
       seq.push_back(R);
-      if ((int)seq.size() < RPlan::kMax) search(L / R, cost + 2.0 * n / lanes * it->second + per_pass);
+      if ((int)seq.size() < RPlan::kMax) search(L / R, cost + 2.0 * n / lanes * it->second + per_pass(R));
       seq.pop_back();
     }
   };

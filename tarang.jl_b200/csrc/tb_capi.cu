@@ -971,6 +971,28 @@ void pad_band(ClassLayout& L) {
   L.ku = kTauKU;
 }
 
+// Partitions of the tau solve of a new plan, by the number of 4-mode groups and
+// the (padded) band rows; tb_plan_tune may choose another.
+//   From 2 groups per SM on, one warp per group: the groups alone fill the GPU
+//   and the partitions' response records only add bytes (RK222 steps, one warp
+//   against 4 partitions: 64x64x32, 528 groups, 431 against 531 us; 48x48x24,
+//   300 groups, 279 against 341 us); short systems already from one group per
+//   SM on (1536x48, 193 groups, 162 against 168 us).
+//   Below, the sequential sweeps bound the solve and are cut into partitions:
+//   eight (1024x256: 496, 348, 332, 338 us at 1, 4, 8, 16 partitions), four on
+//   systems of fewer than 144 rows (512x48: 94.5 against 95.0 us), and 16,
+//   which keep y in global scratch, where eight do not fit shared memory
+//   (1536x384: 926 against 1059 us with one warp, 192x384: 283 against 545).
+int default_tau_parts(int groups, int npad) {
+  auto fits = [&](int parts) {
+    return npad / kBwdWin >= parts && tau_solve_smem_bytes(npad, parts) <= 227 * 1024;
+  };
+  if (groups >= 2 * 148 || (groups > 148 && npad < 144)) return 1;
+  if (npad >= 144 && fits(kTauParts8)) return kTauParts8;
+  if (fits(kTauParts)) return kTauParts;
+  return fits(kTauParts16) ? kTauParts16 : 1;
+}
+
 void install_system(tb_plan* P, int sy, TauLayout lay) {
   TauSystem& S = P->sys[sy];
   auto to_int = [](long long v) {
@@ -1004,10 +1026,7 @@ void install_system(tb_plan* P, int sy, TauLayout lay) {
   TB_REQUIRE(lay.cls[0].n == lay.cls[1].n, TB_ENOTSUPPORTED, "parity classes of unequal size");
   const int n = lay.cls[0].n;
   S.npad = (n + kTauRowPad - 1) / kTauRowPad * kTauRowPad;
-  // partitioned solve (kTauParts warps per mode group) when its shared memory
-  // fits and the modes alone do not fill the GPU, else one warp per group
-  const bool many_groups = (P->Nk + kSolveModes - 1) / kSolveModes >= 4 * 148;
-  S.tau_parts = (!many_groups && tau_solve_smem_bytes(S.npad, kTauParts) <= 227 * 1024) ? kTauParts : 1;
+  S.tau_parts = default_tau_parts((P->Nk + kSolveModes - 1) / kSolveModes, S.npad);
   TB_REQUIRE(tau_solve_smem_bytes(S.npad, S.tau_parts) <= 227 * 1024, TB_ENOTSUPPORTED,
              "Nz too large for the staged tau solve");
   const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, S.tau_parts) * sizeof(double);
@@ -1297,6 +1316,10 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
     P->tau.p = static_cast<char*>(P->X.p) + P->nplanes * pb;
     P->tau.bytes = (size_t)P->ntau * P->Nk * sizeof(double2);
     if (!d3) {
+      // the x-products in place (event-timed at 1024x256 23.1 us against 35.2
+      // one transform after another and 34.9 batched, at 128x32 10.4 against
+      // 16.8 and 10.5); form 1 where four arrays do not fit
+      P->xrows = xprod2d_form_fits(P, 3) ? 3 : 1;
       P->G.alloc(12 * (size_t)((P->Nz + 1) / 2) * P->Nk * sizeof(double2));
       P->H.alloc(3 * pb);
       if (P->mixed) {
@@ -1610,8 +1633,8 @@ tb_status tb_plan_tune(tb_plan* P, double dt, int trial_steps, int* tau_parts, i
       for (int r : {1, 2, 4})
         if (rbc3d_xrows_ok(P, r)) rows_c.push_back(r);
     } else {
-      for (int form : {1, 2, 3})  // per field, batched, batched in place
-        if (xprod2d_form_fits(P, form)) rows_c.push_back(form);
+      // the in-place form wherever it fits: it measured fastest at every size
+      rows_c.push_back(xprod2d_form_fits(P, 3) ? 3 : 1);
     }
     float best = 1e30f;
     int bp = P->sys[0].tau_parts, br = P->xrows;

@@ -1229,7 +1229,7 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
     upload(P->twM, twiddles(P->M));
     upload(P->ptwM, pass_twiddles(P->fpM));
     P->mixed = desc->precision == TB_PREC_MIXED;
-    TB_REQUIRE(make_rplan(P->M, P->mixed ? 8 : 16, &P->rpM), TB_ENOTSUPPORTED, "Nx must be of the form 2^a 3^b");
+    TB_REQUIRE(make_rplan(P->M, P->mixed ? 8 : 16, &P->rpM, 6), TB_ENOTSUPPORTED, "Nx must be of the form 2^a 3^b");
     if (!P->mixed) upload(P->iptwM, rplan_table<double2>(P->rpM));
     upload(P->twN, twiddles(P->Nx));
     if (P->mixed) {

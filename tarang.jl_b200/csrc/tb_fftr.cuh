@@ -48,6 +48,12 @@ __host__ __device__ constexpr int rpad(int n) {
   return (n + 15) & ~15;
 }
 
+// Products that are rounded on their own: without them the compiler may fuse a
+// product into either of two sums, so that two instantiations of a kernel (rows
+// a block) would round differently.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
 __device__ __forceinline__ int fdiv(int x, unsigned magic) { return magic ? (int)__umulhi((unsigned)x, magic) : x; }
 
 // v * exp(SIGN 2 pi i E / N), N in {6, 9, 12, 16}, 0 <= E < N

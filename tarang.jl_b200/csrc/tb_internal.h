@@ -139,9 +139,13 @@ struct RPlan {
   int R[kMax], m[kMax], tw[kMax];
   unsigned dm[kMax], db[kMax];
 };
-// n = 2^a 3^b; element_bytes 8 (float2) or 16 (double2) selects the bank model.
-bool make_rplan(int n, int element_bytes, RPlan* out);
+// n = 2^a 3^b; element_bytes 8 (float2) or 16 (double2) selects the bank model;
+// arrays that share a block's passes; last: the largest radix of the last pass.
+bool make_rplan(int n, int element_bytes, RPlan* out, int arrays, int last = 8);
 // Twiddles of the plan's passes, (cos, sin) pairs, in the layout the passes read.
 std::vector<double> rplan_twiddles(const RPlan& p);
+// Position of output i after the dif passes: i = d_0 + R_0 (d_1 + R_1 (...)) is
+// left at sum_s d_s m_s.
+std::vector<unsigned short> rplan_positions(const RPlan& p);
 
 }  // namespace tb

@@ -433,19 +433,20 @@ double pass_wavefronts(int n, int L, int R, int lanes) {
 
 }  // namespace
 
-bool make_rplan(int n, int element_bytes, RPlan* out) {
+bool make_rplan(int n, int element_bytes, RPlan* out, int arrays, int last) {
   int rest = n;
   while (rest % 2 == 0) rest /= 2;
   while (rest % 3 == 0) rest /= 3;
   if (n < 2 || rest != 1) return false;
   const int lanes = element_bytes == 16 ? 8 : 16;
-  // A pass costs its wavefronts (one read and one write of the array) plus its
-  // barrier and the serial chain of a butterfly, which grows with the radix.
-  // The charge decides between equal pass counts: balanced radices win
-  // (event-timed FP64 rows: 192 points 6, 4, 8 9.6 us against 12, 8, 2 10.7;
-  // 1152 points 12, 12, 8 18.9 against 16, 9, 8 20.1), while 1536 points stay
-  // at three passes (16, 12, 8 23.0 us, the best four-pass order 25.0).
-  auto per_pass = [](int R) { return 25.0 + 4.0 * R; };
+  // A pass costs the wavefronts of its arrays (one read and one write each) plus
+  // its barrier and the serial chain of a butterfly, which grows with the
+  // radix.  The charge decides between equal pass counts: balanced radices win
+  // (event-timed FP64 rows of six arrays: 192 points 6, 4, 8 9.6 us against 12,
+  // 8, 2 10.7; 1152 points 12, 12, 8 18.9 against 16, 9, 8 20.1), while 1536
+  // points stay at three passes (16, 12, 8 23.0 us, the best four-pass order
+  // 25.0).
+  auto per_pass = [](int R) { return 150.0 + 24.0 * R; };
   const int radices[] = {16, 12, 9, 8, 6, 4, 3, 2};
   std::map<std::pair<int, int>, double> memo;
   std::vector<int> seq, best;
@@ -458,11 +459,11 @@ bool make_rplan(int n, int element_bytes, RPlan* out) {
       return;
     }
     for (int R : radices) {
-      if (L % R || (L == R && (R > 8))) continue;  // the last pass runs fused, in registers: at most 8
+      if (L % R || (L == R && R > last)) continue;  // the last pass may run fused with a product
       auto it = memo.find({L, R});
       if (it == memo.end()) it = memo.emplace(std::make_pair(L, R), pass_wavefronts(n, L, R, lanes)).first;
       seq.push_back(R);
-      if ((int)seq.size() < RPlan::kMax) search(L / R, cost + 2.0 * n / lanes * it->second + per_pass(R));
+      if ((int)seq.size() < RPlan::kMax) search(L / R, cost + 2.0 * n / lanes * arrays * it->second + per_pass(R));
       seq.pop_back();
     }
   };
@@ -485,6 +486,19 @@ bool make_rplan(int n, int element_bytes, RPlan* out) {
   p.ntw = off;
   *out = p;
   return true;
+}
+
+std::vector<unsigned short> rplan_positions(const RPlan& p) {
+  std::vector<unsigned short> t(p.n);
+  for (int i = 0; i < p.n; ++i) {
+    int rest = i, at = 0;
+    for (int s = 0; s < p.np; ++s) {
+      at += rest % p.R[s] * p.m[s];
+      rest /= p.R[s];
+    }
+    t[i] = (unsigned short)at;
+  }
+  return t;
 }
 
 std::vector<double> rplan_twiddles(const RPlan& p) {

@@ -25,11 +25,12 @@
 //   F_s = RHS(Y_s);  q_{n+1} = q_n + dt sum_s (bE_s F_s - bI_s L^ Y_s)
 // (a stage RHS whose weights are all zero, the first stage's, is skipped).
 //
-// Kernels per step: k_turb_yinv (per kx column: derived fields, projection,
-// y padding, 4 inverse FFTs along y), transpose, k_turb_xpass (per padded y
-// row: 2 packed inverse real FFTs along x, product, forward FFT, x
-// truncation), transpose, k_turb_yfwd (per kx column: forward FFT along y,
-// folds, truncation, SBDF update).
+// Kernels of one right-hand side: k_turb_yinv (groups of kx columns: derived
+// fields, projection, y padding, inverse FFT along y, written as rows over
+// kx), k_turb_xpass (pairs of padded y rows: packed inverse real FFTs along x,
+// products, one packed forward FFT, x truncation), k_turb_yfwd (groups of kx
+// columns: forward FFT along y, folds, truncation, and the SBDF update or the
+// next RK stage combination).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,25 +38,25 @@
 #include <memory>
 #include <vector>
 
-#include "tb_fft.cuh"
+#include "tb_fftr.cuh"
 #include "tb_internal.h"
 #include "tb_plan.h"
 #include "tb_turb.h"
 
 using namespace tb;
 namespace F = tb::fftg;
+namespace Rp = tb::fftr;
 
 struct tb_turb {
   tb_context* ctx = nullptr;
-  int Nx = 0, Ny = 0, Mx = 0, My = 0, Kx = 0;
+  int Nx = 0, Ny = 0, Mx = 0, My = 0, Kx = 0, Kp = 0;  // Kp: Kx rounded up to whole 32-byte sectors
   double Lx = 0, Ly = 0, nu = 0;
-  FftPlan fpMx{}, fpMy{};
-  int nptx = 0, npty = 0;
+  RPlan rx, ry;            // in-place passes of the Mx and My transforms
   cudaStream_t st = nullptr;
   DevBuf Q[2], Fb;         // q_n / q_{n-1} (roles alternate), F_{n-1} (updated in place); [Kx][Ny] complex64
-  DevBuf mix, mixT;        // 4 x [Kx][My] and 4 x [My][Kx]
-  DevBuf pm, pmT;          // [My][Kx] and [Kx][My]
-  DevBuf ptx, pty;         // per-pass twiddles (FP32) of the Mx and My plans
+  DevBuf mix;              // 4 x [My][Kp]: u, v, d_x q, d_y q (and the staging of state copies)
+  DevBuf pm;               // [My][Kp]: the products, x truncated
+  DevBuf twx, twy, posy;   // twiddles of the Mx and My passes, digit-reversed positions of the My transform
   // DiagonalIMEX RK (rk true): tableau and per-stage states / right-hand sides
   bool rk = false;
   int stages = 0;
@@ -79,12 +80,12 @@ namespace {
 constexpr int kTurbThreads = 256;
 
 struct TurbArgs {
-  int Nx, Ny, Mx, My, Kx;
+  int Nx, Ny, Mx, My, Kx, Kp;
   float kx0, ky0, nu;
-  FftPlan fpx, fpy;
-  int nptx, npty;
-  const float2* ptx;
-  const float2* pty;
+  RPlan rx, ry;
+  const float2* twx;
+  const float2* twy;
+  const unsigned short* posy;  // position of y mode / row i after the dif passes
 };
 
 __device__ __forceinline__ float ky_of(int ky, int Ny) { return (float)(ky < Ny / 2 ? ky : ky - Ny); }
@@ -102,206 +103,239 @@ struct TurbComb {
   float2* out;
 };
 
+__device__ __forceinline__ float2 combine_terms(const TurbComb& c, size_t e, float L) {
+  float2 acc = c.base[e];
+#pragma unroll
+  for (int t = 0; t < kCombMax; ++t) {
+    if (t < c.n) {
+      const float2 v = c.src[t][e];
+      const float wt = c.isL[t] ? c.w[t] * L : c.w[t];
+      acc = F::mk<float2>(fmaf(wt, v.x, acc.x), fmaf(wt, v.y, acc.y));
+    }
+  }
+  return acc;
+}
+__device__ __forceinline__ float2 combine_scale(const TurbComb& c, float2 acc, float L) {
+  if (c.dgam == 0.f) return acc;
+  const float den = 1.0f / (1.0f + c.dgam * L);
+  return F::mk<float2>(acc.x * den, acc.y * den);
+}
+
 __global__ void __launch_bounds__(256) k_turb_combine(TurbArgs a, TurbComb c) {
   const size_t total = (size_t)a.Kx * a.Ny;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
     const int kx = (int)(e / a.Ny), ky = (int)(e % a.Ny);
     const float kxv = a.kx0 * kx, kyv = a.ky0 * ky_of(ky, a.Ny);
     const float L = a.nu * (kxv * kxv + kyv * kyv);
-    float2 acc = c.base[e];
-#pragma unroll
-    for (int t = 0; t < kCombMax; ++t) {
-      if (t < c.n) {
-        const float2 v = c.src[t][e];
-        const float wt = c.isL[t] ? c.w[t] * L : c.w[t];
-        acc = F::mk<float2>(fmaf(wt, v.x, acc.x), fmaf(wt, v.y, acc.y));
-      }
-    }
-    if (c.dgam != 0.f) {
-      const float den = 1.0f / (1.0f + c.dgam * L);
-      acc = F::mk<float2>(acc.x * den, acc.y * den);
-    }
-    c.out[e] = acc;
+    c.out[e] = combine_scale(c, combine_terms(c, e, L), L);
   }
 }
 
-// Per kx column: the four factors u, v, d_x q, d_y q of the products, with the
+// Column buffers of the y kernels: entry i of column c at c * ystride + sw(i);
+// four extra entries a column put the same entry of neighbouring columns on
+// different banks.
+__host__ __device__ inline int ystride(int My) { return Rp::rpad<float2>(My) + 4; }
+
+// One factor (blockIdx.y: 0 u, 1 v, 2 d_x q, 3 d_y q) of CW kx columns, with the
 // grid round trip's projection, the x Nyquist split and the y padding, inverse
-// FFT along y; out: mix[f][kx][y], f = u, v, qx, qy.
-__global__ void __launch_bounds__(kTurbThreads) k_turb_yinv(TurbArgs a, const float2* __restrict__ q,
-                                                            float2* __restrict__ mix) {
-  extern __shared__ float2 sm[];
-  const int My = a.My, Ny = a.Ny, kx = blockIdx.x;
-  const int Ms = (My + 7) & ~7;
-  float2* A = sm;
-  float2* B = sm + Ms;
-  float2* qs = sm + 2 * Ms;        // the q^ column
-  float2* pt = qs + Ny;            // twiddles of the My plan
-  for (int t = threadIdx.x; t < a.npty; t += blockDim.x) pt[t] = a.pty[t];
-  for (int t = threadIdx.x; t < Ny; t += blockDim.x) qs[t] = q[(size_t)kx * Ny + t];
+// FFT along y; out: mix[f][y][kx].  The columns of a group share the passes'
+// barriers and their rows are stored together (32 bytes at CW = 4), which
+// replaces a separate transpose: bound by shared-memory traffic.
+template <int CW>
+__global__ void __launch_bounds__(kTurbThreads, 3) k_turb_yinv(TurbArgs a, const float2* __restrict__ q,
+                                                               float2* __restrict__ mix) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int My = a.My, Ny = a.Ny, kx0 = blockIdx.x * CW, f = blockIdx.y;
+  const int Ms = ystride(My), hy = Ny / 2;
+  float2* tw = sm + CW * Ms;
+  for (int t = threadIdx.x; t < a.ry.ntw; t += blockDim.x) tw[t] = a.twy[t];
+  for (int t = threadIdx.x; t < CW * Ny; t += blockDim.x) {
+    const int c = t / Ny, ky = t - c * Ny, kx = kx0 + c;
+    if (kx >= a.Kx) break;
+    const float kxv = a.kx0 * kx, kyv = a.ky0 * ky_of(ky, Ny);
+    float2 v = q[(size_t)kx * Ny + ky];
+    // the kx = 0 / Nyquist columns lose their non-Hermitian part in the grid
+    // round trip, before any derivative is taken
+    if (kx == 0 || 2 * kx == a.Nx) {
+      const float2 w = q[(size_t)kx * Ny + (ky ? Ny - ky : 0)];
+      v = F::mk<float2>(0.5f * (v.x + w.x), 0.5f * (v.y - w.y));
+    }
+    if (f < 2) {  // psi = -q / k^2, 0 at k = 0
+      const float k2 = kxv * kxv + kyv * kyv;
+      v = k2 > 1e-12f ? F::mk<float2>(-v.x / k2, -v.y / k2) : F::mk<float2>(0.f, 0.f);
+    }
+    const float d = (f == 0) ? -kyv : (f == 3 ? kyv : kxv);  // u = -i ky psi, v = i kx psi, i kx q, i ky q
+    const float xs = (2 * kx == a.Nx) ? 0.5f : 1.0f;         // even-N Nyquist split along x
+    v = F::mk<float2>(-(d * v.y) * xs, (d * v.x) * xs);
+    float2* col = sm + c * Ms;
+    if (ky < hy) {
+      col[Rp::sw<float2>(ky)] = v;
+    } else if (ky == hy) {
+      v = F::scale(v, 0.5f);
+      col[Rp::sw<float2>(hy)] = v;
+      col[Rp::sw<float2>(My - hy)] = v;
+    } else {
+      col[Rp::sw<float2>(My - Ny + ky)] = v;
+    }
+  }
+  const int gap = My - Ny - 1;  // y bins hy + 1 .. My - hy - 1 are zero
+  for (int t = threadIdx.x; t < gap; t += blockDim.x)
+#pragma unroll
+    for (int c = 0; c < CW; ++c) sm[c * Ms + Rp::sw<float2>(hy + 1 + t)] = F::mk<float2>(0.f, 0.f);
   __syncthreads();
-  const float kxv = a.kx0 * kx;
-  const bool edge = (kx == 0) || (2 * kx == a.Nx);  // columns whose grid round trip is real
-  const float xs = (2 * kx == a.Nx) ? 0.5f : 1.0f;  // even-N Nyquist split along x
-  // q^ of the grid round trip: the kx = 0 / Nyquist columns lose their
-  // non-Hermitian part before any derivative is taken
-  auto qproj = [&](int ky) -> float2 {
-    const float2 c = qs[ky];
-    if (!edge) return c;
-    const float2 w = qs[(Ny - ky) % Ny];
-    return F::mk<float2>(0.5f * (c.x + w.x), 0.5f * (c.y - w.y));
-  };
-  auto factor = [&](int f, int ky) -> float2 {
-    const float kyv = a.ky0 * ky_of(ky, Ny);
-    const float2 c = qproj(ky);
-    const float k2 = kxv * kxv + kyv * kyv;
-    float2 psi = k2 > 1e-12f ? F::mk<float2>(-c.x / k2, -c.y / k2) : F::mk<float2>(0.f, 0.f);
-    // i k z = (-k z.y, k z.x)
-    if (f == 0) return F::mk<float2>(kyv * psi.y, -kyv * psi.x);   // -i ky psi
-    if (f == 1) return F::mk<float2>(-kxv * psi.y, kxv * psi.x);   //  i kx psi
-    if (f == 2) return F::mk<float2>(-kxv * c.y, kxv * c.x);       //  i kx q
-    return F::mk<float2>(-kyv * c.y, kyv * c.x);                    //  i ky q
-  };
-  for (int f = 0; f < 4; ++f) {
-    for (int y = threadIdx.x; y < My; y += blockDim.x) A[F::fidx<true>(y)] = F::mk<float2>(0.f, 0.f);
+  for (int s = 0; s < a.ry.np; ++s) {
+    Rp::pass_any<true, 1>(sm, CW, Ms, a.ry, s, tw);
     __syncthreads();
-    for (int ky = threadIdx.x; ky < Ny; ky += blockDim.x) {
-      float2 v = factor(f, ky);
-      v = F::scale(v, xs);
-      if (2 * ky < Ny) {
-        A[F::fidx<true>(ky)] = v;
-      } else if (2 * ky == Ny) {
-        const float2 h = F::scale(v, 0.5f);
-        A[F::fidx<true>(Ny / 2)] = h;
-        A[F::fidx<true>(My - Ny / 2)] = h;
-      } else {
-        A[F::fidx<true>(My - Ny + ky)] = v;
+  }
+  float2* out = mix + (size_t)f * My * a.Kp + kx0;
+  for (int t = threadIdx.x; t < CW * My; t += blockDim.x) {
+    const int c = t % CW, y = t / CW;
+    if (kx0 + c < a.Kx) out[(size_t)y * a.Kp + c] = sm[c * Ms + Rp::sw<float2>(a.posy[y])];
+  }
+}
+
+// Products u d_x q + v d_y q of two padded y rows (y0, y0 + 1): u + i v and
+// d_x q + i d_y q of each row to the padded x grid (four arrays), the products
+// of the rows as one complex array forward, bins 0..Nx/2 of both out.  The last
+// inverse pass, the product and the first forward pass stay in registers.
+template <int R>
+__device__ __forceinline__ void xmiddle(float2* __restrict__ A, int Ms, int n) {
+  for (int b = threadIdx.x; b < n / R; b += blockDim.x) {
+    int at[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) at[r] = Rp::sw<float2>(b * R + r);
+    float2 u[R], g[R], z[R];
+#pragma unroll
+    for (int row = 0; row < 2; ++row) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) u[r] = A[(2 * row) * Ms + at[r]];
+      Rp::dft<R, 1>(u);
+#pragma unroll
+      for (int r = 0; r < R; ++r) g[r] = A[(2 * row + 1) * Ms + at[r]];
+      Rp::dft<R, 1>(g);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float p = u[r].x * g[r].x + u[r].y * g[r].y;
+        if (row)
+          z[r].y = p;
+        else
+          z[r].x = p;
       }
     }
-    __syncthreads();
-    float2* R = F::fft<true>(A, B, a.fpy, pt, +1);
-    float2* out = mix + ((size_t)f * a.Kx + kx) * My;
-    for (int y = threadIdx.x; y < My; y += blockDim.x) out[y] = R[F::fidx<true>(y)];
-    __syncthreads();
+    Rp::dft<R, -1>(z);
+#pragma unroll
+    for (int r = 0; r < R; ++r) A[at[r]] = z[r];
   }
 }
 
-// Batched transpose: in[b][R][C] -> out[b][C][R] (32 x 32 tiles).
-__global__ void __launch_bounds__(256) k_transpose_c64(const float2* __restrict__ in, float2* __restrict__ out, int R,
-                                                        int C) {
-  __shared__ float2 tile[32][33];
-  const size_t boff = (size_t)blockIdx.z * R * C;
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    if (r < R && c < C) tile[i][threadIdx.x] = in[boff + (size_t)r * C + c];
-  }
-  __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int c = c0 + i, r = r0 + threadIdx.x;
-    if (r < R && c < C) out[boff + (size_t)c * R + r] = tile[threadIdx.x][i];
-  }
-}
-
-// Per padded y row: u, v, d_x q, d_y q on the padded x grid (two packed inverse
-// real FFTs), the product u d_x q + v d_y q, its forward FFT, bins 0..Nx/2.
-__global__ void __launch_bounds__(kTurbThreads) k_turb_xpass(TurbArgs a, const float2* __restrict__ mixT,
-                                                             float2* __restrict__ pm) {
-  extern __shared__ float2 sm[];
-  const int Mx = a.Mx, Kx = a.Kx, My = a.My, y = blockIdx.x;
-  const int Ms = (Mx + 7) & ~7;
-  float2* Z1 = sm;
-  float2* Z2 = sm + Ms;
-  float2* S1 = sm + 2 * Ms;
-  float2* S2 = sm + 3 * Ms;
-  float2* pt = sm + 4 * Ms;
-  for (int t = threadIdx.x; t < a.nptx; t += blockDim.x) pt[t] = a.ptx[t];
-  auto row = [&](int f) { return mixT + ((size_t)f * My + y) * Kx; };
-  const float2 *ru = row(0), *rv = row(1), *rqx = row(2), *rqy = row(3);
-  // half-spectrum bin k of a factor (zero past the data; DC and Nyquist kept
-  // real, as the factor's own irfft on Nx points does)
-  auto bin = [&](const float2* r, int k) -> float2 {
-    if (k >= Kx) return F::mk<float2>(0.f, 0.f);
-    float2 v = r[k];
-    if (k == 0 || 2 * k == a.Nx) v.y = 0.f;
-    return v;
-  };
-  for (int k = threadIdx.x; k <= Mx / 2; k += blockDim.x) {
-    const float2 U = bin(ru, k), V = bin(rv, k), QX = bin(rqx, k), QY = bin(rqy, k);
-    // spectrum of a + i b: A + i B at k, conj(A) + i conj(B) at Mx - k
-    Z1[F::fidx<true>(k)] = F::mk<float2>(U.x - V.y, U.y + V.x);
-    Z2[F::fidx<true>(k)] = F::mk<float2>(QX.x - QY.y, QX.y + QY.x);
-    if (k > 0 && k < Mx / 2) {
-      Z1[F::fidx<true>(Mx - k)] = F::mk<float2>(U.x + V.y, -U.y + V.x);
-      Z2[F::fidx<true>(Mx - k)] = F::mk<float2>(QX.x + QY.y, -QX.y + QY.x);
+__global__ void __launch_bounds__(kTurbThreads, 3) k_turb_xpass(TurbArgs a, const float2* __restrict__ mix,
+                                                                float2* __restrict__ pm) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int Mx = a.Mx, hN = a.Nx / 2, y0 = 2 * blockIdx.x;
+  const int Ms = Rp::rpad<float2>(Mx);
+  float2* tw = sm + 4 * Ms;
+  for (int t = threadIdx.x; t < a.rx.ntw; t += blockDim.x) tw[t] = a.twx[t];
+  const size_t plane = (size_t)a.My * a.Kp;
+  const float2* in = mix + (size_t)y0 * a.Kp;
+  for (int k = threadIdx.x; k <= hN; k += blockDim.x) {
+    float2 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = in[(size_t)(i % 4) * plane + (size_t)(i / 4) * a.Kp + k];
+    if (k == 0 || k == hN)  // DC and Nyquist kept real, as the factor's own irfft on Nx points does
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i].y = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // array 2 row + pair: spectrum of first + i second
+      const float2 P = v[2 * i], Q = v[2 * i + 1];
+      sm[i * Ms + Rp::sw<float2>(k)] = F::mk<float2>(P.x - Q.y, P.y + Q.x);
+      if (k > 0) sm[i * Ms + Rp::sw<float2>(Mx - k)] = F::mk<float2>(P.x + Q.y, -P.y + Q.x);
     }
   }
+  for (int k = hN + 1 + threadIdx.x; k < Mx - hN; k += blockDim.x)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sm[i * Ms + Rp::sw<float2>(k)] = F::mk<float2>(0.f, 0.f);
   __syncthreads();
-  float2* z1 = F::fft<true>(Z1, S1, a.fpx, pt, +1);
-  float2* z2 = F::fft<true>(Z2, S2, a.fpx, pt, +1);
-  float2* P = (z1 == Z1) ? S1 : Z1;
-  float2* W = (z2 == Z2) ? S2 : Z2;
-  for (int x = threadIdx.x; x < Mx; x += blockDim.x) {
-    const int i = F::fidx<true>(x);
-    const float2 s = z1[i], t = z2[i];
-    P[i] = F::mk<float2>(s.x * t.x + s.y * t.y, 0.f);
+  const int last = a.rx.np - 1;
+  for (int s = 0; s < last; ++s) {
+    Rp::pass_any<true, 1>(sm, 4, Ms, a.rx, s, tw);
+    __syncthreads();
+  }
+  switch (a.rx.R[last]) {
+    case 8: xmiddle<8>(sm, Ms, Mx); break;
+    case 6: xmiddle<6>(sm, Ms, Mx); break;
+    case 4: xmiddle<4>(sm, Ms, Mx); break;
+    case 3: xmiddle<3>(sm, Ms, Mx); break;
+    default: xmiddle<2>(sm, Ms, Mx); break;
   }
   __syncthreads();
-  float2* C = F::fft<true>(P, W, a.fpx, pt, -1);
-  for (int k = threadIdx.x; k < Kx; k += blockDim.x) pm[(size_t)y * Kx + k] = C[F::fidx<true>(k)];
+  for (int s = last - 1; s >= 0; --s) {
+    Rp::pass_any<false, -1>(sm, 1, Ms, a.rx, s, tw);
+    __syncthreads();
+  }
+  float2* out = pm + (size_t)y0 * a.Kp;
+  for (int k = threadIdx.x; k <= hN; k += blockDim.x) {
+    const float2 c = sm[Rp::sw<float2>(k)], w = sm[Rp::sw<float2>(k ? Mx - k : 0)];
+    out[k] = F::mk<float2>(0.5f * (c.x + w.x), 0.5f * (c.y - w.y));
+    out[a.Kp + k] = F::mk<float2>(0.5f * (c.y + w.y), -0.5f * (c.x - w.x));
+  }
 }
 
-// Per kx column: forward FFT along y, the Nyquist folds and truncation to Ny,
-// F = -(...) / (Nx Ny Mx My), and the SBDF1 / SBDF2 update in place.
-//   qn: q_n [Kx][Ny];  qo: q_{n-1} on entry, q_{n+1} on exit;  Fp: F_{n-1} on
-//   entry, F_n on exit.  first: 1 SBDF1 startup (q_{n+1} written to qo),
-//   0 SBDF2, 2 the right-hand side alone (Fp = F; qn and qo untouched).
-__global__ void __launch_bounds__(kTurbThreads) k_turb_yfwd(TurbArgs a, const float2* __restrict__ pmT,
-                                                            const float2* __restrict__ qn, float2* __restrict__ qo,
-                                                            float2* __restrict__ Fp, float dt, int first) {
-  extern __shared__ float2 sm[];
-  const int My = a.My, Ny = a.Ny, kx = blockIdx.x;
-  const int Ms = (My + 7) & ~7;
-  float2* A = sm;
-  float2* B = sm + Ms;
-  float2* pt = sm + 2 * Ms;
-  for (int t = threadIdx.x; t < a.npty; t += blockDim.x) pt[t] = a.pty[t];
-  const float2* col = pmT + (size_t)kx * My;
-  for (int y = threadIdx.x; y < My; y += blockDim.x) A[F::fidx<true>(y)] = col[y];
+// CW kx columns: forward FFT along y, the Nyquist folds and truncation to Ny,
+// F = -(...) / (Nx Ny Mx My), then
+//   mode 0 SBDF2 / 1 SBDF1: the update; qn: q_n [Kx][Ny], qo: q_{n-1} on entry
+//          and q_{n+1} on exit, Fp: F_{n-1} on entry and F_n on exit;
+//   mode 2 an RK stage: F_s to Fp (null: no later stage reads it) and the next
+//          combination c with the term wF F_s added (the stage's own right-hand
+//          side never makes a round trip through memory).
+template <int CW>
+__global__ void __launch_bounds__(kTurbThreads, 3) k_turb_yfwd(TurbArgs a, const float2* __restrict__ pm,
+                                                               const float2* __restrict__ qn, float2* __restrict__ qo,
+                                                               float2* __restrict__ Fp, float dt, int mode, TurbComb c,
+                                                               float wF) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int My = a.My, Ny = a.Ny, kx0 = blockIdx.x * CW, hy = Ny / 2;
+  const int Ms = ystride(My);
+  float2* tw = sm + CW * Ms;
+  for (int t = threadIdx.x; t < a.ry.ntw; t += blockDim.x) tw[t] = a.twy[t];
+  for (int t = threadIdx.x; t < CW * My; t += blockDim.x) {  // columns past Kx read the row padding
+    const int cc = t % CW, y = t / CW;
+    sm[cc * Ms + Rp::sw<float2>(y)] = pm[(size_t)y * a.Kp + kx0 + cc];
+  }
   __syncthreads();
-  const float2* Q = F::fft<true>(A, B, a.fpy, pt, -1);
-  const bool xnyq = (2 * kx == a.Nx);
-  // Q'(y) with the x fold: Q(Nx/2, y) + conj(Q(Nx/2, -y))
-  auto qf = [&](int yy) -> float2 {
-    float2 v = Q[F::fidx<true>(yy)];
-    if (xnyq) {
-      const float2 w = Q[F::fidx<true>((My - yy) % My)];
-      v = F::mk<float2>(v.x + w.x, v.y - w.y);
-    }
-    return v;
-  };
+  for (int s = 0; s < a.ry.np; ++s) {
+    Rp::pass_any<true, -1>(sm, CW, Ms, a.ry, s, tw);
+    __syncthreads();
+  }
   const float sc = -1.0f / ((float)a.Nx * (float)Ny * (float)a.Mx * (float)My);
-  const float kxv = a.kx0 * kx;
-  for (int ky = threadIdx.x; ky < Ny; ky += blockDim.x) {
-    float2 r;
-    if (2 * ky < Ny) {
-      r = qf(ky);
-    } else if (2 * ky == Ny) {
-      r = F::add(qf(Ny / 2), qf(My - Ny / 2));
-    } else {
-      r = qf(My - Ny + ky);
-    }
+  for (int t = threadIdx.x; t < CW * Ny; t += blockDim.x) {
+    const int cc = t / Ny, ky = t - cc * Ny, kx = kx0 + cc;
+    if (kx >= a.Kx) break;
+    const bool xnyq = 2 * kx == a.Nx;
+    // Q'(y) with the x fold: Q(Nx/2, y) + conj(Q(Nx/2, -y))
+    auto qf = [&](int yy) -> float2 {
+      float2 v = sm[cc * Ms + Rp::sw<float2>(a.posy[yy])];
+      if (xnyq) {
+        const float2 w = sm[cc * Ms + Rp::sw<float2>(a.posy[yy ? My - yy : 0])];
+        v = F::mk<float2>(v.x + w.x, v.y - w.y);
+      }
+      return v;
+    };
+    float2 r = qf(ky <= hy ? ky : My - Ny + ky);
+    if (ky == hy) r = F::add(r, qf(My - hy));
     const float2 Fn = F::scale(r, sc);
     const size_t e = (size_t)kx * Ny + ky;
-    if (first == 2) {
-      Fp[e] = Fn;
+    const float kxv = a.kx0 * kx, kyv = a.ky0 * ky_of(ky, Ny);
+    const float L = a.nu * (kxv * kxv + kyv * kyv);
+    if (mode == 2) {
+      if (Fp) Fp[e] = Fn;
+      float2 acc = combine_terms(c, e, L);
+      acc = F::mk<float2>(fmaf(wF, Fn.x, acc.x), fmaf(wF, Fn.y, acc.y));
+      c.out[e] = combine_scale(c, acc, L);
       continue;
     }
-    const float kyv = a.ky0 * ky_of(ky, Ny);
-    const float L = a.nu * (kxv * kxv + kyv * kyv);
     const float2 q0 = qn[e];
     float2 q1;
-    if (first) {
+    if (mode == 1) {
       const float den = 1.0f / (1.0f + dt * L);
       q1 = F::mk<float2>((q0.x + dt * Fn.x) * den, (q0.y + dt * Fn.y) * den);
     } else {
@@ -315,17 +349,48 @@ __global__ void __launch_bounds__(kTurbThreads) k_turb_yfwd(TurbArgs a, const fl
   }
 }
 
-size_t yinv_smem(const tb_turb* T) {
-  const size_t Ms = (T->My + 7) & ~7;
-  return (2 * Ms + T->Ny + T->npty) * sizeof(float2);
+// State copies: the device's [kx][ky] FP32 coefficients <-> the caller's layout
+// (ky rows of Kx complex128), 32 x 32 tiles.
+template <bool OUT>
+__global__ void __launch_bounds__(256) k_turb_state(float2* __restrict__ q, double2* __restrict__ pub, int Kx, int Ny) {
+  __shared__ float2 tile[32][33];
+  const int kx0 = blockIdx.x * 32, ky0 = blockIdx.y * 32;
+  for (int i = threadIdx.y; i < 32; i += 8) {
+    if (OUT) {
+      const int kx = kx0 + i, ky = ky0 + threadIdx.x;
+      if (kx < Kx && ky < Ny) tile[i][threadIdx.x] = q[(size_t)kx * Ny + ky];
+    } else {
+      const int ky = ky0 + i, kx = kx0 + threadIdx.x;
+      if (kx < Kx && ky < Ny) {
+        const double2 v = pub[(size_t)ky * Kx + kx];
+        tile[i][threadIdx.x] = make_float2((float)v.x, (float)v.y);
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.y; i < 32; i += 8) {
+    if (OUT) {
+      const int ky = ky0 + i, kx = kx0 + threadIdx.x;
+      if (kx < Kx && ky < Ny) {
+        const float2 v = tile[threadIdx.x][i];
+        pub[(size_t)ky * Kx + kx] = make_double2(v.x, v.y);
+      }
+    } else {
+      const int kx = kx0 + i, ky = ky0 + threadIdx.x;
+      if (kx < Kx && ky < Ny) q[(size_t)kx * Ny + ky] = tile[threadIdx.x][i];
+    }
+  }
 }
-size_t xpass_smem(const tb_turb* T) {
-  const size_t Ms = (T->Mx + 7) & ~7;
-  return (4 * Ms + T->nptx) * sizeof(float2);
-}
-size_t yfwd_smem(const tb_turb* T) {
-  const size_t Ms = (T->My + 7) & ~7;
-  return (2 * Ms + T->npty) * sizeof(float2);
+
+size_t y_smem(const tb_turb* T, int cw) { return ((size_t)cw * ystride(T->My) + T->ry.ntw) * sizeof(float2); }
+size_t x_smem(const tb_turb* T) { return (4 * (size_t)Rp::rpad<float2>(T->Mx) + T->rx.ntw) * sizeof(float2); }
+
+// kx columns a block: four store and load whole 32-byte sectors, but few
+// columns leave SMs idle, so the widest that still gives 1.5 blocks an SM.
+int columns_per_block(int Kx, int factors) {
+  for (int cw : {4, 2})
+    if ((Kx + cw - 1) / cw * factors >= 222) return cw;
+  return 1;
 }
 
 TurbArgs args_of(const tb_turb* T) {
@@ -335,30 +400,33 @@ TurbArgs args_of(const tb_turb* T) {
   a.Mx = T->Mx;
   a.My = T->My;
   a.Kx = T->Kx;
+  a.Kp = T->Kp;
   a.kx0 = (float)(2.0 * M_PI / T->Lx);
   a.ky0 = (float)(2.0 * M_PI / T->Ly);
   a.nu = (float)T->nu;
-  a.fpx = T->fpMx;
-  a.fpy = T->fpMy;
-  a.nptx = T->nptx;
-  a.npty = T->npty;
-  a.ptx = T->ptx.as<float2>();
-  a.pty = T->pty.as<float2>();
+  a.rx = T->rx;
+  a.ry = T->ry;
+  a.twx = T->twx.as<float2>();
+  a.twy = T->twy.as<float2>();
+  a.posy = T->posy.as<unsigned short>();
   return a;
 }
 
-// The RHS chain on q, ending in k_turb_yfwd with mode first (see there).
-void enqueue_rhs(tb_turb* T, const float2* q, float2* qo, float2* Fp, double dt, int first) {
+// The RHS chain on q, ending in k_turb_yfwd with its mode (see there).
+void enqueue_rhs(tb_turb* T, const float2* q, float2* qo, float2* Fp, double dt, int mode, const TurbComb& c,
+                 double wF) {
   const TurbArgs a = args_of(T);
   float2* mix = T->mix.as<float2>();
-  float2* mixT = T->mixT.as<float2>();
-  k_turb_yinv<<<T->Kx, kTurbThreads, yinv_smem(T), T->st>>>(a, q, mix);
-  dim3 tb(32, 8);
-  k_transpose_c64<<<dim3((T->My + 31) / 32, (T->Kx + 31) / 32, 4), tb, 0, T->st>>>(mix, mixT, T->Kx, T->My);
-  k_turb_xpass<<<T->My, kTurbThreads, xpass_smem(T), T->st>>>(a, mixT, T->pm.as<float2>());
-  k_transpose_c64<<<dim3((T->Kx + 31) / 32, (T->My + 31) / 32, 1), tb, 0, T->st>>>(T->pm.as<float2>(),
-                                                                                   T->pmT.as<float2>(), T->My, T->Kx);
-  k_turb_yfwd<<<T->Kx, kTurbThreads, yfwd_smem(T), T->st>>>(a, T->pmT.as<float2>(), q, qo, Fp, (float)dt, first);
+  float2* pm = T->pm.as<float2>();
+  // about one butterfly of radix 8 a thread
+  auto threads = [](int arrays, int n) { return arrays * n <= 1024 ? kTurbThreads / 2 : kTurbThreads; };
+  const int ci = columns_per_block(T->Kx, 4), cf = columns_per_block(T->Kx, 1);
+  auto yinv = ci == 4 ? k_turb_yinv<4> : ci == 2 ? k_turb_yinv<2> : k_turb_yinv<1>;
+  auto yfwd = cf == 4 ? k_turb_yfwd<4> : cf == 2 ? k_turb_yfwd<2> : k_turb_yfwd<1>;
+  yinv<<<dim3((T->Kx + ci - 1) / ci, 4), threads(ci, T->My), y_smem(T, ci), T->st>>>(a, q, mix);
+  k_turb_xpass<<<T->My / 2, threads(4, T->Mx), x_smem(T), T->st>>>(a, mix, pm);
+  yfwd<<<(T->Kx + cf - 1) / cf, threads(cf, T->My), y_smem(T, cf), T->st>>>(a, pm, q, qo, Fp, (float)dt, mode, c,
+                                                                            (float)wF);
 }
 
 void launch_combine(tb_turb* T, const TurbComb& c) {
@@ -381,30 +449,35 @@ void enqueue_rk_step(tb_turb* T, double dt) {
     ++c.n;
   };
   const int s = T->stages;
-  for (int i = 0; i < s; ++i) {
-    if (i > 0) {
-      TurbComb c{};
-      c.base = qn;
-      for (int j = 0; j < i; ++j) {
-        if (std::fabs(T->AE[i][j]) > 1e-14) add(c, T->Fs[j].as<float2>(), dt * T->AE[i][j], 0);
-        if (std::fabs(T->AI[i][j]) > 1e-14) add(c, Y[j], -dt * T->AI[i][j], 1);
-      }
-      c.dgam = std::fabs(T->AI[i][i]) > 1e-14 ? (float)(dt * T->AI[i][i]) : 0.f;
-      c.out = T->Ys[i].as<float2>();
-      launch_combine(T, c);
-      Y[i] = T->Ys[i].as<float2>();
+  // the combination that gives stage i (i = s: q_{n+1}) without the term of its
+  // newest right-hand side, whose weight goes to *w
+  auto combination = [&](int i, double* w) {
+    const double* wE = i < s ? T->AE[i] : T->bE;
+    const double* wI = i < s ? T->AI[i] : T->bI;
+    TurbComb c{};
+    c.base = qn;
+    for (int j = 0; j < i; ++j) {
+      if (j < i - 1 && std::fabs(wE[j]) > 1e-14) add(c, T->Fs[j].as<float2>(), dt * wE[j], 0);
+      if (std::fabs(wI[j]) > 1e-14) add(c, Y[j], -dt * wI[j], 1);
     }
-    if (T->f_used[i]) enqueue_rhs(T, Y[i], nullptr, T->Fs[i].as<float2>(), dt, 2);
-  }
-  TurbComb c{};
-  c.base = qn;
+    *w = dt * wE[i - 1];
+    c.dgam = i < s && std::fabs(T->AI[i][i]) > 1e-14 ? (float)(dt * T->AI[i][i]) : 0.f;
+    c.out = i < s ? T->Ys[i].as<float2>() : qo;
+    return c;
+  };
   for (int i = 0; i < s; ++i) {
-    if (std::fabs(T->bE[i]) > 1e-14) add(c, T->Fs[i].as<float2>(), dt * T->bE[i], 0);
-    if (std::fabs(T->bI[i]) > 1e-14) add(c, Y[i], -dt * T->bI[i], 1);
+    double w = 0.0;
+    if (!T->f_used[i]) {  // no weight anywhere: the next combination stands alone
+      launch_combine(T, combination(i + 1, &w));
+    } else {
+      // F_i is kept only where a combination after the next one reads it
+      bool later = i + 1 < s && std::fabs(T->bE[i]) > 1e-14;
+      for (int k = i + 2; k < s; ++k) later = later || std::fabs(T->AE[k][i]) > 1e-14;
+      const TurbComb c = combination(i + 1, &w);
+      enqueue_rhs(T, Y[i], nullptr, later ? T->Fs[i].as<float2>() : nullptr, dt, 2, c, w);
+    }
+    if (i + 1 < s) Y[i + 1] = T->Ys[i + 1].as<float2>();
   }
-  c.dgam = 0.f;
-  c.out = qo;
-  launch_combine(T, c);
 }
 
 void enqueue_step(tb_turb* T, double dt, int first) {
@@ -414,22 +487,13 @@ void enqueue_step(tb_turb* T, double dt, int first) {
   }
   float2* qn = T->Q[T->cur].as<float2>();
   float2* qo = T->Q[1 - T->cur].as<float2>();
-  enqueue_rhs(T, qn, qo, T->Fb.as<float2>(), dt, first);
+  enqueue_rhs(T, qn, qo, T->Fb.as<float2>(), dt, first, TurbComb{}, 0.0);
 }
 
-std::vector<float2> pass_twiddles_f(const FftPlan& fp) {
-  std::vector<float2> t;
-  const long double pi = 3.141592653589793238462643383279502884L;
-  int Ns = 1;
-  for (int s = 0; s < fp.nstages; ++s) {
-    const int R = fp.radix[s];
-    const int tstride = fp.n / (Ns * R);
-    for (int j = 0; j < Ns; ++j) {
-      const long double ang = -2.0L * pi * (long double)(j * tstride) / (long double)fp.n;
-      t.push_back(make_float2((float)cosl(ang), (float)sinl(ang)));
-    }
-    Ns *= R;
-  }
+std::vector<float2> pass_table(const RPlan& p) {
+  const std::vector<double> w = rplan_twiddles(p);
+  std::vector<float2> t(w.size() / 2);
+  for (size_t i = 0; i < t.size(); ++i) t[i] = make_float2((float)w[2 * i], (float)w[2 * i + 1]);
   return t;
 }
 
@@ -453,12 +517,11 @@ cudaGraphExec_t capture(tb_turb* T, double dt) {
 }  // namespace
 
 size_t tb::turb_estimate_bytes(int Nx, int Ny, int timestepper) {
-  const size_t Kx = Nx / 2 + 1, Mx = padded_len(Nx), My = padded_len(Ny);
-  (void)Mx;
+  const size_t Kx = Nx / 2 + 1, Kp = (Kx + 3) / 4 * 4, My = padded_len(Ny);
   // SBDF2: q_n, q_{n-1}, F_{n-1}; RK: q_n, q_{n+1} and up to 3 stage states
   // and 3 stage right-hand sides (4 stages, the first state and RHS not kept)
   const size_t specs = timestepper == TB_SBDF2 ? 3 : (timestepper == TB_RK222 ? 6 : 8);
-  return sizeof(float2) * (specs * Kx * Ny + 8 * Kx * My + 2 * Kx * My) + (4u << 20);
+  return sizeof(float2) * (specs * Kx * Ny + 5 * Kp * My) + (4u << 20);
 }
 
 tb_turb* tb::turb_create(tb_context* ctx, const tb_problem_desc& d, const double* q0) {
@@ -499,7 +562,8 @@ tb_turb* tb::turb_create(tb_context* ctx, const tb_problem_desc& d, const double
   T->Lx = d.Lx;
   T->Ly = d.Ly;
   T->nu = d.nu;
-  TB_REQUIRE(make_fft_plan(T->Mx, &T->fpMx) && make_fft_plan(T->My, &T->fpMy), TB_ENOTSUPPORTED,
+  T->Kp = (T->Kx + 3) / 4 * 4;
+  TB_REQUIRE(make_rplan(T->Mx, sizeof(float2), &T->rx, 5) && make_rplan(T->My, sizeof(float2), &T->ry, 2), TB_ENOTSUPPORTED,
              "Nx, Ny must be of the form 2^a 3^b");
   TB_CUDA_TRY(cudaSetDevice(ctx->device));
   TB_CUDA_TRY(create_work_stream(&T->st));
@@ -512,19 +576,18 @@ tb_turb* tb::turb_create(tb_context* ctx, const tb_problem_desc& d, const double
   } else {
     T->Fb.alloc(spec);
   }
-  T->mix.alloc(4 * (size_t)T->Kx * T->My * sizeof(float2));
-  T->mixT.alloc(T->mix.bytes);
-  T->pm.alloc((size_t)T->Kx * T->My * sizeof(float2));
-  T->pmT.alloc(T->pm.bytes);
-  upload(T->ptx, pass_twiddles_f(T->fpMx));
-  upload(T->pty, pass_twiddles_f(T->fpMy));
-  T->nptx = F::pass_twiddle_count(T->fpMx);
-  T->npty = F::pass_twiddle_count(T->fpMy);
-  TB_REQUIRE(xpass_smem(T.get()) <= 227 * 1024 && yinv_smem(T.get()) <= 227 * 1024, TB_ENOTSUPPORTED,
+  T->mix.alloc(4 * (size_t)T->My * T->Kp * sizeof(float2));
+  T->pm.alloc((size_t)T->My * T->Kp * sizeof(float2));
+  TB_CUDA_TRY(cudaMemsetAsync(T->pm.p, 0, T->pm.bytes, T->st));  // the row padding stays zero
+  upload(T->twx, pass_table(T->rx));
+  upload(T->twy, pass_table(T->ry));
+  upload(T->posy, rplan_positions(T->ry));
+  TB_REQUIRE(x_smem(T.get()) <= 227 * 1024 && y_smem(T.get(), 4) <= 227 * 1024, TB_ENOTSUPPORTED,
              "turbulence grid too large for the shared-memory transforms");
-  TB_CUDA_TRY(cudaFuncSetAttribute(k_turb_yinv, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-  TB_CUDA_TRY(cudaFuncSetAttribute(k_turb_xpass, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-  TB_CUDA_TRY(cudaFuncSetAttribute(k_turb_yfwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+  for (const void* k : {(const void*)k_turb_yinv<1>, (const void*)k_turb_yinv<2>, (const void*)k_turb_yinv<4>,
+                        (const void*)k_turb_xpass, (const void*)k_turb_yfwd<1>, (const void*)k_turb_yfwd<2>,
+                        (const void*)k_turb_yfwd<4>})
+    TB_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   turb_set(T.get(), q0);
   return T.release();
 }
@@ -534,14 +597,11 @@ tb_turb* tb::turb_create(tb_context* ctx, const tb_problem_desc& d, const double
 // the plan's own (non-blocking) stream, so the next step is ordered after it.
 void tb::turb_set(tb_turb* T, const double* q0) {
   const size_t spec = (size_t)T->Kx * T->Ny * sizeof(float2);
-  std::vector<float2> h((size_t)T->Kx * T->Ny);
-  for (int ky = 0; ky < T->Ny; ++ky)
-    for (int kx = 0; kx < T->Kx; ++kx) {
-      const size_t s = (size_t)ky * T->Kx + kx;
-      h[(size_t)kx * T->Ny + ky] = make_float2((float)q0[2 * s], (float)q0[2 * s + 1]);
-    }
-  TB_CUDA_TRY(cudaStreamSynchronize(T->st));  // no step still reads the buffers
-  TB_CUDA_TRY(cudaMemcpyAsync(T->Q[0].p, h.data(), spec, cudaMemcpyHostToDevice, T->st));
+  double2* stage = T->mix.as<double2>();  // free between steps
+  TB_CUDA_TRY(cudaMemcpyAsync(stage, q0, 2 * spec, cudaMemcpyHostToDevice, T->st));
+  k_turb_state<false><<<dim3((T->Kx + 31) / 32, (T->Ny + 31) / 32), dim3(32, 8), 0, T->st>>>(T->Q[0].as<float2>(), stage,
+                                                                                            T->Kx, T->Ny);
+  TB_CUDA_TRY(cudaGetLastError());
   TB_CUDA_TRY(cudaMemsetAsync(T->Q[1].p, 0, spec, T->st));
   if (T->Fb.p) TB_CUDA_TRY(cudaMemsetAsync(T->Fb.p, 0, spec, T->st));
   TB_CUDA_TRY(cudaStreamSynchronize(T->st));
@@ -584,8 +644,8 @@ void tb::turb_launch_steps(tb_turb* T, double dt, int steps) {
 }
 
 size_t tb::turb_device_bytes(const tb_turb* T) {
-  size_t b = T->Q[0].bytes + T->Q[1].bytes + T->Fb.bytes + T->mix.bytes + T->mixT.bytes + T->pm.bytes +
-             T->pmT.bytes + T->ptx.bytes + T->pty.bytes;
+  size_t b = T->Q[0].bytes + T->Q[1].bytes + T->Fb.bytes + T->mix.bytes + T->pm.bytes + T->twx.bytes + T->twy.bytes +
+             T->posy.bytes;
   for (int i = 0; i < 4; ++i) b += T->Ys[i].bytes + T->Fs[i].bytes;
   return b;
 }
@@ -593,16 +653,12 @@ size_t tb::turb_device_bytes(const tb_turb* T) {
 size_t tb::turb_field_doubles(const tb_turb* T) { return 2 * (size_t)T->Kx * T->Ny; }
 
 void tb::turb_fetch(tb_turb* T, double* host) {
-  std::vector<float2> h((size_t)T->Kx * T->Ny);
-  TB_CUDA_TRY(cudaMemcpyAsync(h.data(), T->Q[T->cur].p, h.size() * sizeof(float2), cudaMemcpyDeviceToHost, T->st));
+  double2* stage = T->mix.as<double2>();  // free between steps
+  k_turb_state<true><<<dim3((T->Kx + 31) / 32, (T->Ny + 31) / 32), dim3(32, 8), 0, T->st>>>(T->Q[T->cur].as<float2>(),
+                                                                                           stage, T->Kx, T->Ny);
+  TB_CUDA_TRY(cudaGetLastError());
+  TB_CUDA_TRY(cudaMemcpyAsync(host, stage, (size_t)T->Kx * T->Ny * sizeof(double2), cudaMemcpyDeviceToHost, T->st));
   TB_CUDA_TRY(cudaStreamSynchronize(T->st));
-  for (int ky = 0; ky < T->Ny; ++ky)
-    for (int kx = 0; kx < T->Kx; ++kx) {
-      const float2 v = h[(size_t)kx * T->Ny + ky];
-      const size_t s = (size_t)ky * T->Kx + kx;
-      host[2 * s] = v.x;
-      host[2 * s + 1] = v.y;
-    }
 }
 
 extern "C" {

@@ -253,7 +253,7 @@ __device__ C* fft_multi(C* a, C* b, int NA, int Ms, const FftPlan& fp, const C* 
 // Swizzle keyed to the element size: the low bits of an index are XORed with
 // the next ones over a group of 128 bytes (8 double2 or 16 float2), so that the
 // stride-R stores of a pass and the unit-stride loads both spread over all
-// banks.  Buffers are padded to whole groups (pad_swz).
+// banks.  Buffers are padded to whole groups.
 template <class C>
 struct SwzGroup;
 template <>
@@ -265,240 +265,9 @@ struct SwzGroup<float2> {
   static constexpr int shift = 4;
 };
 template <class C>
-__host__ __device__ constexpr int pad_swz(int n) {
-  return (n + (1 << SwzGroup<C>::shift) - 1) & ~((1 << SwzGroup<C>::shift) - 1);
-}
-template <class C>
 __device__ __forceinline__ int sidx(int i) {
   constexpr int s = SwzGroup<C>::shift;
   return i ^ ((i >> s) & ((1 << s) - 1));
-}
-
-// Radix of stage s of the Stockham plan of length n (radices 8, then 4, 2, 3:
-// the order make_fft_plan uses), 0 past the last stage.
-__host__ __device__ constexpr int ct_radix(int n, int s) {
-  int k = 0;
-  while (n % 8 == 0) {
-    if (k == s) return 8;
-    n /= 8;
-    ++k;
-  }
-  while (n % 4 == 0) {
-    if (k == s) return 4;
-    n /= 4;
-    ++k;
-  }
-  while (n % 2 == 0) {
-    if (k == s) return 2;
-    n /= 2;
-    ++k;
-  }
-  while (n % 3 == 0) {
-    if (k == s) return 3;
-    n /= 3;
-    ++k;
-  }
-  return 0;
-}
-
-template <int R, class C>
-__device__ __forceinline__ void twiddle_apply(C (&v)[R], C w1) {
-  if constexpr (R == 8) {
-    const C w2 = mul(w1, w1), w4 = mul(w2, w2), w3 = mul(w1, w2);
-    v[1] = mul(v[1], w1);
-    v[2] = mul(v[2], w2);
-    v[3] = mul(v[3], w3);
-    v[4] = mul(v[4], w4);
-    v[5] = mul(v[5], mul(w1, w4));
-    v[6] = mul(v[6], mul(w2, w4));
-    v[7] = mul(v[7], mul(w3, w4));
-  } else if constexpr (R == 4) {
-    const C w2 = mul(w1, w1);
-    v[1] = mul(v[1], w1);
-    v[2] = mul(v[2], w2);
-    v[3] = mul(v[3], mul(w1, w2));
-  } else if constexpr (R == 3) {
-    v[1] = mul(v[1], w1);
-    v[2] = mul(v[2], mul(w1, w1));
-  } else {
-    v[1] = mul(v[1], w1);
-  }
-}
-
-// Compile-time form of pass_batch for a length-N plan (constant divisors and
-// strides, typed swizzle).
-template <int R, int NS, int N, class C>
-__device__ __forceinline__ void pass_ct(const C* __restrict__ in, C* __restrict__ out, const C* __restrict__ pt,
-                                        int sign, int nb, int stride) {
-  constexpr int nR = N / R;
-  for (int t = threadIdx.x; t < nb * nR; t += blockDim.x) {
-    const int q = t / nR, idx = t - q * nR;
-    const int j = idx % NS, k = idx / NS;
-    const C* src = in + (size_t)q * stride;
-    C* dst = out + (size_t)q * stride;
-    C v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[sidx<C>(idx + r * nR)];
-    if constexpr (NS > 1) {
-      C w1 = pt[j];
-      if (sign > 0) w1.y = -w1.y;
-      twiddle_apply<R>(v, w1);
-    }
-    dft_small<R>(v, sign);
-    const int ob = k * NS * R + j;
-#pragma unroll
-    for (int r = 0; r < R; ++r) dst[sidx<C>(ob + r * NS)] = v[r];
-  }
-}
-
-template <int N, int S, int NS, class C>
-__device__ __forceinline__ C* stages_ct(C* in, C* out, const C* __restrict__ pt, int sign, int nb, int stride) {
-  constexpr int R = ct_radix(N, S);
-  if constexpr (R == 0) {
-    return in;
-  } else {
-    pass_ct<R, NS, N>(in, out, pt, sign, nb, stride);
-    __syncthreads();
-    return stages_ct<N, S + 1, NS * R>(out, in, pt + NS, sign, nb, stride);
-  }
-}
-
-// nb CTA-wide length-N transforms (N a compile-time constant) between buffer
-// sets a and b; returns the set holding the results.  Same arithmetic and
-// twiddle tables as fft_batch with the runtime plan of length N.
-template <int N, class C>
-__device__ C* fft_batch_ct(C* a, C* b, int nb, int stride, const C* __restrict__ pt, int sign) {
-  return stages_ct<N, 0, 1>(a, b, pt, sign, nb, stride);
-}
-
-// ---------------------------------------------------------------------------
-// Length-384 transforms in two register passes (384 = 16 x 24, four-step):
-// pass 1 takes, per (transform, n2 < 24), the 16 inputs x[24 n1 + n2] into
-// registers, a 16-point DFT (4 x 4 in registers), the twiddles w^(n2 k1), and
-// stores row k1 of a [16][25] scratch; pass 2 takes, per (transform, k1 < 16),
-// scratch row k1, a 24-point DFT (8 x 3 in registers) and stores X[k1 + 16 k2].
-// Two shared-memory round trips per element instead of the four of the
-// Stockham plan (8, 8, 2, 3).  Buffers in natural order (no swizzle), at least
-// kLen384Buf elements apart.  w: exp(-2 pi i k / 384), k < 384.
-// ---------------------------------------------------------------------------
-constexpr int kLen384Buf = 400;  // 16 rows of 25 (padding spreads the row starts over the banks)
-
-template <class C>
-__device__ __forceinline__ C tw384(const C* __restrict__ w, int k, int sign) {
-  C t = w[k];
-  if (sign > 0) t.y = -t.y;
-  return t;
-}
-
-// In-register DFT of length R1 R2 (natural order in and out); internal
-// twiddles w_{R1 R2}^j = w_384^(j WS) with WS = 384 / (R1 R2).
-template <int R1, int R2, int WS, class C>
-__device__ __forceinline__ void dft_reg(C (&x)[R1 * R2], const C* __restrict__ w, int sign) {
-  C y[R1 * R2];
-#pragma unroll
-  for (int n2 = 0; n2 < R2; ++n2) {
-    C a[R1];
-#pragma unroll
-    for (int n1 = 0; n1 < R1; ++n1) a[n1] = x[R2 * n1 + n2];
-    dft_small<R1>(a, sign);
-#pragma unroll
-    for (int k1 = 0; k1 < R1; ++k1) y[k1 * R2 + n2] = (n2 * k1 == 0) ? a[k1] : mul(a[k1], tw384(w, n2 * k1 * WS, sign));
-  }
-#pragma unroll
-  for (int k1 = 0; k1 < R1; ++k1) {
-    C b[R2];
-#pragma unroll
-    for (int n2 = 0; n2 < R2; ++n2) b[n2] = y[k1 * R2 + n2];
-    dft_small<R2>(b, sign);
-#pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) x[k1 + R1 * k2] = b[k2];
-  }
-}
-
-// nb length-384 transforms, buffer q at a + q * stride (stride >= kLen384Buf),
-// b the scratch set; results in a (returned).  sign -1 forward, +1 inverse,
-// unnormalised.
-template <class C>
-__device__ C* fft384_batch(C* a, C* b, int nb, int stride, const C* __restrict__ w, int sign) {
-  for (int t = threadIdx.x; t < nb * 24; t += blockDim.x) {
-    const int q = t / 24, n2 = t - 24 * q;
-    const C* src = a + (size_t)q * stride;
-    C* dst = b + (size_t)q * stride;
-    C v[16];
-#pragma unroll
-    for (int n1 = 0; n1 < 16; ++n1) v[n1] = src[24 * n1 + n2];
-    dft_reg<4, 4, 24>(v, w, sign);
-#pragma unroll
-    for (int k1 = 0; k1 < 16; ++k1) dst[k1 * 25 + n2] = (k1 == 0 || n2 == 0) ? v[k1] : mul(v[k1], tw384(w, n2 * k1, sign));
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < nb * 16; t += blockDim.x) {
-    const int q = t / 16, k1 = t - 16 * q;
-    const C* src = b + (size_t)q * stride + k1 * 25;
-    C* dst = a + (size_t)q * stride;
-    C v[24];
-#pragma unroll
-    for (int n2 = 0; n2 < 24; ++n2) v[n2] = src[n2];
-    dft_reg<8, 3, 16>(v, w, sign);
-#pragma unroll
-    for (int k2 = 0; k2 < 24; ++k2) dst[k1 + 16 * k2] = v[k2];
-  }
-  __syncthreads();
-  return a;
-}
-
-// Batched form: nb transforms of length fp.n, buffer q at a + q * stride (and
-// b + q * stride), all butterflies of a pass spread over the CTA (typed swizzle).
-template <int R, bool SW, class C>
-__device__ __forceinline__ void pass_batch(const C* __restrict__ in, C* __restrict__ out, int n, int Ns,
-                                           const C* __restrict__ pt, int sign, int nb, int stride) {
-  const int nR = n / R;
-  for (int t = threadIdx.x; t < nb * nR; t += blockDim.x) {
-    const int q = t / nR, idx = t - q * nR;
-    const int j = idx % Ns, k = idx / Ns;
-    const C* src = in + (size_t)q * stride;
-    C* dst = out + (size_t)q * stride;
-    C v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[SW ? sidx<C>(idx + r * nR) : idx + r * nR];
-    if (Ns > 1) {
-      C w1 = pt[j];
-      if (sign > 0) w1.y = -w1.y;
-      twiddle_apply<R>(v, w1);
-    }
-    dft_small<R>(v, sign);
-    const int ob = k * Ns * R + j;
-#pragma unroll
-    for (int r = 0; r < R; ++r) dst[SW ? sidx<C>(ob + r * Ns) : ob + r * Ns] = v[r];
-  }
-}
-
-// nb CTA-wide transforms between buffer sets a and b (buffer q at + q * stride);
-// returns the set holding the results.
-template <bool SW, class C>
-__device__ C* fft_batch(C* a, C* b, int nb, int stride, const FftPlan& fp, const C* __restrict__ pt, int sign) {
-  const int n = fp.n;
-  int Ns = 1;
-  C* in = a;
-  C* out = b;
-  for (int s = 0; s < fp.nstages; ++s) {
-    const int R = fp.radix[s];
-    if (R == 8)
-      pass_batch<8, SW>(in, out, n, Ns, pt, sign, nb, stride);
-    else if (R == 4)
-      pass_batch<4, SW>(in, out, n, Ns, pt, sign, nb, stride);
-    else if (R == 2)
-      pass_batch<2, SW>(in, out, n, Ns, pt, sign, nb, stride);
-    else
-      pass_batch<3, SW>(in, out, n, Ns, pt, sign, nb, stride);
-    __syncthreads();
-    C* t = in;
-    in = out;
-    out = t;
-    pt += Ns;
-    Ns *= R;
-  }
-  return in;
 }
 
 // Number of per-pass twiddle entries of a plan (sum of the passes' Ns).

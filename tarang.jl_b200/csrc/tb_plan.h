@@ -176,8 +176,8 @@ struct tb_plan {
   // 3D RHS program (element type of the RHS precision): Cartesian copy of the
   // state, Chebyshev half planes, y-transformed factors, x-pass products,
   // y-forward output, per-pass twiddles of the padded x / y plans
-  DevBuf kmag, Xc, G3, mix3, pm3, H3, ptwX, ptwY;
-  FftPlan fpMy{};
+  DevBuf kmag, Xc, G3, mix3, pm3, H3, ptwX, ptwY, posY;
+  RPlan rpX{}, rpY{};  // in-place passes of the padded x and y lengths
   // 3D field transforms and state I/O: plan and per-pass twiddles of the Ny
   // transform, one complex plane of scratch
   FftPlan fpNy{};

@@ -19,15 +19,15 @@
 //   k3_prep   state -> Cartesian b, u_x, u_y, u_z (RHS precision)
 //   GEMM      Chebyshev backward: values and z-derivatives as even/odd half
 //             planes over the z grid (tensor-core DMMA in FP64, SIMT in FP32)
-//   k3_yinv   per (kx, z pair): value, d_y and d_z of each field with the grid
+//   k3_yinv   per (group of kx, field, z pair): value, d_y and d_z with the grid
 //             round trip's Hermitian projection of the kx = 0 / Nyquist columns,
-//             the x Nyquist split, y padding with the Nyquist split, 12 inverse
-//             FFTs along y
+//             the x Nyquist split, y padding with the Nyquist split, inverse
+//             FFTs along y, stored as rows over kx
 //   k3_xpass  per (y rows, z): d_x from the x bins, 15 real inverse FFTs along
 //             x (8 packed), the 4 products, 2 packed forward FFTs, x truncation
 //             with the Nyquist fold
-//   k3_yfwd   per (kx, z): 4 forward FFTs along y, Nyquist fold, truncation,
-//             scale, rotation of the momentum rows
+//   k3_yfwd   per (group of kx, z): 4 forward FFTs along y, Nyquist fold,
+//             truncation, scale, rotation of the momentum rows
 //   GEMM      Chebyshev forward into C^(2) rows (S fwd) of the stage vector.
 #include <cuda_runtime.h>
 
@@ -36,7 +36,7 @@
 #include <type_traits>
 #include <vector>
 
-#include "tb_fft.cuh"
+#include "tb_fftr.cuh"
 #include "tb_internal.h"
 #include "tb_kernels.cuh"
 #include "tb_plan.h"
@@ -45,14 +45,15 @@ namespace tb {
 namespace {
 
 namespace F = tb::fftg;
+namespace Rp = tb::fftr;
 
 constexpr int kR3Threads = 256;
 
 struct R3Args {
   int Nx, Ny, Nz, Kx, Mx, My, Nk, H;
+  int Kp;  // Kx rounded up to whole 32-byte sectors: row length of the y-transformed arrays
   double kx0, ky0;
-  FftPlan fpx, fpy;
-  int nptx, npty;
+  RPlan rx, ry;
 };
 
 __device__ __forceinline__ int ky_index(int iy, int Ny) { return iy < Ny / 2 ? iy : iy - Ny; }
@@ -87,239 +88,291 @@ __global__ void __launch_bounds__(256) k3_prep(R3Args a, const double2* __restri
   Xc[3 * plane + i] = F::mk<C>((T)uz.x, (T)uz.y);
 }
 
-// The FP32 kernels at the 384-point padded length run the two-pass register
-// transform (natural-order buffers, kLen384Buf apart, twiddle table w^k for
-// k < 384); other compiled lengths the Stockham plan with constant strides,
-// the rest the runtime plan (both on swizzled buffers, per-pass twiddles).
-template <class C, int M>
-constexpr bool kReg384 = std::is_same<C, float2>::value && M == 384;
-
-template <class C, int M>
-__device__ __forceinline__ int bidx(int i) {
-  if constexpr (kReg384<C, M>)
-    return i;
-  else
-    return F::sidx<C>(i);
+// Column buffers of the y kernels: array a's entry i at a * ystride + sw(i); the
+// extra entries put the same entry of neighbouring columns on different banks.
+template <class C>
+__host__ __device__ inline int ystride(int My) {
+  return Rp::rpad<C>(My) + 32 / (int)sizeof(C);
 }
 
-template <class C, int M>
-__host__ __device__ constexpr int buf_len(int m) {
-  return kReg384<C, M> ? F::kLen384Buf : F::pad_swz<C>(m);
-}
-
-// Batched FFT of nb buffers.
-template <int N, class C>
-__device__ __forceinline__ C* fftb(C* a, C* b, int nb, int stride, const FftPlan& fp, const C* __restrict__ pt,
-                                   int sign) {
-  if constexpr (kReg384<C, N>)
-    return F::fft384_batch(a, b, nb, stride, pt, sign);
-  else if constexpr (N > 0)
-    return F::fft_batch_ct<N>(a, b, nb, stride, pt, sign);
-  else
-    return F::fft_batch<true>(a, b, nb, stride, fp, pt, sign);
-}
-
-// Per (kx column ix, z pair j / Nz-1-j).  G: 16 half planes (field f, w) at
-// G + (4 f + w) hplane, w = 0 even values, 1 odd values, 2 even d_z, 3 odd d_z,
-// element (j, m).  Output mix[z][q][ix][y], q = 3 f + kind (value, d_y, d_z).
-template <class C, int MY>
-__global__ void __launch_bounds__(kR3Threads) k3_yinv(R3Args a, const C* __restrict__ G, const C* __restrict__ pty,
-                                                       C* __restrict__ mix) {
+// CW kx columns of one field (blockIdx.y) at the z pair j / Nz-1-j (blockIdx.z).
+// G: 16 half planes (field f, w) at G + (4 f + w) hplane, w = 0 even values, 1
+// odd values, 2 even d_z, 3 odd d_z, element (j, m).  Output mix[z][q][y][kx],
+// q = 3 f + kind (value, d_y, d_z).  The 6 CW transforms (both levels) share the
+// passes; rows leave in groups of CW neighbours (32 bytes at the widest), so
+// the x pass reads whole rows.  Bound by shared-memory traffic.
+template <class C, int CW>
+__global__ void __launch_bounds__(kR3Threads, sizeof(C) == 8 ? 3 : 2)
+    k3_yinv(R3Args a, const C* __restrict__ G, const C* __restrict__ twy, const unsigned short* __restrict__ posy,
+            C* __restrict__ mix) {
   using T = typename F::Real<C>::type;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   C* sm = reinterpret_cast<C*>(sm_raw);
-  const int Ny = a.Ny, My = MY > 0 ? MY : a.My, ix = blockIdx.x, j = blockIdx.y;
-  const int Ms = buf_len<C, MY>(My);
-  C* stg = sm;                    // [16][Ny]
-  C* A = stg + 16 * Ny;           // [12][Ms]
-  C* B = A + 12 * Ms;             // [12][Ms]
-  C* pt = B + 12 * Ms;            // [npty]
+  const int Ny = a.Ny, My = a.My, ix0 = blockIdx.x * CW, f = blockIdx.y, j = blockIdx.z;
+  const int Ms = ystride<C>(My), hy = Ny / 2;
+  C* tw = sm + 6 * CW * Ms;
+  for (int t = threadIdx.x; t < a.ry.ntw; t += blockDim.x) tw[t] = twy[t];
   const size_t hplane = (size_t)a.H * a.Nk;
-  for (int t = threadIdx.x; t < a.npty; t += blockDim.x) pt[t] = pty[t];
-  for (int t = threadIdx.x; t < 16 * Ny; t += blockDim.x) {
-    const int q = t / Ny, iy = t - q * Ny;
-    stg[t] = G[(size_t)q * hplane + (size_t)j * a.Nk + (size_t)ix * Ny + iy];
+  const C* g = G + (size_t)(4 * f) * hplane + (size_t)j * a.Nk;
+  for (int t = threadIdx.x; t < CW * Ny; t += blockDim.x) {
+    const int c = t / Ny, iy = t - c * Ny, ix = ix0 + c;
+    if (ix >= a.Kx) break;
+    C h[4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) h[w] = g[w * hplane + (size_t)ix * Ny + iy];
+    if (ix == 0 || 2 * ix == a.Nx) {
+      // columns whose grid round trip is Hermitian; the factor is a derivative of
+      // the field's round trip, so the projection comes first (it differs from
+      // projecting i ky v at the self-paired ky = -Ny/2 mode)
+      const int ip = iy ? Ny - iy : 0;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const C p = g[w * hplane + (size_t)ix * Ny + ip];
+        h[w] = F::mk<C>((T)0.5 * (h[w].x + p.x), (T)0.5 * (h[w].y - p.y));
+      }
+    }
+    const T xs = (2 * ix == a.Nx) ? (T)0.5 : (T)1.0;  // even-N Nyquist split along x
+    const T kyv = (T)(a.ky0 * ky_index(iy, Ny));
+    const int y = iy <= hy ? iy : My - Ny + iy;
+#pragma unroll
+    for (int lev = 0; lev < 2; ++lev) {
+      const C v = F::scale(lev ? F::sub(h[0], h[1]) : F::add(h[0], h[1]), xs);
+      const C d = F::scale(lev ? F::sub(h[3], h[2]) : F::add(h[2], h[3]), xs);
+      const C out[3] = {v, F::mk<C>(-kyv * v.y, kyv * v.x), d};
+#pragma unroll
+      for (int kind = 0; kind < 3; ++kind) {
+        C* col = sm + ((lev * 3 + kind) * CW + c) * Ms;
+        const C o = iy == hy ? F::scale(out[kind], (T)0.5) : out[kind];
+        col[Rp::sw<C>(y)] = o;
+        if (iy == hy) col[Rp::sw<C>(My - hy)] = o;
+      }
+    }
   }
+  const int gap = My - Ny - 1;  // y bins hy + 1 .. My - hy - 1 are zero
+  for (int t = threadIdx.x; t < gap; t += blockDim.x)
+    for (int arr = 0; arr < 6 * CW; ++arr) sm[arr * Ms + Rp::sw<C>(hy + 1 + t)] = F::mk<C>((T)0, (T)0);
   __syncthreads();
-  const bool edge = (ix == 0) || (2 * ix == a.Nx);  // columns whose grid round trip is Hermitian
-  const T xs = (2 * ix == a.Nx) ? (T)0.5 : (T)1.0;  // even-N Nyquist split along x
-  const int hy = Ny / 2, gap = My - Ny - 1;          // y bins hy+1 .. My-hy-1 stay zero
-  for (int lev = 0; lev < 2; ++lev) {
-    const int zl = lev ? a.Nz - 1 - j : j;
-    // value (kind 0, 1) or z-derivative (kind 2) of field f at grid level zl
-    auto base = [&](int f, int kind, int iy) -> C {
-      const C e = stg[(4 * f + (kind == 2 ? 2 : 0)) * Ny + iy];
-      const C o = stg[(4 * f + (kind == 2 ? 3 : 1)) * Ny + iy];
-      if (kind == 2) return lev ? F::sub(o, e) : F::add(e, o);
-      return lev ? F::sub(e, o) : F::add(e, o);
-    };
-    for (int t = threadIdx.x; t < 12 * gap; t += blockDim.x) {
-      const int q = t / gap, y = hy + 1 + (t - q * gap);
-      A[(size_t)q * Ms + bidx<C, MY>(y)] = F::mk<C>((T)0, (T)0);
-    }
-    for (int t = threadIdx.x; t < 12 * Ny; t += blockDim.x) {
-      const int q = t / Ny, iy = t - q * Ny;
-      const int f = q / 3, kind = q - 3 * f;
-      // the factor is a derivative of the field's grid round trip, so the
-      // projection comes first (it differs from projecting i ky v at the
-      // self-paired ky = -Ny/2 mode)
-      C v = base(f, kind, iy);
-      if (edge) {
-        const C w = base(f, kind, (Ny - iy) % Ny);
-        v = F::mk<C>((T)0.5 * (v.x + w.x), (T)0.5 * (v.y - w.y));
-      }
-      if (kind == 1) {
-        const T kyv = (T)(a.ky0 * ky_index(iy, Ny));
-        v = F::mk<C>(-kyv * v.y, kyv * v.x);  // i ky v
-      }
-      v = F::scale(v, xs);
-      C* col = A + (size_t)q * Ms;
-      if (iy < hy) {
-        col[bidx<C, MY>(iy)] = v;
-      } else if (iy == hy) {
-        const C h = F::scale(v, (T)0.5);
-        col[bidx<C, MY>(hy)] = h;
-        col[bidx<C, MY>(My - hy)] = h;
-      } else {
-        col[bidx<C, MY>(My - Ny + iy)] = v;
-      }
-    }
+  for (int s = 0; s < a.ry.np; ++s) {
+    Rp::pass_any<true, 1>(sm, 6 * CW, Ms, a.ry, s, tw);
     __syncthreads();
-    C* R = fftb<MY>(A, B, 12, Ms, a.fpy, pt, +1);
-    for (int t = threadIdx.x; t < 12 * My; t += blockDim.x) {
-      const int q = t / My, y = t - q * My;
-      mix[(((size_t)zl * 12 + q) * a.Kx + ix) * My + y] = R[(size_t)q * Ms + bidx<C, MY>(y)];
-    }
-    __syncthreads();
+  }
+  for (int t = threadIdx.x; t < CW * My; t += blockDim.x) {
+    const int c = t % CW, y = t / CW;
+    if (ix0 + c >= a.Kx) continue;
+    const int p = Rp::sw<C>(posy[y]);
+#pragma unroll
+    for (int lev = 0; lev < 2; ++lev)
+#pragma unroll
+      for (int kind = 0; kind < 3; ++kind) {
+        const int zl = lev ? a.Nz - 1 - j : j;
+        mix[(((size_t)zl * 12 + 3 * f + kind) * My + y) * a.Kp + ix0 + c] = sm[((lev * 3 + kind) * CW + c) * Ms + p];
+      }
   }
 }
 
-// Per (RR consecutive padded y rows, z level).  mix[z][q][kx][y] ->
-// pm[z][f][kx][y] (f = b, u_x, u_y, u_z; kx < Kx, Nyquist folded).
-// Factors on the x grid (15 real, packed in pairs a + i b): 0 u_x, 1 u_y,
-// 2 u_z, 3..6 d_x f, 7..10 d_y f, 11..14 d_z f (f = b, u_x, u_y, u_z).
-template <class C, int RR, int MX>
-__global__ void __launch_bounds__(RR == 4 ? 2 * kR3Threads : kR3Threads) k3_xpass(R3Args a, const C* __restrict__ mix, const C* __restrict__ ptx,
-                                                        C* __restrict__ pm) {
+// The last inverse pass (radix R) of the eight packed factors of row r, the four
+// products and the first forward pass of the two packed products, in registers;
+// arrays p * RR + r in, products in arrays r (b, u_x) and RR + r (u_y, u_z).
+template <int R, int RR, class C>
+__device__ __forceinline__ void xmiddle3(C* __restrict__ A, int Ms, int n) {
+  using T = typename F::Real<C>::type;
+  const int nb = n / R;
+  for (int item = threadIdx.x; item < RR * nb; item += blockDim.x) {
+    int r = 0, b = item;
+    while (b >= nb) {
+      b -= nb;
+      ++r;
+    }
+    int at[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) at[q] = Rp::sw<C>(b * R + q);
+    T u[R], v[R], w[R];
+    C pa[R], pb[R], z[R];  // products (b, u_x) and (u_y, u_z)
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) z[q] = A[(p * RR + r) * Ms + at[q]];
+      Rp::dft<R, 1>(z);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        // 0 (u_x, u_y)  1 (u_z, d_x b)  2 (d_x u_x, d_x u_y)  3 (d_x u_z, d_y b)
+        // 4 (d_y u_x, d_y u_y)  5 (d_y u_z, d_z b)  6 (d_z u_x, d_z u_y)  7 (d_z u_z, -)
+        if (p == 0) {
+          u[q] = z[q].x;
+          v[q] = z[q].y;
+        } else if (p == 1) {
+          w[q] = z[q].x;
+          pa[q].x = Rp::mul_rn(u[q], z[q].y);
+        } else if (p == 2) {
+          pa[q].y = Rp::mul_rn(u[q], z[q].x);
+          pb[q].x = Rp::mul_rn(u[q], z[q].y);
+        } else if (p == 3) {
+          pb[q].y = Rp::mul_rn(u[q], z[q].x);
+          pa[q].x = fma(v[q], z[q].y, pa[q].x);
+        } else if (p == 4) {
+          pa[q].y = fma(v[q], z[q].x, pa[q].y);
+          pb[q].x = fma(v[q], z[q].y, pb[q].x);
+        } else if (p == 5) {
+          pb[q].y = fma(v[q], z[q].x, pb[q].y);
+          pa[q].x = fma(w[q], z[q].y, pa[q].x);
+        } else if (p == 6) {
+          pa[q].y = fma(w[q], z[q].x, pa[q].y);
+          pb[q].x = fma(w[q], z[q].y, pb[q].x);
+        } else {
+          pb[q].y = fma(w[q], z[q].x, pb[q].y);
+        }
+      }
+    }
+    Rp::dft<R, -1>(pa);
+    Rp::dft<R, -1>(pb);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      A[r * Ms + at[q]] = pa[q];
+      A[(RR + r) * Ms + at[q]] = pb[q];
+    }
+  }
+}
+
+// Per (RR consecutive padded y rows, z level).  mix[z][q][y][kx] ->
+// pm[z][f][y][kx] (f = b, u_x, u_y, u_z; kx < Kx, Nyquist folded): the packed
+// spectra of the 15 factors straight from the rows, dif passes over 8 RR
+// arrays in one buffer, xmiddle3, dit passes over 2 RR arrays.  Bound by
+// shared-memory traffic; at 384 points an entry makes 5 accesses a factor
+// where the two-buffer Stockham form with staged spectra made 9.
+template <class C, int RR>
+__global__ void __launch_bounds__(kR3Threads, sizeof(C) == 8 ? 3 : 2)
+    k3_xpass(R3Args a, const C* __restrict__ mix, const C* __restrict__ twx, C* __restrict__ pm) {
   using T = typename F::Real<C>::type;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   C* sm = reinterpret_cast<C*>(sm_raw);
-  const int Mx = MX > 0 ? MX : a.Mx, Kx = a.Kx, My = a.My, hN = a.Nx / 2;
-  const int y0 = blockIdx.x * RR, z = blockIdx.y;
-  const int Ms = buf_len<C, MX>(Mx);
-  constexpr int NB = 8 * RR;
-  C* Z = sm;              // [NB][Ms]
-  C* S = Z + NB * Ms;     // [NB][Ms]
-  C* pt = S + NB * Ms;    // [nptx]
-  for (int t = threadIdx.x; t < a.nptx; t += blockDim.x) pt[t] = ptx[t];
-  // 1. half spectra of the 15 factors, [r][factor][k < Kx], staged in S (DC and
-  // Nyquist kept real, as the factors' own irfft on Nx points does)
-  C* hs = S;
-  for (int t = threadIdx.x; t < 12 * Kx * RR; t += blockDim.x) {
-    const int r = t % RR, rest = t / RR;
-    const int k = rest % Kx, q = rest / Kx;
-    C v = mix[(((size_t)z * 12 + q) * Kx + k) * My + y0 + r];
-    const bool edge = (k == 0 || k == hN);
-    if (edge) v.y = (T)0;
-    const int f = q / 3, kind = q - 3 * f;
-    C* row = hs + (size_t)r * 15 * Kx;
-    if (kind == 0) {
-      if (f > 0) row[(size_t)(f - 1) * Kx + k] = v;
-      const T kk = (T)(a.kx0 * k);
-      row[(size_t)(3 + f) * Kx + k] = edge ? F::mk<C>((T)0, (T)0) : F::mk<C>(-kk * v.y, kk * v.x);  // i kx v
-    } else {
-      row[(size_t)((kind == 1 ? 7 : 11) + f) * Kx + k] = v;
+  const int Mx = a.Mx, My = a.My, hN = a.Nx / 2, y0 = blockIdx.x * RR, z = blockIdx.y;
+  const int Ms = Rp::rpad<C>(Mx);
+  C* tw = sm + 8 * RR * Ms;
+  for (int t = threadIdx.x; t < a.rx.ntw; t += blockDim.x) tw[t] = twx[t];
+  const size_t rowq = (size_t)My * a.Kp;  // one factor's rows of a level
+  const C* in = mix + (size_t)z * 12 * rowq + (size_t)y0 * a.Kp;
+  // bin k of the 15 factors of row r from the 12 rows (value, d_y, d_z of b, u_x,
+  // u_y, u_z), packed a + i b: A + i B at k, conj(A) + i conj(B) at Mx - k
+  auto put = [&](int r, int k, const C (&v)[12], T kk) {
+    auto dx = [&](int f) { return F::mk<C>(Rp::mul_rn(-kk, v[3 * f].y), Rp::mul_rn(kk, v[3 * f].x)); };
+    const C zero = F::mk<C>((T)0, (T)0);
+    const C A[8] = {v[3], v[9], dx(1), dx(3), v[4], v[10], v[5], v[11]};
+    const C B[8] = {v[6], dx(0), dx(2), v[1], v[7], v[2], v[8], zero};
+    const int at = Rp::sw<C>(k), am = Rp::sw<C>(k ? Mx - k : 0);
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      C* dst = sm + (p * RR + r) * Ms;
+      dst[at] = F::mk<C>(A[p].x - B[p].y, A[p].y + B[p].x);
+      if (k > 0) dst[am] = F::mk<C>(A[p].x + B[p].y, -A[p].y + B[p].x);
     }
-  }
-  __syncthreads();
-  // 2. packed spectra: Z[p] = spectrum of factor 2p + i factor 2p+1 on Mx points
-  const int nh = Mx / 2 + 1;
-  for (int t = threadIdx.x; t < RR * 8 * nh; t += blockDim.x) {
-    const int r = t % RR, rest = t / RR;
-    const int k = rest % nh, p = rest / nh;
-    const C* row = hs + (size_t)r * 15 * Kx;
-    const C A = k < Kx ? row[(size_t)(2 * p) * Kx + k] : F::mk<C>((T)0, (T)0);
-    const C B = (k < Kx && p < 7) ? row[(size_t)(2 * p + 1) * Kx + k] : F::mk<C>((T)0, (T)0);
-    C* dst = Z + (size_t)(r * 8 + p) * Ms;
-    // spectrum of a + i b: A + i B at k, conj(A) + i conj(B) at Mx - k
-    dst[bidx<C, MX>(k)] = F::mk<C>(A.x - B.y, A.y + B.x);
-    if (k > 0 && k < Mx / 2) dst[bidx<C, MX>(Mx - k)] = F::mk<C>(A.x + B.y, -A.y + B.x);
-  }
-  __syncthreads();
-  C* Rg = fftb<MX>(Z, S, NB, Ms, a.fpx, pt, +1);
-  C* W = (Rg == Z) ? S : Z;
-  for (int t = threadIdx.x; t < RR * Mx; t += blockDim.x) {
-    const int r = t / Mx, x = t - r * Mx;
-    const int i = bidx<C, MX>(x);
-    const C* g = Rg + (size_t)r * 8 * Ms;
-    const C z0 = g[i], z1 = g[Ms + i], z2 = g[2 * Ms + i], z3 = g[3 * Ms + i];
-    const C z4 = g[4 * Ms + i], z5 = g[5 * Ms + i], z6 = g[6 * Ms + i], z7 = g[7 * Ms + i];
-    const T ux = z0.x, uy = z0.y, uz = z1.x;
-    const T pb = ux * z1.y + uy * z3.y + uz * z5.y;   // d_x b, d_y b, d_z b
-    const T pu = ux * z2.x + uy * z4.x + uz * z6.x;   // d_x u_x, d_y u_x, d_z u_x
-    const T pv = ux * z2.y + uy * z4.y + uz * z6.y;   // d_x u_y, d_y u_y, d_z u_y
-    const T pw = ux * z3.x + uy * z5.x + uz * z7.x;   // d_x u_z, d_y u_z, d_z u_z
-    W[(size_t)(2 * r) * Ms + i] = F::mk<C>(pb, pu);
-    W[(size_t)(2 * r + 1) * Ms + i] = F::mk<C>(pv, pw);
-  }
-  __syncthreads();
-  C* Fq = fftb<MX>(W, Rg, 2 * RR, Ms, a.fpx, pt, -1);
-  for (int t = threadIdx.x; t < RR * 2 * Kx; t += blockDim.x) {
-    const int r = t % RR, rest = t / RR;
-    const int k = rest % Kx, h = rest / Kx;
-    const C* buf = Fq + (size_t)(2 * r + h) * Ms;
-    const C c = buf[bidx<C, MX>(k)], cm = buf[bidx<C, MX>((Mx - k) % Mx)];
-    // first: (c + conj(cm))/2, second: (c - conj(cm))/(2i)
-    C o1 = F::mk<C>((T)0.5 * (c.x + cm.x), (T)0.5 * (c.y - cm.y));
-    C o2 = F::mk<C>((T)0.5 * (c.y + cm.y), (T)-0.5 * (c.x - cm.x));
-    if (k == 0) {
-      o1.y = (T)0;
-      o2.y = (T)0;
-    } else if (k == hN) {  // fold of the -Nx/2 image: 2 Re
-      o1 = F::mk<C>((T)2 * o1.x, (T)0);
-      o2 = F::mk<C>((T)2 * o2.x, (T)0);
+  };
+  for (int t = threadIdx.x; t < RR * hN; t += blockDim.x) {
+    int r = 0, k = t;
+    while (k >= hN) {
+      k -= hN;
+      ++r;
     }
-    pm[(((size_t)z * 4 + 2 * h) * Kx + k) * My + y0 + r] = o1;
-    pm[(((size_t)z * 4 + 2 * h + 1) * Kx + k) * My + y0 + r] = o2;
+    C v[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) v[q] = in[q * rowq + (size_t)r * a.Kp + k];
+    if (k == 0)  // DC kept real, as the factors' own irfft on Nx points does
+#pragma unroll
+      for (int q = 0; q < 12; ++q) v[q].y = (T)0;
+    put(r, k, v, (T)(a.kx0 * k));
+  }
+  if (threadIdx.x < RR) {  // the Nyquist bin, kept real, no x derivative
+    const int r = threadIdx.x;
+    C v[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) v[q] = F::mk<C>(in[q * rowq + (size_t)r * a.Kp + hN].x, (T)0);
+    put(r, hN, v, (T)0);
+  }
+  for (int k = hN + 1 + threadIdx.x; k < Mx - hN; k += blockDim.x) {
+    const int at = Rp::sw<C>(k);
+    for (int arr = 0; arr < 8 * RR; ++arr) sm[arr * Ms + at] = F::mk<C>((T)0, (T)0);
+  }
+  __syncthreads();
+  const int last = a.rx.np - 1;
+  for (int s = 0; s < last; ++s) {
+    Rp::pass_any<true, 1>(sm, 8 * RR, Ms, a.rx, s, tw);
+    __syncthreads();
+  }
+  switch (a.rx.R[last]) {  // at most kLastX
+    case 4: xmiddle3<4, RR>(sm, Ms, Mx); break;
+    case 3: xmiddle3<3, RR>(sm, Ms, Mx); break;
+    default: xmiddle3<2, RR>(sm, Ms, Mx); break;
+  }
+  __syncthreads();
+  for (int s = last - 1; s >= 0; --s) {
+    Rp::pass_any<false, -1>(sm, 2 * RR, Ms, a.rx, s, tw);
+    __syncthreads();
+  }
+  C* out = pm + (size_t)z * 4 * rowq + (size_t)y0 * a.Kp;
+  for (int t = threadIdx.x; t < RR * a.Kx; t += blockDim.x) {
+    int r = 0, k = t;
+    while (k >= a.Kx) {
+      k -= a.Kx;
+      ++r;
+    }
+    const int at = Rp::sw<C>(k), am = Rp::sw<C>(k ? Mx - k : 0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const C* buf = sm + (h * RR + r) * Ms;
+      const C c = buf[at], cm = buf[am];
+      // first: (c + conj(cm))/2, second: (c - conj(cm))/(2i)
+      C o1 = F::mk<C>((T)0.5 * (c.x + cm.x), (T)0.5 * (c.y - cm.y));
+      C o2 = F::mk<C>((T)0.5 * (c.y + cm.y), (T)-0.5 * (c.x - cm.x));
+      if (k == 0) {
+        o1.y = (T)0;
+        o2.y = (T)0;
+      } else if (k == hN) {  // fold of the -Nx/2 image: 2 Re
+        o1 = F::mk<C>((T)2 * o1.x, (T)0);
+        o2 = F::mk<C>((T)2 * o2.x, (T)0);
+      }
+      out[(2 * h) * rowq + (size_t)r * a.Kp + k] = o1;
+      out[(2 * h + 1) * rowq + (size_t)r * a.Kp + k] = o2;
+    }
   }
 }
 
-// Per (kx column ix, z level): forward FFTs along y of the 4 products, y
+// CW kx columns at one z level: forward FFTs along y of the 4 products, y
 // Nyquist fold and truncation, F = -P / (Nx Ny Mx My), rotation of the
 // horizontal momentum rows; out[f][z][m] for f = b, u_par, u_z, u_perp.
-template <class C, int MY>
-__global__ void __launch_bounds__(kR3Threads) k3_yfwd(R3Args a, const C* __restrict__ pm, const C* __restrict__ pty,
-                                                       C* __restrict__ out) {
+template <class C, int CW>
+__global__ void __launch_bounds__(kR3Threads, sizeof(C) == 8 ? 3 : 2)
+    k3_yfwd(R3Args a, const C* __restrict__ pm, const C* __restrict__ twy, const unsigned short* __restrict__ posy,
+            C* __restrict__ out) {
   using T = typename F::Real<C>::type;
   extern __shared__ __align__(16) unsigned char sm_raw[];
   C* sm = reinterpret_cast<C*>(sm_raw);
-  const int Ny = a.Ny, My = MY > 0 ? MY : a.My, ix = blockIdx.x, z = blockIdx.y;
-  const int Ms = buf_len<C, MY>(My);
-  C* A = sm;
-  C* B = A + 4 * Ms;
-  C* pt = B + 4 * Ms;
-  for (int t = threadIdx.x; t < a.npty; t += blockDim.x) pt[t] = pty[t];
-  for (int t = threadIdx.x; t < 4 * My; t += blockDim.x) {
-    const int f = t / My, y = t - f * My;
-    A[(size_t)f * Ms + bidx<C, MY>(y)] = pm[(((size_t)z * 4 + f) * a.Kx + ix) * My + y];
+  const int Ny = a.Ny, My = a.My, ix0 = blockIdx.x * CW, z = blockIdx.y;
+  const int Ms = ystride<C>(My), hy = Ny / 2;
+  C* tw = sm + 4 * CW * Ms;
+  for (int t = threadIdx.x; t < a.ry.ntw; t += blockDim.x) tw[t] = twy[t];
+  const C* in = pm + (size_t)z * 4 * My * a.Kp + ix0;
+  for (int t = threadIdx.x; t < CW * My; t += blockDim.x) {  // columns past Kx read the row padding
+    const int c = t % CW, y = t / CW, at = Rp::sw<C>(y);
+#pragma unroll
+    for (int f = 0; f < 4; ++f) sm[(f * CW + c) * Ms + at] = in[((size_t)f * My + y) * a.Kp + c];
   }
   __syncthreads();
-  const C* Q = fftb<MY>(A, B, 4, Ms, a.fpy, pt, -1);
+  for (int s = 0; s < a.ry.np; ++s) {
+    Rp::pass_any<true, -1>(sm, 4 * CW, Ms, a.ry, s, tw);
+    __syncthreads();
+  }
   const double sc = -1.0 / ((double)a.Nx * (double)Ny * (double)a.Mx * (double)My);
   const size_t plane = (size_t)a.Nz * a.Nk;
-  for (int iy = threadIdx.x; iy < Ny; iy += blockDim.x) {
+  for (int t = threadIdx.x; t < CW * Ny; t += blockDim.x) {
+    const int c = t / Ny, iy = t - c * Ny, ix = ix0 + c;
+    if (ix >= a.Kx) break;
+    const int p = Rp::sw<C>(posy[iy <= hy ? iy : My - Ny + iy]);
+    const int pf = Rp::sw<C>(posy[My - hy]);
     double2 v[4];
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-      const C* col = Q + (size_t)f * Ms;
-      C r;
-      if (2 * iy < Ny) {
-        r = col[bidx<C, MY>(iy)];
-      } else if (2 * iy == Ny) {
-        r = F::add(col[bidx<C, MY>(Ny / 2)], col[bidx<C, MY>(My - Ny / 2)]);
-      } else {
-        r = col[bidx<C, MY>(My - Ny + iy)];
-      }
+      const C* col = sm + (f * CW + c) * Ms;
+      C r = col[p];
+      if (iy == hy) r = F::add(r, col[pf]);
       v[f] = make_double2(sc * (double)r.x, sc * (double)r.y);
     }
     double cx, cy;
@@ -562,59 +615,50 @@ R3Args args_of(const tb_plan* P) {
   a.H = P->Nz / 2;
   a.kx0 = P->k0;
   a.ky0 = P->k0y;
-  a.fpx = P->fpM;
-  a.fpy = P->fpMy;
-  // the FP32 384-point transform reads the full table exp(-2 pi i k/384)
-  a.nptx = (P->mixed && P->M == 384) ? 384 : F::pass_twiddle_count(P->fpM);
-  a.npty = (P->mixed && P->My == 384) ? 384 : F::pass_twiddle_count(P->fpMy);
+  a.Kp = (P->Kx + 3) / 4 * 4;
+  a.rx = P->rpX;
+  a.ry = P->rpY;
   return a;
 }
 
-// Buffer length of the transform kernels for padded length m (see buf_len).
 template <class C>
-size_t buf_len_host(int m) {
-  return (std::is_same<C, float2>::value && m == 384) ? (size_t)F::kLen384Buf : (size_t)F::pad_swz<C>(m);
+size_t yinv_smem(const R3Args& a, int cw) {
+  return ((size_t)6 * cw * ystride<C>(a.My) + a.ry.ntw) * sizeof(C);
+}
+template <class C>
+size_t xpass_smem(const R3Args& a, int rr) {
+  return ((size_t)8 * rr * Rp::rpad<C>(a.Mx) + a.rx.ntw) * sizeof(C);
+}
+template <class C>
+size_t yfwd_smem(const R3Args& a, int cw) {
+  return ((size_t)4 * cw * ystride<C>(a.My) + a.ry.ntw) * sizeof(C);
 }
 
+// kx columns a block of the y kernels: 32 bytes of a row where two blocks then
+// share an SM, fewer at long My.
 template <class C>
-size_t yinv_smem(const R3Args& a) {
-  const size_t Ms = buf_len_host<C>(a.My);
-  return (16 * (size_t)a.Ny + 24 * Ms + (size_t)a.npty) * sizeof(C);
-}
-template <class C, int RR>
-size_t xpass_smem(const R3Args& a) {
-  const size_t Ms = buf_len_host<C>(a.Mx);
-  return (16 * RR * Ms + (size_t)a.nptx) * sizeof(C);
-}
-template <class C>
-size_t yfwd_smem(const R3Args& a) {
-  const size_t Ms = buf_len_host<C>(a.My);
-  return (8 * Ms + (size_t)a.npty) * sizeof(C);
+int columns_per_block(const R3Args& a) {
+  int cw = 32 / (int)sizeof(C);
+  while (cw > 1 && 2 * yinv_smem<C>(a, cw) > 227 * 1024) cw /= 2;
+  return cw;
 }
 
-// Rows per x-pass CTA: 2 in FP32, 1 in FP64 (same shared memory).
-template <class C>
-struct XRows;
-template <>
-struct XRows<float2> {
-  static constexpr int value = 2;
-};
-template <>
-struct XRows<double2> {
-  static constexpr int value = 1;
-};
+// Largest radix of the last x pass: xmiddle3 holds nine such runs in registers.
+constexpr int kLastX = 4;
 
-// Padded transform length with compiled plans (the 256-point grids of the 3D
-// benchmark configuration); other lengths run the runtime plan.
-constexpr int kFixedLen = 384;
+// The grids the 3D transforms are offered for: padded lengths of which 24 (y) and
+// 16 per row (x) buffers and 16 y columns fit one SM's shared memory.
+template <class C>
+bool sizes_ok(const R3Args& a, int rr) {
+  auto pad = [](int n) { return (size_t)(n + 7) / 8 * 8; };
+  return (16 * (size_t)a.Ny + 24 * pad(a.My)) * sizeof(C) <= 224 * 1024 && 16 * rr * pad(a.Mx) * sizeof(C) <= 224 * 1024;
+}
 
 template <class C>
 void set_limits(int bytes) {
-  const void* fns[] = {(const void*)k3_yinv<C, 0>,         (const void*)k3_yinv<C, kFixedLen>,
-                       (const void*)k3_xpass<C, 1, 0>,    (const void*)k3_xpass<C, 1, kFixedLen>,
-                       (const void*)k3_xpass<C, 2, 0>,    (const void*)k3_xpass<C, 2, kFixedLen>,
-                       (const void*)k3_xpass<C, 4, 0>,    (const void*)k3_xpass<C, 4, kFixedLen>,
-                       (const void*)k3_yfwd<C, 0>,         (const void*)k3_yfwd<C, kFixedLen>};
+  const void* fns[] = {(const void*)k3_yinv<C, 1>,  (const void*)k3_yinv<C, 2>,  (const void*)k3_yinv<C, 4>,
+                       (const void*)k3_xpass<C, 1>, (const void*)k3_xpass<C, 2>, (const void*)k3_xpass<C, 4>,
+                       (const void*)k3_yfwd<C, 1>,  (const void*)k3_yfwd<C, 2>,  (const void*)k3_yfwd<C, 4>};
   for (const void* fn : fns) TB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
@@ -622,20 +666,26 @@ void set_limits(int bytes) {
 template <class C>
 bool xrows_ok(const tb_plan* P, const R3Args& a, int rr) {
   if (rr != 1 && rr != 2 && rr != 4) return false;
-  if (P->My % rr) return false;
-  const size_t Ms = buf_len_host<C>(a.Mx);
-  return (16 * (size_t)rr * Ms + (size_t)a.nptx) * sizeof(C) <= 227 * 1024;
+  return P->My % rr == 0 && sizes_ok<C>(a, rr);
 }
 
-// Four rows per CTA run with 512 threads (one CTA per SM by shared memory):
-// the staged loads then take whole 32-byte sectors (4 consecutive y of FP32
-// complex) where one or two rows take a quarter or half of each.
-template <class C, int RR>
-void launch_xpass(tb_plan* P, const R3Args& a, cudaStream_t st) {
-  auto kern = (P->M == kFixedLen) ? k3_xpass<C, RR, kFixedLen> : k3_xpass<C, RR, 0>;
-  const int threads = RR == 4 ? 2 * kR3Threads : kR3Threads;
-  kern<<<dim3(P->My / RR, P->Nz), threads, xpass_smem<C, RR>(a), st>>>(a, P->mix3.as<C>(), P->ptwX.as<C>(),
-                                                                       P->pm3.as<C>());
+// Rows per x-pass CTA of a new plan: as many as leave the CTAs an SM that the
+// registers allow (3 in FP32, 2 in FP64).  Short rows gain from sharing passes
+// (event-timed, 1 / 2 / 4 rows: 64x64x32 FP64 52.1, 36.6, 27.1 us, 128x128x64 FP32
+// 150, 105, 85), 384-point FP32 rows are best at 2 (747, 574, 595).
+template <class C>
+int default_xrows(const tb_plan* P, const R3Args& a) {
+  const int ctas = sizeof(C) == 8 ? 3 : 2;
+  for (int rr : {4, 2})
+    if (xrows_ok<C>(P, a, rr) && ctas * xpass_smem<C>(a, rr) <= 227 * 1024) return rr;
+  return 1;
+}
+
+template <class C>
+void launch_xpass(tb_plan* P, const R3Args& a, int rr, cudaStream_t st) {
+  auto kern = rr == 4 ? k3_xpass<C, 4> : rr == 2 ? k3_xpass<C, 2> : k3_xpass<C, 1>;
+  kern<<<dim3(P->My / rr, P->Nz), kR3Threads, xpass_smem<C>(a, rr), st>>>(a, P->mix3.as<C>(), P->ptwX.as<C>(),
+                                                                         P->pm3.as<C>());
 }
 
 inline int pad16(int k) { return (k + 15) / 16 * 16; }
@@ -676,23 +726,17 @@ void enqueue_rhs_t(tb_plan* P, const double2* Xin, double2* out4) {
                                       (w & 1) ? P->Ko : P->Ke, pad16((w & 1) ? P->Ko : P->Ke), GEMM_PARITY, w & 1};
     timed(P, "z_backward_gemm", [&] { launch_gemm_f64(bt, 16, ncol, ncol, ncol, N, P->st); });
   }
-  const bool fy = P->My == kFixedLen, fx = P->M == kFixedLen;
+  const int cw = columns_per_block<C>(a), groups = (P->Kx + cw - 1) / cw;
+  const unsigned short* posy = P->posY.as<unsigned short>();
   timed(P, "rhs3_yinv", [&] {
-    auto kern = fy ? k3_yinv<C, kFixedLen> : k3_yinv<C, 0>;
-    kern<<<dim3(P->Kx, H), kR3Threads, yinv_smem<C>(a), P->st>>>(a, G, P->ptwY.as<C>(), P->mix3.as<C>());
+    auto kern = cw == 4 ? k3_yinv<C, 4> : cw == 2 ? k3_yinv<C, 2> : k3_yinv<C, 1>;
+    kern<<<dim3(groups, 4, H), kR3Threads, yinv_smem<C>(a, cw), P->st>>>(a, G, P->ptwY.as<C>(), posy, P->mix3.as<C>());
   });
-  (void)fx;
-  timed(P, "rhs3_xpass", [&] {
-    if (P->xrows == 4)
-      launch_xpass<C, 4>(P, a, P->st);
-    else if (P->xrows == 2)
-      launch_xpass<C, 2>(P, a, P->st);
-    else
-      launch_xpass<C, 1>(P, a, P->st);
-  });
+  timed(P, "rhs3_xpass", [&] { launch_xpass<C>(P, a, P->xrows, P->st); });
   timed(P, "rhs3_yfwd", [&] {
-    auto kern = fy ? k3_yfwd<C, kFixedLen> : k3_yfwd<C, 0>;
-    kern<<<dim3(P->Kx, N), kR3Threads, yfwd_smem<C>(a), P->st>>>(a, P->pm3.as<C>(), P->ptwY.as<C>(), P->H3.as<C>());
+    auto kern = cw == 4 ? k3_yfwd<C, 4> : cw == 2 ? k3_yfwd<C, 2> : k3_yfwd<C, 1>;
+    kern<<<dim3(groups, N), kR3Threads, yfwd_smem<C>(a, cw), P->st>>>(a, P->pm3.as<C>(), P->ptwY.as<C>(), posy,
+                                                                     P->H3.as<C>());
   });
   const C* H3 = P->H3.as<C>();
   if constexpr (f32) {
@@ -725,20 +769,21 @@ void enqueue_rhs_t(tb_plan* P, const double2* Xin, double2* out4) {
 
 template <class C>
 void setup_t(tb_plan* P) {
-  constexpr int RR = XRows<C>::value;
+  TB_REQUIRE(make_rplan(P->M, sizeof(C), &P->rpX, 20, kLastX) && make_rplan(P->My, sizeof(C), &P->rpY, 16), TB_ENOTSUPPORTED,
+             "Nx and Ny must be of the form 2^a 3^b");
   const R3Args a = args_of(P);
-  TB_REQUIRE(P->My % RR == 0, TB_ENOTSUPPORTED, "padded Ny must be a multiple of the x-pass rows");
   const size_t lim = 227 * 1024;
-  TB_REQUIRE(yinv_smem<C>(a) <= lim && xrows_ok<C>(P, a, RR) && yfwd_smem<C>(a) <= lim, TB_ENOTSUPPORTED,
-             "Nx or Ny too large for the 3D transform kernels");
-  P->xrows = RR;
+  // (two rows in FP32: the footprint the size limit was set by; My is even)
+  TB_REQUIRE(sizes_ok<C>(a, sizeof(C) == 8 ? 2 : 1), TB_ENOTSUPPORTED, "Nx or Ny too large for the 3D transform kernels");
+  P->xrows = default_xrows<C>(P, a);
   set_limits<C>((int)lim);
   const size_t plane = P->plane, H = (size_t)P->Nz / 2;
   P->Xc.alloc(4 * plane * sizeof(C));
   P->G3.alloc(16 * H * P->Nk * sizeof(C));
-  const size_t slab = (size_t)P->Nz * P->Kx * P->My;
+  const size_t slab = (size_t)P->Nz * P->My * a.Kp;
   P->mix3.alloc(12 * slab * sizeof(C));
   P->pm3.alloc(4 * slab * sizeof(C));
+  TB_CUDA_TRY(cudaMemsetAsync(P->pm3.p, 0, P->pm3.bytes, P->st));  // the row padding stays zero
   P->H3.alloc(4 * plane * sizeof(C));
   if constexpr (std::is_same<C, float2>::value) {
     // the streaming tensor-core form of the z transforms
@@ -756,26 +801,25 @@ void setup_t(tb_plan* P) {
     }
     P->tc32 = P->tc3;  // the default GEMM path of a 3D plan: faster than SIMT at every supported size measured
   }
-  auto table = [&](const FftPlan& fp) {
-    if (std::is_same<C, float2>::value && fp.n == 384) {
-      std::vector<C> t(384);
-      const long double pi = 3.141592653589793238462643383279502884L;
-      for (int k = 0; k < 384; ++k) {
-        t[k].x = (decltype(t[k].x))cosl(-2.0L * pi * k / 384.0L);
-        t[k].y = (decltype(t[k].y))sinl(-2.0L * pi * k / 384.0L);
-      }
-      return t;
+  auto table = [](const RPlan& rp) {
+    const std::vector<double> w = rplan_twiddles(rp);
+    std::vector<C> t(w.size() / 2);
+    for (size_t i = 0; i < t.size(); ++i) {
+      t[i].x = (decltype(t[i].x))w[2 * i];
+      t[i].y = (decltype(t[i].y))w[2 * i + 1];
     }
-    return pass_twiddles_t<C>(fp);
+    return t;
   };
-  upload(P->ptwX, table(P->fpM));
-  upload(P->ptwY, table(P->fpMy));
+  upload(P->ptwX, table(P->rpX));
+  upload(P->ptwY, table(P->rpY));
+  upload(P->posY, rplan_positions(P->rpY));
 }
 
 }  // namespace
 
 void rbc3d_setup(tb_plan* P) {
-  TB_REQUIRE(make_fft_plan(P->My, &P->fpMy) && make_fft_plan(P->Ny, &P->fpNy), TB_ENOTSUPPORTED,
+  FftPlan padded;  // the padded length must be of the same form
+  TB_REQUIRE(make_fft_plan(P->My, &padded) && make_fft_plan(P->Ny, &P->fpNy), TB_ENOTSUPPORTED,
              "Ny must be of the form 2^a 3^b with a padded length 3Ny/2 of the same form");
   upload(P->ptwNy, pass_twiddles_t<double2>(P->fpNy));
   P->tmp3.alloc(std::max(P->plane, (size_t)9 * P->Nk) * sizeof(double2));
@@ -822,7 +866,7 @@ void rbc3d_mx_project(tb_plan* P, double2* MX, cudaStream_t st) {
 
 size_t rbc3d_device_bytes(const tb_plan* P) {
   return P->kmag.bytes + P->Xc.bytes + P->G3.bytes + P->mix3.bytes + P->pm3.bytes + P->H3.bytes + P->ptwX.bytes +
-         P->ptwY.bytes + P->ptwNy.bytes + P->tmp3.bytes;
+         P->ptwY.bytes + P->posY.bytes + P->ptwNy.bytes + P->tmp3.bytes;
 }
 
 namespace {

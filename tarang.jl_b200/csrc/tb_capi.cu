@@ -479,19 +479,108 @@ void join_side(tb_plan* P) {
   TB_CUDA_TRY(cudaStreamWaitEvent(P->st, P->ev_join, 0));
 }
 
+StageTerms stage_args(const tb_plan* P, const double2* X) {
+  StageTerms a{};
+  a.Nz = P->Nz;
+  a.Nk = P->Nk;
+  a.Nkm = P->Nkm;
+  a.Nx = P->Nx;
+  a.s3 = P->s3.as<double>();
+  a.k0 = P->k0;
+  a.s = P->s;
+  a.kappa = P->d.kappa;
+  a.nu = P->d.nu;
+  a.kappa_m = P->kappa_m.as<double>();
+  a.nu_m = P->nu_m.as<double>();
+  a.X = X;
+  return a;
+}
+
+// One RK step of a 2D plan.  Between two solves runs one pass over the stage
+// vectors (launch_stage_rhs: M X_0 or L X_{i-1}, and the combination).  The
+// last stage is solved into X2, so that the final update can form its L X from
+// X2 while it overwrites X.
+void enqueue_rk_step_2d(tb_plan* P, double dt) {
+  const Tableau T = tableau(P->d.timestepper);
+  const double beta = dt * T.AI[1][1];
+  FactorSet* fs = get_factors(P, 0, 1.0, beta);  // done before capture by the caller
+  double2* X = P->X.as<double2>();
+  const double2* Xi = X;  // the state of stage i
+  // the terms that give stage i (i = s: the new state), those of stage i - 1 fused in
+  auto terms = [&](int i) {
+    const double* wE = i < T.s ? T.AE[i] : T.bE;
+    const double* wI = i < T.s ? T.AI[i] : T.bI;
+    StageTerms a = stage_args(P, Xi);
+    auto add = [&](const double2* src, double w) {
+      TB_REQUIRE(a.n < 6, TB_EINVAL, "too many stage terms");
+      a.in[a.n] = src;
+      a.w[a.n++] = w;
+    };
+    if (i == 1) {
+      a.mx = P->MX0.as<double2>();
+      a.w_mx = 1.0;
+    } else {
+      add(P->MX0.as<double2>(), 1.0);
+      a.lx = P->LXP[i - 1].as<double2>();
+      a.w_lx = -dt * wI[i - 1];
+      a.ibeta = 1.0 / beta;
+    }
+    for (int j = 0; j < i; ++j) {
+      if (std::fabs(dt * wE[j]) > 1e-14) add(P->FP[j].as<double2>(), dt * wE[j]);
+      if (j > 0 && j < i - 1 && std::fabs(dt * wI[j]) > 1e-14) add(P->LXP[j].as<double2>(), -dt * wI[j]);
+    }
+    return a;
+  };
+  int nk = 0;
+  for (int i = 0; i < T.s; ++i) {
+    if (i > 0) {
+      timed(P, "stage_lincomb", [&] { launch_stage_rhs(terms(i), P->LXP[i].as<double2>(), P->st); });
+      TauArgs a = tau_args(P, 0, fs, P->LXP[i].as<double2>());
+      if (i == T.s - 1) {
+        a.X = P->X2.as<double2>();
+        a.tau = a.X + (size_t)P->nplanes * P->plane;
+        Xi = a.X;
+      }
+      set_x32(P, &a);
+      if (P->bc_dynamic) {  // wall values at the stage time t_n + c_i dt
+        double ci = 0.0;
+        for (int j = 0; j < i; ++j) ci += T.AE[i][j];
+        a.bcdyn = P->bcdyn.as<double2>();
+        a.t_dev = P->t_dev.as<double>();
+        a.bc_toff = ci * dt;
+      }
+      timed(P, "tau_solve", [&] { launch_tau_solve(a, P->sys[0].tau_parts, P->st); });
+      nk += 2;
+    }
+    // the stage solve (i > 0) has written the FP32 copy of X_i
+    enqueue_rhs(P, Xi, P->FP[i].as<double2>() + P->plane, true, i > 0);
+    nk += P->mixed && i == 0 ? 4 : 3;
+  }
+  timed(P, "rk_final", [&] { launch_stage_final(terms(T.s), X, P->tau.as<double2>(), P->ntau, P->st); });
+  ++nk;
+  if (P->bc_dynamic) {
+    launch_advance_time(P->t_dev.as<double>(), dt, P->st);
+    ++nk;
+  }
+  P->kernels_per_step = nk;
+}
+
 void enqueue_rk_step(tb_plan* P, double dt) {
+  if (P->ndim == 2) {
+    enqueue_rk_step_2d(P, dt);
+    return;
+  }
   const Tableau T = tableau(P->d.timestepper);
   const double gamma = T.AI[1][1];
   const double beta = dt * gamma;
   FactorSet* fs = get_factors(P, 0, 1.0, beta);  // done before capture by the caller
-  FactorSet* fs2 = P->nsys > 1 ? get_factors(P, 1, 1.0, beta) : nullptr;
+  FactorSet* fs2 = get_factors(P, 1, 1.0, beta);
   const long long cnt = (long long)P->nplanes * (long long)P->plane;
   double2* X = P->X.as<double2>();
-  const bool d3 = P->ndim == 3;
   // M X_0 on the side stream, beside the first right-hand side
   fork_side(P);
   timed(P, "mass_apply", [&] {
-    launch_mass_apply(X, P->MX0.as<double2>(), P->s3.as<double>(), P->Nz, P->Nk, P->Nx, 0, P->nf, side(P), P->Nkm);
+    launch_mass_apply(X, P->MX0.as<double2>(), P->s3.as<double>(), P->Nz, P->Nk, P->nf, side(P));
   });
   int nk = 1;
   for (int i = 0; i < T.s; ++i) {
@@ -511,7 +600,6 @@ void enqueue_rk_step(tb_plan* P, double dt) {
       }
       timed(P, "stage_lincomb", [&] { launch_lincomb(lc, P->LXP[i].as<double2>(), cnt, P->st); });
       TauArgs a = tau_args(P, 0, fs, P->LXP[i].as<double2>());
-      set_x32(P, &a);
       if (P->bc_dynamic) {  // wall values at the stage time t_n + c_i dt
         double ci = 0.0;
         for (int j = 0; j < i; ++j) ci += T.AE[i][j];
@@ -520,32 +608,18 @@ void enqueue_rk_step(tb_plan* P, double dt) {
         a.bc_toff = ci * dt;
       }
       timed(P, "tau_solve", [&] { launch_tau_solve(a, P->sys[0].tau_parts, P->st); });
-      if (fs2) {
-        TauArgs a2 = tau_args(P, 1, fs2, P->LXP[i].as<double2>());
-        timed(P, "tau_solve_perp", [&] { launch_tau_solve(a2, P->sys[1].tau_parts, P->st); });
-        ++nk;
-      }
+      TauArgs a2 = tau_args(P, 1, fs2, P->LXP[i].as<double2>());
+      timed(P, "tau_solve_perp", [&] { launch_tau_solve(a2, P->sys[1].tau_parts, P->st); });
       // L X_i = (rhs - M X_i) / beta on the side stream, beside F(X_i)
       fork_side(P);
       timed(P, "lx_finalize", [&] {
-        launch_lx_finalize(P->LXP[i].as<double2>(), X, P->s3.as<double>(), P->Nz, P->Nk, d3 ? 0 : P->Nx, P->k0, P->s,
-                           P->d.kappa, P->d.nu, beta, P->nf, side(P), P->Nkm, P->kappa_m.as<double>(),
-                           P->nu_m.as<double>());
+        launch_lx_finalize(P->LXP[i].as<double2>(), X, P->s3.as<double>(), P->Nz, P->Nk, beta, P->nf, side(P));
       });
-      nk += 3;
-      if (d3) {
-        rbc3d_lx_project(P, P->LXP[i].as<double2>(), beta, side(P));
-        ++nk;
-      }
+      rbc3d_lx_project(P, P->LXP[i].as<double2>(), beta, side(P));
+      nk += 5;
     }
-    if (d3) {
-      rbc3d_enqueue_rhs(P, X, P->FP[i].as<double2>() + P->plane);
-      nk += P->mixed ? 6 : 5;
-    } else {
-      // the stage solve (i > 0) has written the FP32 copy of X_i
-      enqueue_rhs(P, X, P->FP[i].as<double2>() + P->plane, true, i > 0);
-      nk += P->mixed && i == 0 ? 4 : 3;
-    }
+    rbc3d_enqueue_rhs(P, X, P->FP[i].as<double2>() + P->plane);
+    nk += P->mixed ? 6 : 5;
     join_side(P);  // M X_0 or L X_i is in place before the next combination
   }
   LinComb lc{};
@@ -598,60 +672,71 @@ void enqueue_sbdf_step(tb_plan* P, double dt, int order) {
   const SbdfCoefs K = sbdf_coefs(order, dt);
   const double a0 = K.a0, a1 = K.a1, a2 = K.a2, c1 = K.c1, c2 = K.c2;
   FactorSet* fs = get_factors(P, 0, a0, 1.0);
-  FactorSet* fs2 = P->nsys > 1 ? get_factors(P, 1, a0, 1.0) : nullptr;
-  const long long cnt = (long long)P->nplanes * (long long)P->plane;
   double2* X = P->X.as<double2>();
   double2* Fcur = P->FP[0].as<double2>();
-  double2* MXcur = P->MX0.as<double2>();
-  const bool d3 = P->ndim == 3;
-  int extra = 0;
-  // M X of the projected fields (2D drops Im at the DC / Nyquist modes; 3D
-  // subtracts M delta on the kx = 0 / Nyquist planes) on the side stream,
-  // beside the right-hand side
-  fork_side(P);
-  timed(P, "mass_apply", [&] {
-    launch_mass_apply(X, MXcur, P->s3.as<double>(), P->Nz, P->Nk, P->Nx, d3 ? 0 : 1, P->nf, side(P), P->Nkm);
-  });
-  if (d3) {
-    rbc3d_mx_project(P, MXcur, side(P));
-    ++extra;
-  }
-  if (d3)
-    rbc3d_enqueue_rhs(P, X, Fcur + P->plane);
-  else
+  auto solve = [&] {
+    TauArgs a = tau_args(P, 0, fs, P->Rsb.as<double2>());
+    if (P->bc_dynamic) {  // wall values at t_{n+1}
+      a.bcdyn = P->bcdyn.as<double2>();
+      a.t_dev = P->t_dev.as<double>();
+      a.bc_toff = dt;
+    }
+    timed(P, "tau_solve", [&] { launch_tau_solve(a, P->sys[0].tau_parts, P->st); });
+  };
+  if (P->ndim == 2) {
+    // M X (of the state with Im dropped at the DC / Nyquist modes), the
+    // combination and the shift of the history in one pass
     enqueue_rhs(P, X, Fcur + P->plane, true);
-  join_side(P);
-  LinComb lc{};
-  lc.in[lc.n] = Fcur;
-  lc.w[lc.n++] = c1;
-  lc.in[lc.n] = MXcur;
-  lc.w[lc.n++] = -a1;
-  if (order == 2) {
-    lc.in[lc.n] = P->Fprev.as<double2>();
-    lc.w[lc.n++] = c2;
-    lc.in[lc.n] = P->MXprev.as<double2>();
-    lc.w[lc.n++] = -a2;
+    StageTerms t = stage_args(P, X);
+    t.in[0] = Fcur;
+    t.w[0] = c1;
+    t.n = 1;
+    t.w_mx = -a1;
+    t.project = 1;
+    t.h0 = P->Fprev.as<double2>();
+    t.h1 = P->MXprev.as<double2>();
+    if (order == 2) {
+      t.w_h0 = c2;
+      t.w_h1 = -a2;
+    }
+    timed(P, "stage_lincomb", [&] { launch_stage_rhs(t, P->Rsb.as<double2>(), P->st); });
+    solve();
+    P->kernels_per_step = (P->mixed ? 4 : 3) + 2;
+  } else {
+    FactorSet* fs2 = get_factors(P, 1, a0, 1.0);
+    const long long cnt = (long long)P->nplanes * (long long)P->plane;
+    double2* MXcur = P->MX0.as<double2>();
+    // M X of the projected fields (M delta subtracted on the kx = 0 / Nyquist
+    // planes) on the side stream, beside the right-hand side
+    fork_side(P);
+    timed(P, "mass_apply",
+          [&] { launch_mass_apply(X, MXcur, P->s3.as<double>(), P->Nz, P->Nk, P->nf, side(P)); });
+    rbc3d_mx_project(P, MXcur, side(P));
+    rbc3d_enqueue_rhs(P, X, Fcur + P->plane);
+    join_side(P);
+    LinComb lc{};
+    lc.in[lc.n] = Fcur;
+    lc.w[lc.n++] = c1;
+    lc.in[lc.n] = MXcur;
+    lc.w[lc.n++] = -a1;
+    if (order == 2) {
+      lc.in[lc.n] = P->Fprev.as<double2>();
+      lc.w[lc.n++] = c2;
+      lc.in[lc.n] = P->MXprev.as<double2>();
+      lc.w[lc.n++] = -a2;
+    }
+    timed(P, "stage_lincomb", [&] { launch_lincomb(lc, P->Rsb.as<double2>(), cnt, P->st); });
+    // the history for the next step (read by the combination above) is copied
+    // on the side stream while the tau systems are solved
+    fork_side(P);
+    TB_CUDA_TRY(cudaMemcpyAsync(P->Fprev.p, Fcur, sizeof(double2) * cnt, cudaMemcpyDeviceToDevice, side(P)));
+    TB_CUDA_TRY(cudaMemcpyAsync(P->MXprev.p, MXcur, sizeof(double2) * cnt, cudaMemcpyDeviceToDevice, side(P)));
+    solve();
+    TauArgs s2 = tau_args(P, 1, fs2, P->Rsb.as<double2>());
+    timed(P, "tau_solve_perp", [&] { launch_tau_solve(s2, P->sys[1].tau_parts, P->st); });
+    join_side(P);
+    P->kernels_per_step = (P->mixed ? 6 : 5) + 5;
   }
-  timed(P, "stage_lincomb", [&] { launch_lincomb(lc, P->Rsb.as<double2>(), cnt, P->st); });
-  // the history for the next step (read by the combination above) is copied
-  // on the side stream while the tau systems are solved
-  fork_side(P);
-  TB_CUDA_TRY(cudaMemcpyAsync(P->Fprev.p, Fcur, sizeof(double2) * cnt, cudaMemcpyDeviceToDevice, side(P)));
-  TB_CUDA_TRY(cudaMemcpyAsync(P->MXprev.p, MXcur, sizeof(double2) * cnt, cudaMemcpyDeviceToDevice, side(P)));
-  TauArgs a = tau_args(P, 0, fs, P->Rsb.as<double2>());
-  if (P->bc_dynamic) {  // wall values at t_{n+1}
-    a.bcdyn = P->bcdyn.as<double2>();
-    a.t_dev = P->t_dev.as<double>();
-    a.bc_toff = dt;
-  }
-  timed(P, "tau_solve", [&] { launch_tau_solve(a, P->sys[0].tau_parts, P->st); });
-  if (fs2) {
-    TauArgs a2 = tau_args(P, 1, fs2, P->Rsb.as<double2>());
-    timed(P, "tau_solve_perp", [&] { launch_tau_solve(a2, P->sys[1].tau_parts, P->st); });
-    ++extra;
-  }
-  join_side(P);
-  P->kernels_per_step = (d3 ? (P->mixed ? 6 : 5) : (P->mixed ? 4 : 3)) + 1 + 1 + 1 + extra;
   if (P->bc_dynamic) {
     launch_advance_time(P->t_dev.as<double>(), dt, P->st);
     P->kernels_per_step += 1;
@@ -857,7 +942,7 @@ void tb::plan_prepare(tb_plan* P, double dt, int graph_steps) {
 
 size_t tb::plan_device_bytes(const tb_plan* P) {
   size_t b = 0;
-  const DevBuf* bufs[] = {&P->X,   &P->G,   &P->H,    &P->MX0,  &P->Fprev, &P->MXprev, &P->Rsb, &P->tmpgrid,
+  const DevBuf* bufs[] = {&P->X,   &P->X2,  &P->G,   &P->H,    &P->MX0,  &P->Fprev, &P->MXprev, &P->Rsb, &P->tmpgrid,
                           &P->bwd, &P->fwd, &P->s3,   &P->twM,  &P->twN,   &P->ptwM,   &P->bEv, &P->bOv,
                           &P->bEd, &P->bOd, &P->fE,   &P->fO,   &P->sfE,   &P->sfO,    &P->err_mode,
                           &P->solve_scratch, &P->bcdyn,  &P->t_dev};
@@ -1332,6 +1417,8 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
       rbc3d_setup(P);
     }
     P->MX0.alloc(P->nplanes * pb);
+    const bool rk = desc->timestepper == TB_RK222 || desc->timestepper == TB_RK443;
+    if (rk && !d3) P->X2.alloc(P->X.bytes);
     const int nst = tableau(desc->timestepper).s;
     const int nstage = (desc->timestepper == TB_SBDF1 || desc->timestepper == TB_SBDF2) ? 1 : nst;
     for (int i = 0; i < nstage; ++i) {
@@ -1353,6 +1440,7 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
     if (sbdf) {
       TB_CUDA_TRY(cudaMemsetAsync(P->Fprev.p, 0, P->Fprev.bytes, P->st));
       TB_CUDA_TRY(cudaMemsetAsync(P->MXprev.p, 0, P->MXprev.bytes, P->st));
+      TB_CUDA_TRY(cudaMemsetAsync(P->Rsb.p, 0, P->Rsb.bytes, P->st));  // its continuity rows stay zero
     }
     TB_CUDA_TRY(cudaStreamSynchronize(P->st));
 }
@@ -1659,11 +1747,11 @@ tb_status tb_plan_tune(tb_plan* P, double dt, int trial_steps, int* tau_parts, i
         }
       }
     plan_set_variant(P, bp, br);
-    // then the side stream on or off, on a longer trial (the difference is a
-    // few percent)
+    // then, in 3D, the side stream on or off, on a longer trial (the difference
+    // is a few percent)
     const int ov_steps = std::max(trial_steps, 10);
     float ov_ms[2] = {1e30f, 1e30f};  // best of two alternating trials each
-    for (int t = 0; t < 4; ++t) {
+    for (int t = 0; t < (P->ndim == 3 ? 4 : 0); ++t) {
       const int ov = t & 1;
       if (P->overlap != (ov == 1)) {
         P->overlap = ov == 1;

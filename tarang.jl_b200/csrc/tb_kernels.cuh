@@ -304,18 +304,49 @@ void launch_lincomb(const LinComb& lc, double2* out, long long count, cudaStream
 
 void launch_advance_time(double* t, double dt, cudaStream_t st);
 
-// Velocity-like fields of a stage vector: nf = 3 (2D: b, u_x, u_z in X planes
-// 0..2, equation planes 1..3) or 4 (3D adds u_perp in X plane 4 with its
-// momentum rows in equation plane 4).
-// MX[e][k][m] = S X_f, cont rows zero; optional DC/Nyquist projection (2D).
-void launch_mass_apply(const double2* X, double2* MX, const double* s3, int Nz, int Nk, int Nx, int project,
-                       int nf, cudaStream_t st, int Nkm = 0);
-// LX (in place over rhsP) = (rhsP - PM X)/beta, minus PL delta at the 2D
-// DC/Nyquist modes when Nx > 0 (3D passes Nx = 0 and corrects separately).
-// Batched plans: Nkm modes per instance, per-instance kappa / nu (null: the scalars).
-void launch_lx_finalize(double2* LX, const double2* X, const double* s3, int Nz, int Nk, int Nx, double k0,
-                        double s, double kappa, double nu, double beta, int nf, cudaStream_t st, int Nkm = 0,
-                        const double* kappa_m = nullptr, const double* nu_m = nullptr);
+// 2D stage vectors (equation planes cont, b, u_x, u_z of Nz x Nk): the kernels
+// that build a solve's right-hand side and the final state.
+struct StageTerms {
+  int Nz, Nk, Nkm, Nx;        // Nkm modes an instance (stacked plans)
+  const double* s3;           // S[k][k], S[k][k+2], S[k][k+4]
+  double k0, s, kappa, nu;    // 2 pi / Lx, 2 / Lz, diffusivities (or per instance:)
+  const double* kappa_m;
+  const double* nu_m;
+  const double2* X;           // the state that M X / L X below refer to
+  const double2* in[6];       // plain terms w_t in_t
+  double w[6];
+  int n;
+  // L X of the newest stage: on entry lx holds that stage's right-hand side, and
+  // L X = (rhs - M X) / beta - L delta (delta: Im of the DC / Nyquist modes); the
+  // term w_lx L X is added and L X written back to lx
+  double2* lx;
+  double w_lx, ibeta;
+  // M X (project: of the state with Im dropped at the DC / Nyquist modes): where
+  // w_mx is nonzero the term w_mx M X is added, and M X written to mx if given
+  double2* mx;
+  double w_mx;
+  int project;
+  // multistep history: terms w_h0 h0 and w_h1 h1 are added where nonzero, then
+  // h0 takes in[0] and h1 takes M X
+  double2* h0;
+  double2* h1;
+  double w_h0, w_h1;
+};
+// out (four equation planes, the continuity rows outside the DC / Nyquist modes
+// left as they are: zero) = the sum of the terms of a.
+void launch_stage_rhs(const StageTerms& a, double2* out, cudaStream_t st);
+// Xout_f = S^{-1} (the sum of the terms of a)[eq(f)] for b, u_x, u_z; p and the
+// taus of Xout zeroed.  a.X may not be Xout.
+void launch_stage_final(const StageTerms& a, double2* Xout, double2* tau, int ntau, cudaStream_t st);
+
+// 3D: the velocity-like fields of a stage vector, nf = 4 (b, u_par, u_z in X
+// planes 0..2 and equation planes 1..3, u_perp in plane 4 of both).
+// MX[e][k][m] = S X_f, cont rows zero.
+void launch_mass_apply(const double2* X, double2* MX, const double* s3, int Nz, int Nk, int nf, cudaStream_t st);
+// LX (in place over rhsP) = (rhsP - PM X)/beta (the L delta correction is the
+// 3D program's own).
+void launch_lx_finalize(double2* LX, const double2* X, const double* s3, int Nz, int Nk, double beta, int nf,
+                        cudaStream_t st);
 // X_f = S^{-1} (lincomb)[eq(f)] for the nf velocity-like fields; p and the ntau taus zeroed.
 void launch_rk_final(const LinComb& lc, double2* X, double2* tau, const double* s3, int Nz, int Nk, int nf,
                      int ntau, cudaStream_t st);

@@ -171,7 +171,8 @@ struct tb_plan {
   // state and work arrays
   // X holds the state planes followed by the tau rows (tau views its tail),
   // so one 32-bit element offset from X addresses every unknown of the solve
-  DevBuf X, G, H, MX0, FP[4], LXP[4], Fprev, MXprev, Rsb, tmpgrid;
+  // X2 (2D RK): the last stage's state, laid out as X
+  DevBuf X, X2, G, H, MX0, FP[4], LXP[4], Fprev, MXprev, Rsb, tmpgrid;
   DevView tau;
   // 3D RHS program (element type of the RHS precision): Cartesian copy of the
   // state, Chebyshev half planes, y-transformed factors, x-pass products,
@@ -207,7 +208,7 @@ struct tb_plan {
   // caller's host buffer on a side stream while the plan steps on
   DevBuf stage_grid;
   cudaStream_t io_st = nullptr;
-  // side stream of the step: work independent of the RHS chain (L X
+  // side stream of a 3D step: work independent of the RHS chain (L X
   // finalisation, M X, the SBDF history copies) forks onto it and joins back
   // before its results are used, inside the captured step graphs
   cudaStream_t st2 = nullptr;

@@ -1049,90 +1049,160 @@ __device__ __forceinline__ double2 proj(double2 v, bool p) { return p ? make_dou
 __device__ __forceinline__ int xplane_of(int q) { return q < 3 ? q : 4; }
 __device__ __forceinline__ int eplane_of(int q) { return q < 3 ? 1 + q : 4; }
 
-// One thread per (row k, mode m): grid (ceil(Nk / 128), Nz).
 // Advance the device time of dynamic wall values by dt (end of a step).
 __global__ void k_advance_time(double* t, double dt) { *t += dt; }
 
+// One thread per (row k, mode m): grid (ceil(Nk / 128), Nz).
 __global__ void __launch_bounds__(128) k_mass_apply(const double2* __restrict__ X, double2* __restrict__ MX,
-                                                    const double* __restrict__ s3, int Nz, int Nk, int Nx,
-                                                    int project, int nf, int Nkm) {
+                                                    const double* __restrict__ s3, int Nz, int Nk, int nf) {
   const int k = blockIdx.y, m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= Nk) return;
   const size_t i = (size_t)k * Nk + m;
-  const int ml = m % Nkm;  // mode within its instance
-  const bool pj = project && (ml == 0 || 2 * ml == Nx);
   const double s0 = s3[3 * k], s1 = s3[3 * k + 1], s2 = s3[3 * k + 2];
   MX[i] = make_double2(0.0, 0.0);
   for (int f = 0; f < nf; ++f) {
     const double2* Xf = X + (size_t)xplane_of(f) * Nz * Nk;
     double2 acc = make_double2(0.0, 0.0);
-    acc = cfma(s0, proj(Xf[i], pj), acc);
-    if (k + 2 < Nz) acc = cfma(s1, proj(Xf[i + 2 * (size_t)Nk], pj), acc);
-    if (k + 4 < Nz) acc = cfma(s2, proj(Xf[i + 4 * (size_t)Nk], pj), acc);
+    acc = cfma(s0, Xf[i], acc);
+    if (k + 2 < Nz) acc = cfma(s1, Xf[i + 2 * (size_t)Nk], acc);
+    if (k + 4 < Nz) acc = cfma(s2, Xf[i + 4 * (size_t)Nk], acc);
     MX[(size_t)eplane_of(f) * Nz * Nk + i] = acc;
   }
 }
 
 // One thread per (row k, mode m): grid (ceil(Nk / 128), Nz).
 __global__ void __launch_bounds__(128) k_lx_finalize(double2* __restrict__ LX, const double2* __restrict__ X,
-                                                     const double* __restrict__ s3, int Nz, int Nk, int Nx, double k0,
-                                                     double s, double kappa, double nu, double beta, int nf, int Nkm,
-                                                     const double* __restrict__ kappa_m,
-                                                     const double* __restrict__ nu_m) {
+                                                     const double* __restrict__ s3, int Nz, int Nk, double beta,
+                                                     int nf) {
   const double ib = 1.0 / beta;
-  {
-    const int k = blockIdx.y, m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= Nk) return;
-    const size_t i = (size_t)k * Nk + m;
-    const double s0 = s3[3 * k], s1 = s3[3 * k + 1], s2 = s3[3 * k + 2];
-    auto xf = [&](int f, int kk) -> double2 {
-      return (kk < Nz) ? X[((size_t)f * Nz + kk) * Nk + m] : make_double2(0.0, 0.0);
-    };
-    auto Sx = [&](int f) -> double2 {
-      double2 acc = make_double2(0.0, 0.0);
-      acc = cfma(s0, xf(f, k), acc);
-      acc = cfma(s1, xf(f, k + 2), acc);
-      acc = cfma(s2, xf(f, k + 4), acc);
-      return acc;
-    };
-    const size_t plane = (size_t)Nz * Nk;
-    double2 out[4];
-    for (int e = 0; e < 4; ++e) {
-      double2 r = LX[(size_t)e * plane + i];
-      if (e > 0) {
-        double2 mx = Sx(e - 1);
-        r.x -= mx.x;
-        r.y -= mx.y;
-      }
-      out[e] = make_double2(r.x * ib, r.y * ib);
+  const int k = blockIdx.y, m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= Nk) return;
+  const size_t i = (size_t)k * Nk + m, plane = (size_t)Nz * Nk;
+  const double s0 = s3[3 * k], s1 = s3[3 * k + 1], s2 = s3[3 * k + 2];
+  auto xf = [&](int f, int kk) -> double2 {
+    return (kk < Nz) ? X[((size_t)f * Nz + kk) * Nk + m] : make_double2(0.0, 0.0);
+  };
+  auto Sx = [&](int f) -> double2 {
+    double2 acc = make_double2(0.0, 0.0);
+    acc = cfma(s0, xf(f, k), acc);
+    acc = cfma(s1, xf(f, k + 2), acc);
+    acc = cfma(s2, xf(f, k + 4), acc);
+    return acc;
+  };
+  double2 out[4];
+  for (int e = 0; e < 4; ++e) {
+    double2 r = LX[(size_t)e * plane + i];
+    if (e > 0) {
+      double2 mx = Sx(e - 1);
+      r.x -= mx.x;
+      r.y -= mx.y;
     }
-    if (nf > 3) {  // u_perp rows (3D): the equation plane after the pressure
-      double2 r = LX[4 * plane + i];
-      const double2 mx = Sx(4);
-      LX[4 * plane + i] = make_double2((r.x - mx.x) * ib, (r.y - mx.y) * ib);
+    out[e] = make_double2(r.x * ib, r.y * ib);
+  }
+  if (nf > 3) {  // u_perp rows: the equation plane after the pressure
+    double2 r = LX[4 * plane + i];
+    const double2 mx = Sx(4);
+    LX[4 * plane + i] = make_double2((r.x - mx.x) * ib, (r.y - mx.y) * ib);
+  }
+  for (int e = 0; e < 4; ++e) LX[(size_t)e * plane + i] = out[e];
+}
+
+// ---- fused 2D stage kernels ----
+// M X, L X and the combination of a stage read and write the same entries, so
+// one pass over them replaces three: each input is read once, and the launches
+// between two solves, which bound the small grids, drop from three to one.
+// Threads are one per (equation plane, row, mode), so that a thread has every
+// load (up to 11) in flight at once; one thread per (row, mode) over the four
+// planes kept too few (measured no faster than the separate kernels at
+// 1024x256).
+
+// L delta at (equation plane e, row k) of a DC / Nyquist mode, delta = i Im(X) of
+// b, u_x, u_z (the part a grid round trip drops)
+__device__ double2 l_delta(const StageTerms& a, int e, int k, int m) {
+  auto dl = [&](int f, int kk) -> double { return (kk < a.Nz) ? a.X[((size_t)f * a.Nz + kk) * a.Nk + m].y : 0.0; };
+  auto Sd = [&](int f) -> double {
+    return a.s3[3 * k] * dl(f, k) + a.s3[3 * k + 1] * dl(f, k + 2) + a.s3[3 * k + 2] * dl(f, k + 4);
+  };
+  const double kx = a.k0 * (m % a.Nkm), kx2 = kx * kx, d2 = 2.0 * (k + 2) * a.s * a.s;
+  const double kappa = a.kappa_m ? a.kappa_m[m / a.Nkm] : a.kappa, nu = a.nu_m ? a.nu_m[m / a.Nkm] : a.nu;
+  // every term is i * (real coefficient) * Im(X); cont: i kx S d_ux + SD d_uz, i kx (i a) = -kx a
+  if (e == 0) return make_double2(-kx * Sd(UK_UX), a.s * (dl(UK_UZ, k + 1) - dl(UK_UZ, k + 3)));
+  const int f = e - 1;
+  const double c = f == UK_B ? kappa : nu;
+  double im = c * kx2 * Sd(f) - c * d2 * dl(f, k + 2);
+  if (f == UK_UZ) im -= Sd(UK_B);
+  return make_double2(0.0, im);
+}
+
+// Every load of one entry (equation plane e, row k, mode m), issued together.
+struct StageLoads {
+  double2 v[6], r, h0, h1, x[3];  // x: the field's rows k, k + 2, k + 4 for S X
+};
+__device__ __forceinline__ void stage_load(const StageTerms& a, int e, int k, int m, StageLoads& L) {
+  const size_t i = ((size_t)e * a.Nz + k) * a.Nk + m;
+  const double2 zero = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int t = 0; t < 6; ++t) L.v[t] = t < a.n ? a.in[t][i] : zero;
+  L.r = a.lx ? a.lx[i] : zero;
+  const bool hist = a.h0 && a.w_h0 != 0.0;
+  L.h0 = hist ? a.h0[i] : zero;
+  L.h1 = hist ? a.h1[i] : zero;
+  const bool sx = e > 0 && (a.lx || a.w_mx != 0.0);
+  const double2* x = a.X + ((size_t)(e - 1) * a.Nz + k) * a.Nk + m;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) L.x[q] = sx && k + 2 * q < a.Nz ? x[(size_t)(2 * q) * a.Nk] : zero;
+}
+
+// The sum of the terms; WRITE: L X and M X are written back and the history
+// shifted (each entry by its own thread).
+template <bool WRITE>
+__device__ __forceinline__ double2 stage_sum(const StageTerms& a, int e, int k, int m, const StageLoads& L) {
+  const size_t i = ((size_t)e * a.Nz + k) * a.Nk + m;
+  const int ml = m % a.Nkm;
+  const bool edge = ml == 0 || 2 * ml == a.Nx, pj = a.project && edge;
+  double2 sx = make_double2(0.0, 0.0), acc = sx;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) sx = cfma(a.s3[3 * k + q], proj(L.x[q], pj), sx);
+#pragma unroll
+  for (int t = 0; t < 6; ++t)
+    if (t < a.n) acc = cfma(a.w[t], L.v[t], acc);
+  if (a.lx) {
+    double2 lx = make_double2((L.r.x - sx.x) * a.ibeta, (L.r.y - sx.y) * a.ibeta);
+    if (edge) {
+      const double2 d = l_delta(a, e, k, m);
+      lx.x -= d.x;
+      lx.y -= d.y;
     }
-    const int ml = m % Nkm;  // mode within its instance
-    if (Nx > 0 && (ml == 0 || 2 * ml == Nx)) {
-      // L applied to delta = i Im(X) of b, ux, uz (the part a grid round trip drops)
-      const double kx = k0 * ml, kx2 = kx * kx;
-      if (kappa_m) {
-        kappa = kappa_m[m / Nkm];
-        nu = nu_m[m / Nkm];
-      }
-      auto dl = [&](int f, int kk) -> double { return (kk < Nz) ? X[((size_t)f * Nz + kk) * Nk + m].y : 0.0; };
-      auto Sd = [&](int f) -> double { return s0 * dl(f, k) + s1 * dl(f, k + 2) + s2 * dl(f, k + 4); };
-      const double d2 = 2.0 * (k + 2) * s * s;
-      // every term is i * (real coefficient) * Im(X): subtract from the imaginary part
-      // cont: i kx S d_ux + SD d_uz ; i kx * (i a) = -kx a is real
-      double cont_re = -kx * Sd(UK_UX);
-      double cont_im = s * (dl(UK_UZ, k + 1) - dl(UK_UZ, k + 3));
-      out[0].x -= cont_re;
-      out[0].y -= cont_im;
-      out[1].y -= kappa * kx2 * Sd(UK_B) - kappa * d2 * dl(UK_B, k + 2);
-      out[2].y -= nu * kx2 * Sd(UK_UX) - nu * d2 * dl(UK_UX, k + 2);
-      out[3].y -= nu * kx2 * Sd(UK_UZ) - nu * d2 * dl(UK_UZ, k + 2) - Sd(UK_B);
+    if (WRITE) a.lx[i] = lx;
+    acc = cfma(a.w_lx, lx, acc);
+  }
+  if (a.w_mx != 0.0) {
+    if (WRITE && a.mx) a.mx[i] = sx;
+    acc = cfma(a.w_mx, sx, acc);
+  }
+  if (a.h0) {
+    if (a.w_h0 != 0.0) acc = cfma(a.w_h1, L.h1, cfma(a.w_h0, L.h0, acc));
+    if (WRITE) {
+      a.h0[i] = L.v[0];
+      a.h1[i] = sx;
     }
-    for (int e = 0; e < 4; ++e) LX[(size_t)e * plane + i] = out[e];
+  }
+  return acc;
+}
+
+// Grid (ceil(Nk / 128), Nz, 3): equation planes 1..3; the continuity rows, whose
+// terms are zero outside the DC / Nyquist modes (F, M X and the first right-hand
+// side have none), by the threads of plane 1 there.
+__global__ void __launch_bounds__(128) k_stage_rhs(StageTerms a, double2* __restrict__ out) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y, e = 1 + blockIdx.z;
+  if (m >= a.Nk) return;
+  StageLoads L;
+  stage_load(a, e, k, m, L);
+  out[((size_t)e * a.Nz + k) * a.Nk + m] = stage_sum<true>(a, e, k, m, L);
+  const int ml = m % a.Nkm;
+  if (e == 1 && (ml == 0 || 2 * ml == a.Nx)) {
+    stage_load(a, 0, k, m, L);
+    out[(size_t)k * a.Nk + m] = stage_sum<true>(a, 0, k, m, L);
   }
 }
 
@@ -1145,6 +1215,61 @@ __global__ void __launch_bounds__(128) k_lx_finalize(double2* __restrict__ LX, c
 // rows and the reciprocal diagonal; the first kFinalModes threads run the
 // recurrences out of shared memory, and all threads write X back.
 constexpr int kFinalModes = 8;
+
+// The backward recurrence of one column (rows ri of ys, kFinalModes apart), in place.
+__device__ __forceinline__ void s_solve(double2* ys, const double* sk, int K, int mm) {
+  double2 x2 = make_double2(0.0, 0.0), x4 = make_double2(0.0, 0.0);
+  for (int ri = K - 1; ri >= 0; --ri) {
+    double2 y = ys[ri * kFinalModes + mm];
+    y = cfma(-sk[3 * ri + 1], x2, y);
+    y = cfma(-sk[3 * ri + 2], x4, y);
+    const double inv = sk[3 * ri];
+    const double2 x = make_double2(y.x * inv, y.y * inv);
+    ys[ri * kFinalModes + mm] = x;
+    x4 = x2;
+    x2 = x;
+  }
+}
+
+// The 2D form: the terms (with the last stage's L X) as in k_stage_rhs, p and
+// the taus zeroed here too.
+__global__ void __launch_bounds__(256, 2) k_stage_final(StageTerms a, double2* __restrict__ Xo, double2* __restrict__ tau,
+                                                     int ntau) {
+  extern __shared__ double2 ys[];  // as in k_rk_final
+  constexpr int MB = kFinalModes, RG = 256 / MB;
+  const int f = blockIdx.y >> 1, par = blockIdx.y & 1, Nz = a.Nz, Nk = a.Nk;
+  const int mm = threadIdx.x % MB, ks = threadIdx.x / MB;
+  const int m = blockIdx.x * MB + mm;
+  const size_t plane = (size_t)Nz * Nk;
+  const int K = (Nz - par + 1) / 2;  // rows k = par + 2 ri
+  double* sk = reinterpret_cast<double*>(ys + (size_t)K * MB);
+  for (int q = threadIdx.x; q < K; q += blockDim.x) {
+    const int k = par + 2 * q;
+    sk[3 * q] = 1.0 / a.s3[3 * k];
+    sk[3 * q + 1] = a.s3[3 * k + 1];
+    sk[3 * q + 2] = a.s3[3 * k + 2];
+  }
+  const int mc = m < Nk ? m : Nk - 1;  // clamped column: loads stay in bounds
+  const double2 zero = make_double2(0.0, 0.0);
+  for (int r0 = ks; r0 < K; r0 += 2 * RG) {  // two rows' loads in flight
+    const int r1 = (r0 + RG < K) ? r0 + RG : r0;
+    StageLoads L0, L1;
+    stage_load(a, 1 + f, par + 2 * r0, mc, L0);
+    stage_load(a, 1 + f, par + 2 * r1, mc, L1);
+    ys[r0 * MB + mm] = stage_sum<false>(a, 1 + f, par + 2 * r0, mc, L0);
+    if (r0 + RG < K) ys[r1 * MB + mm] = stage_sum<false>(a, 1 + f, par + 2 * r1, mc, L1);
+  }
+  if (f == 0 && m < Nk)
+    for (int ri = ks; ri < K; ri += RG) Xo[3 * plane + (size_t)(par + 2 * ri) * Nk + m] = zero;
+  if (f == 1 && par == 0 && m < Nk)
+    for (int t = ks; t < ntau; t += RG) tau[(size_t)t * Nk + m] = zero;
+  __syncthreads();
+  if (threadIdx.x < MB) s_solve(ys, sk, K, mm);
+  __syncthreads();
+  if (m < Nk)
+    for (int ri = ks; ri < K; ri += RG) Xo[(size_t)f * plane + (size_t)(par + 2 * ri) * Nk + m] = ys[ri * MB + mm];
+}
+
 template <int N>
 __global__ void __launch_bounds__(256) k_rk_final(LinComb lc, double2* __restrict__ X, const double* __restrict__ s3,
                                                   int Nz, int Nk) {
@@ -1184,19 +1309,7 @@ __global__ void __launch_bounds__(256) k_rk_final(LinComb lc, double2* __restric
     if (r0 + RG < K) ys[(r0 + RG) * MB + mm] = a1;
   }
   __syncthreads();
-  if (threadIdx.x < MB) {
-    double2 x2 = make_double2(0.0, 0.0), x4 = make_double2(0.0, 0.0);
-    for (int ri = K - 1; ri >= 0; --ri) {
-      double2 y = ys[ri * MB + mm];
-      y = cfma(-sk[3 * ri + 1], x2, y);
-      y = cfma(-sk[3 * ri + 2], x4, y);
-      const double inv = sk[3 * ri];
-      const double2 x = make_double2(y.x * inv, y.y * inv);
-      ys[ri * MB + mm] = x;
-      x4 = x2;
-      x2 = x;
-    }
-  }
+  if (threadIdx.x < MB) s_solve(ys, sk, K, mm);
   __syncthreads();
   if (m < Nk)
     for (int ri = ks; ri < K; ri += RG)
@@ -1323,18 +1436,13 @@ void launch_lincomb(const LinComb& lc, double2* out, long long count, cudaStream
 
 void launch_advance_time(double* t, double dt, cudaStream_t st) { k_advance_time<<<1, 1, 0, st>>>(t, dt); }
 
-void launch_mass_apply(const double2* X, double2* MX, const double* s3, int Nz, int Nk, int Nx, int project,
-                       int nf, cudaStream_t st, int Nkm) {
-  dim3 grid((Nk + 127) / 128, Nz);
-  k_mass_apply<<<grid, 128, 0, st>>>(X, MX, s3, Nz, Nk, Nx, project, nf, Nkm > 0 ? Nkm : Nk);
+void launch_mass_apply(const double2* X, double2* MX, const double* s3, int Nz, int Nk, int nf, cudaStream_t st) {
+  k_mass_apply<<<dim3((Nk + 127) / 128, Nz), 128, 0, st>>>(X, MX, s3, Nz, Nk, nf);
 }
 
-void launch_lx_finalize(double2* LX, const double2* X, const double* s3, int Nz, int Nk, int Nx, double k0,
-                        double s, double kappa, double nu, double beta, int nf, cudaStream_t st, int Nkm,
-                        const double* kappa_m, const double* nu_m) {
-  dim3 grid((Nk + 127) / 128, Nz);
-  k_lx_finalize<<<grid, 128, 0, st>>>(LX, X, s3, Nz, Nk, Nx, k0, s, kappa, nu, beta, nf, Nkm > 0 ? Nkm : Nk, kappa_m,
-                                      nu_m);
+void launch_lx_finalize(double2* LX, const double2* X, const double* s3, int Nz, int Nk, double beta, int nf,
+                        cudaStream_t st) {
+  k_lx_finalize<<<dim3((Nk + 127) / 128, Nz), 128, 0, st>>>(LX, X, s3, Nz, Nk, beta, nf);
 }
 
 void launch_rk_final(const LinComb& lc, double2* X, double2* tau, const double* s3, int Nz, int Nk, int nf,
@@ -1354,6 +1462,15 @@ void launch_rk_final(const LinComb& lc, double2* X, double2* tau, const double* 
 #undef TB_RKFINAL_CASE
   cudaMemsetAsync(X + (size_t)3 * Nz * Nk, 0, sizeof(double2) * (size_t)Nz * Nk, st);
   cudaMemsetAsync(tau, 0, sizeof(double2) * (size_t)ntau * Nk, st);
+}
+
+void launch_stage_rhs(const StageTerms& a, double2* out, cudaStream_t st) {
+  k_stage_rhs<<<dim3((a.Nk + 127) / 128, a.Nz, 3), 128, 0, st>>>(a, out);
+}
+
+void launch_stage_final(const StageTerms& a, double2* Xout, double2* tau, int ntau, cudaStream_t st) {
+  k_stage_final<<<dim3((a.Nk + kFinalModes - 1) / kFinalModes, 6), 256, rk_final_smem_bytes(a.Nz), st>>>(a, Xout, tau,
+                                                                                                        ntau);
 }
 
 size_t rk_final_smem_bytes(int Nz) {

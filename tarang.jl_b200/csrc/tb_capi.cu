@@ -942,7 +942,7 @@ void tb::plan_prepare(tb_plan* P, double dt, int graph_steps) {
 
 size_t tb::plan_device_bytes(const tb_plan* P) {
   size_t b = 0;
-  const DevBuf* bufs[] = {&P->X,   &P->X2,  &P->G,   &P->H,    &P->MX0,  &P->Fprev, &P->MXprev, &P->Rsb, &P->tmpgrid,
+  const DevBuf* bufs[] = {&P->X,   &P->X2,  &P->G,   &P->H,    &P->MX0,  &P->Fprev, &P->MXprev, &P->Rsb,
                           &P->bwd, &P->fwd, &P->s3,   &P->twM,  &P->twN,   &P->ptwM,   &P->bEv, &P->bOv,
                           &P->bEd, &P->bOd, &P->fE,   &P->fO,   &P->sfE,   &P->sfO,    &P->err_mode,
                           &P->solve_scratch, &P->bcdyn,  &P->t_dev};
@@ -1298,9 +1298,12 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
         for (int j = 0; j < P->Hz; ++j) o[(size_t)r * Kp + j] = m[(size_t)(2 * r + par) * N + j];
       return o;
     };
-    std::vector<double> bwdp((size_t)N * pad16(N), 0.0);
-    for (int j = 0; j < N; ++j)
-      for (int n = 0; n < N; ++n) bwdp[(size_t)j * pad16(N) + n] = cm.bwd[(size_t)j * N + n];
+    if (desc->ndim == 3) {  // the full backward matrix (2D field transforms use the parity halves)
+      std::vector<double> bwdp((size_t)N * pad16(N), 0.0);
+      for (int j = 0; j < N; ++j)
+        for (int n = 0; n < N; ++n) bwdp[(size_t)j * pad16(N) + n] = cm.bwd[(size_t)j * N + n];
+      upload(P->bwd, bwdp);
+    }
     upload(P->bEv, cols_of(cm.bwd, 0));
     upload(P->bOv, cols_of(cm.bwd, 1));
     upload(P->bEd, cols_of(cm.bwd_d, 0));
@@ -1309,7 +1312,6 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
     upload(P->fO, rows_of(cm.fwd, 1));
     upload(P->sfE, rows_of(cm.sfwd, 0));
     upload(P->sfO, rows_of(cm.sfwd, 1));
-    upload(P->bwd, bwdp);
     upload(P->s3, cm.s3);
     upload(P->twM, twiddles(P->M));
     upload(P->ptwM, pass_twiddles(P->fpM));
@@ -1412,7 +1414,6 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
         P->G32.alloc(12 * (size_t)((P->Nz + 1) / 2) * P->Nk * sizeof(float2));
         P->H32.alloc(3 * P->plane * sizeof(float2));
       }
-      P->tmpgrid.alloc(P->plane * sizeof(double2));
     } else {
       rbc3d_setup(P);
     }
@@ -1873,25 +1874,45 @@ namespace {
 int checkpoint_fields(const tb_plan* P) { return P->ndim == 3 ? 5 : 4; }
 size_t grid_points(const tb_plan* P) { return (size_t)P->Nz * P->Ny * P->Nx; }
 
-// 2D: coefficient plane (Nz, Nx/2+1) -> grid (Nz, Nx) on the plan's stream.
-void grid_of_plane_2d(tb_plan* P, const double2* coeff, double* grid) {
-  double2* mixed = P->tmpgrid.as<double2>();
-  GemmBatch bt{};
-  bt.item[0] = GemmItem{P->bwd.as<double>(), reinterpret_cast<const double*>(coeff), reinterpret_cast<double*>(mixed),
-                        P->Nz, P->Nz, pad16k(P->Nz), GEMM_PLAIN, 0};
-  launch_gemm_f64(bt, 1, 2 * P->Nk, 2 * P->Nk, 2 * P->Nk, P->Nz, P->st);
-  launch_x_irfft(mixed, grid, P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
+// 2D field transforms on the plan's stream, fields back to back: as many fields
+// a launch as the step's scratch G (12 half planes) holds.  Coefficients ->
+// grid goes through the even / odd half planes, which halves the products of the
+// full matrix; grid -> coefficients folds the mirror rows (GEMM_MIRROR).
+constexpr int kFieldsPerLaunch = 6;
+
+void grids_of_planes_2d(tb_plan* P, const double2* coeff, double* grid, int nfields) {
+  const size_t g = (size_t)P->Nz * P->Nx, hplane = (size_t)P->Hz * P->Nk;
+  double2* half = P->G.as<double2>();
+  for (int f0 = 0; f0 < nfields; f0 += kFieldsPerLaunch) {
+    const int nf = std::min(kFieldsPerLaunch, nfields - f0);
+    GemmBatch bt{};
+    for (int f = 0; f < nf; ++f)
+      for (int w = 0; w < 2; ++w)
+        bt.item[2 * f + w] = GemmItem{(w ? P->bOv : P->bEv).as<double>(),
+                                      reinterpret_cast<const double*>(coeff + (size_t)(f0 + f) * P->plane),
+                                      reinterpret_cast<double*>(half + (size_t)(2 * f + w) * hplane), P->Hz,
+                                      w ? P->Ko : P->Ke, pad16k(w ? P->Ko : P->Ke), GEMM_PARITY, w};
+    launch_gemm_f64(bt, 2 * nf, 2 * P->Nk, 2 * P->Nk, 2 * P->Nk, P->Nz, P->st);
+    launch_x_irfft_half(half, grid + f0 * g, nf, P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
+  }
 }
 
-void plane_of_grid_2d(tb_plan* P, const double* grid, double2* coeff) {
-  double2* mixed = P->tmpgrid.as<double2>();
-  launch_x_rfft(grid, mixed, P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
-  GemmBatch bt{};
-  bt.item[0] = GemmItem{P->fE.as<double>(), reinterpret_cast<const double*>(mixed), reinterpret_cast<double*>(coeff),
-                        P->Ke, P->Hz, pad16k(P->Hz), GEMM_MIRROR, 0};
-  bt.item[1] = GemmItem{P->fO.as<double>(), reinterpret_cast<const double*>(mixed), reinterpret_cast<double*>(coeff),
-                        P->Ko, P->Hz, pad16k(P->Hz), GEMM_MIRROR, 1};
-  launch_gemm_f64(bt, P->Ko > 0 ? 2 : 1, 2 * P->Nk, 2 * P->Nk, 2 * P->Nk, P->Nz, P->st);
+void planes_of_grids_2d(tb_plan* P, const double* grid, double2* coeff, int nfields) {
+  const size_t g = (size_t)P->Nz * P->Nx;
+  double2* spec = P->G.as<double2>();  // 12 half planes: room for six planes
+  for (int f0 = 0; f0 < nfields; f0 += kFieldsPerLaunch) {
+    const int nf = std::min(kFieldsPerLaunch, nfields - f0);
+    launch_x_rfft(grid + f0 * g, spec, nf * P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
+    GemmBatch bt{};
+    int nb = 0;
+    for (int f = 0; f < nf; ++f) {
+      const double* in = reinterpret_cast<const double*>(spec + (size_t)f * P->plane);
+      double* out = reinterpret_cast<double*>(coeff + (size_t)(f0 + f) * P->plane);
+      bt.item[nb++] = GemmItem{P->fE.as<double>(), in, out, P->Ke, P->Hz, pad16k(P->Hz), GEMM_MIRROR, 0};
+      if (P->Ko > 0) bt.item[nb++] = GemmItem{P->fO.as<double>(), in, out, P->Ko, P->Hz, pad16k(P->Hz), GEMM_MIRROR, 1};
+    }
+    launch_gemm_f64(bt, nb, 2 * P->Nk, 2 * P->Nk, 2 * P->Nk, P->Nz, P->st);
+  }
 }
 
 }  // namespace
@@ -1926,8 +1947,7 @@ tb_status tb_checkpoint_stage(tb_plan* P, double* host_grid, size_t capacity, do
         rbc3d_transform_backward(P, P->tmp3.as<double2>(), stage + f * g);
       }
     } else {
-      const int planes[4] = {0, 1, 2, 3};  // b, u_x, u_z, p
-      for (int f = 0; f < nf; ++f) grid_of_plane_2d(P, P->Xp(planes[f]), stage + f * g);
+      grids_of_planes_2d(P, P->Xp(0), stage, nf);  // b, u_x, u_z, p
     }
     check_launch("checkpoint staging");
     TB_CUDA_TRY(cudaEventRecord(P->io_ready, P->st));
@@ -1975,7 +1995,7 @@ tb_status tb_checkpoint_load(tb_plan* P, const double* grid, int where, const do
         rbc3d_state_set(P, fields[f], P->tmp3.as<double2>());
       }
     } else {
-      for (int f = 0; f < nf; ++f) plane_of_grid_2d(P, stage + f * g, P->Xp(f));
+      planes_of_grids_2d(P, stage, P->Xp(0), nf);
     }
     check_launch("checkpoint load");
     TB_CUDA_TRY(cudaStreamSynchronize(P->st));
@@ -2003,18 +2023,8 @@ tb_status tb_transform_forward(tb_plan* P, const double* grid, double* coeff, in
       TB_CUDA_TRY(cudaStreamSynchronize(P->st));
     });
   return guard(P->ctx, [&] {
-    const size_t gsz = (size_t)P->Nz * P->Nx;
-    for (int f = 0; f < nfields; ++f) {
-      double2* mixed = P->tmpgrid.as<double2>();
-      launch_x_rfft(grid + f * gsz, mixed, P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
-      GemmBatch bt{};
-      bt.item[0] = GemmItem{P->fE.as<double>(), reinterpret_cast<const double*>(mixed), coeff + f * 2 * P->plane, P->Ke,
-                            P->Hz, pad16k(P->Hz), GEMM_MIRROR, 0};
-      bt.item[1] = GemmItem{P->fO.as<double>(), reinterpret_cast<const double*>(mixed), coeff + f * 2 * P->plane, P->Ko,
-                            P->Hz, pad16k(P->Hz), GEMM_MIRROR, 1};
-      launch_gemm_f64(bt, P->Ko > 0 ? 2 : 1, 2 * P->Nk, 2 * P->Nk, 2 * P->Nk, P->Nz, P->st);
-      check_launch("transform forward");
-    }
+    planes_of_grids_2d(P, grid, reinterpret_cast<double2*>(coeff), nfields);
+    check_launch("transform forward");
     TB_CUDA_TRY(cudaStreamSynchronize(P->st));
   });
 }
@@ -2030,16 +2040,8 @@ tb_status tb_transform_backward(tb_plan* P, const double* coeff, double* grid, i
       TB_CUDA_TRY(cudaStreamSynchronize(P->st));
     });
   return guard(P->ctx, [&] {
-    const size_t gsz = (size_t)P->Nz * P->Nx;
-    for (int f = 0; f < nfields; ++f) {
-      double2* mixed = P->tmpgrid.as<double2>();
-      GemmBatch bt{};
-      bt.item[0] = GemmItem{P->bwd.as<double>(), coeff + f * 2 * P->plane, reinterpret_cast<double*>(mixed), P->Nz,
-                            P->Nz, pad16k(P->Nz), GEMM_PLAIN, 0};
-      launch_gemm_f64(bt, 1, 2 * P->Nk, 2 * P->Nk, 2 * P->Nk, P->Nz, P->st);
-      launch_x_irfft(mixed, grid + f * gsz, P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
-      check_launch("transform backward");
-    }
+    grids_of_planes_2d(P, reinterpret_cast<const double2*>(coeff), grid, nfields);
+    check_launch("transform backward");
     TB_CUDA_TRY(cudaStreamSynchronize(P->st));
   });
 }

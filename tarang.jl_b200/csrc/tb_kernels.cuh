@@ -154,6 +154,10 @@ void launch_x_rfft(const double* grid, double2* spec, int nrows, int Nx, const F
                    cudaStream_t st);
 void launch_x_irfft(const double2* spec, double* grid, int nrows, int Nx, const FftPlan& fp, const double2* tw,
                     cudaStream_t st);
+// Grid fields (Nz x Nx each, back to back) from their even / odd Chebyshev half
+// planes (per field: ceil(Nz/2) x (Nx/2+1) even, then odd).
+void launch_x_irfft_half(const double2* half, double* grid, int nfields, int Nz, int Nx, const FftPlan& fp,
+                         const double2* tw, cudaStream_t st);
 // Standalone 3/2-dealiased product of two grid fields (rows of length Nx).
 void launch_x_dealias_mul(const double* a, const double* b, double* out, int nrows, int Nx, int M,
                           const FftPlan& fpN, const double2* twN, const FftPlan& fpM, const double2* twM,

@@ -172,7 +172,7 @@ struct tb_plan {
   // X holds the state planes followed by the tau rows (tau views its tail),
   // so one 32-bit element offset from X addresses every unknown of the solve
   // X2 (2D RK): the last stage's state, laid out as X
-  DevBuf X, X2, G, H, MX0, FP[4], LXP[4], Fprev, MXprev, Rsb, tmpgrid;
+  DevBuf X, X2, G, H, MX0, FP[4], LXP[4], Fprev, MXprev, Rsb;
   DevView tau;
   // 3D RHS program (element type of the RHS precision): Cartesian copy of the
   // state, Chebyshev half planes, y-transformed factors, x-pass products,

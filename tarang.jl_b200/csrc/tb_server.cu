@@ -235,7 +235,7 @@ std::unique_ptr<Job> make_cohort_job(tb_context* ctx, const std::vector<Request*
   const int Hp = (P->Hz + 15) / 16 * 16;
   for (size_t k = 0; k < members.size(); ++k) {
     TB_CUDA_TRY(cudaMemcpyAsync(grid.p, members[k]->init.data(), grid.bytes, cudaMemcpyHostToDevice, P->st));
-    double2* mixed = P->tmpgrid.as<double2>();  // [Nz][Nkm]
+    double2* mixed = P->G.as<double2>();  // [Nz][Nkm] of the step's scratch
     launch_x_rfft(grid.as<double>(), mixed, P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
     double* out = reinterpret_cast<double*>(P->Xp(0) + k * P->Nkm);
     GemmBatch bt{};

@@ -786,47 +786,90 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_xprod_b(XProdArgs a) 
   }
 }
 
-// rfft of real rows (unnormalised), via a complex FFT of the row.
-__global__ void __launch_bounds__(256) k_x_rfft(const double* __restrict__ grid, double2* __restrict__ spec,
+// rfft of real rows (unnormalised), two rows to a complex FFT: rows 2 i and 2 i + 1
+// as real and imaginary part, the spectra separated by conjugate symmetry.  The
+// kernel is bound by the passes' shared-memory round trips, so half the
+// transforms are half the work.  An odd last row goes with zeros.
+__global__ void __launch_bounds__(256) k_x_rfft(const double* __restrict__ grid, double2* __restrict__ spec, int nrows,
                                                 int Nx, FftPlan fp, const double2* __restrict__ tw) {
   extern __shared__ double2 sm[];
   double2* A = sm;
   double2* B = sm + Nx;
-  const int row = blockIdx.x;
+  const int row = 2 * blockIdx.x;
+  const bool two = row + 1 < nrows;
   const int Nk = Nx / 2 + 1;
-  for (int p = threadIdx.x; p < Nx; p += blockDim.x) A[p] = make_double2(grid[(size_t)row * Nx + p], 0.0);
+  const double* g = grid + (size_t)row * Nx;
+  for (int p = threadIdx.x; p < Nx; p += blockDim.x) A[p] = make_double2(g[p], two ? g[Nx + p] : 0.0);
   __syncthreads();
-  double2* R = fft_cta(A, B, fp, tw, -1);
+  const double2* R = fft_cta(A, B, fp, tw, -1);
+  double2* out = spec + (size_t)row * Nk;
   for (int k = threadIdx.x; k < Nk; k += blockDim.x) {
-    double2 v = R[k];
-    if (k == 0 || 2 * k == Nx) v.y = 0.0;
-    spec[(size_t)row * Nk + k] = v;
+    const double2 c = R[k], w = R[k ? Nx - k : 0];
+    const bool edge = k == 0 || 2 * k == Nx;
+    out[k] = make_double2(0.5 * (c.x + w.x), edge ? 0.0 : 0.5 * (c.y - w.y));
+    if (two) out[Nk + k] = make_double2(0.5 * (c.y + w.y), edge ? 0.0 : -0.5 * (c.x - w.x));
   }
 }
 
-// irfft (1/N) of half-spectrum rows, ignoring Im of DC and Nyquist.
-__global__ void __launch_bounds__(256) k_x_irfft(const double2* __restrict__ spec, double* __restrict__ grid,
+// Spectrum entry k of P + i Q from the half spectra P, Q (DC and Nyquist real)
+// of two real rows of length Nx: q = k or Nx - k is the stored bin.
+__device__ __forceinline__ double2 pair_bin(double2 P, double2 Q, int q, int Nx, bool upper) {
+  if (q == 0 || 2 * q == Nx) P.y = Q.y = 0.0;
+  return upper ? pack2_mirror(P, Q) : pack2(P, Q);
+}
+
+// irfft (1/N) of half-spectrum rows, ignoring Im of DC and Nyquist, rows 2 i and
+// 2 i + 1 together.
+__global__ void __launch_bounds__(256) k_x_irfft(const double2* __restrict__ spec, double* __restrict__ grid, int nrows,
                                                  int Nx, FftPlan fp, const double2* __restrict__ tw) {
   extern __shared__ double2 sm[];
   double2* A = sm;
   double2* B = sm + Nx;
-  const int row = blockIdx.x;
+  const int row = 2 * blockIdx.x;
+  const bool two = row + 1 < nrows;
   const int Nk = Nx / 2 + 1;
   const double2* g = spec + (size_t)row * Nk;
   for (int k = threadIdx.x; k < Nx; k += blockDim.x) {
-    double2 v;
-    if (k < Nk) {
-      v = g[k];
-      if (k == 0 || 2 * k == Nx) v.y = 0.0;
-    } else {
-      v = cconj(g[Nx - k]);
-    }
-    A[k] = v;
+    const bool upper = k >= Nk;
+    const int q = upper ? Nx - k : k;
+    A[k] = pair_bin(g[q], two ? g[Nk + q] : make_double2(0.0, 0.0), q, Nx, upper);
   }
   __syncthreads();
-  double2* R = fft_cta(A, B, fp, tw, +1);
+  const double2* R = fft_cta(A, B, fp, tw, +1);
   const double inv = 1.0 / Nx;
-  for (int p = threadIdx.x; p < Nx; p += blockDim.x) grid[(size_t)row * Nx + p] = R[p].x * inv;
+  double* out = grid + (size_t)row * Nx;
+  for (int p = threadIdx.x; p < Nx; p += blockDim.x) {
+    out[p] = R[p].x * inv;
+    if (two) out[Nx + p] = R[p].y * inv;
+  }
+}
+
+// The same from the even / odd Chebyshev half planes of a field (ev at half +
+// (2 f) hplane, ov after it): row j is E + O and its mirror Nz - 1 - j is E - O,
+// so one read of a half row and one FFT give both.  Grid (ceil(Nz/2), fields).
+__global__ void __launch_bounds__(256) k_x_irfft_half(const double2* __restrict__ half, double* __restrict__ grid, int Nz,
+                                                      int Nx, FftPlan fp, const double2* __restrict__ tw) {
+  extern __shared__ double2 sm[];
+  double2* A = sm;
+  double2* B = sm + Nx;
+  const int j = blockIdx.x, jm = Nz - 1 - j, f = blockIdx.y;
+  const int Nk = Nx / 2 + 1, H = (Nz + 1) / 2;
+  const double2* ev = half + ((size_t)(2 * f) * H + j) * Nk;
+  const double2* ov = ev + (size_t)H * Nk;
+  for (int k = threadIdx.x; k < Nx; k += blockDim.x) {
+    const bool upper = k >= Nk;
+    const int q = upper ? Nx - k : k;
+    const double2 e = ev[q], o = ov[q];
+    A[k] = pair_bin(cadd(e, o), csub(e, o), q, Nx, upper);
+  }
+  __syncthreads();
+  const double2* R = fft_cta(A, B, fp, tw, +1);
+  const double inv = 1.0 / Nx;
+  double* out = grid + (size_t)f * Nz * Nx;
+  for (int p = threadIdx.x; p < Nx; p += blockDim.x) {
+    out[(size_t)j * Nx + p] = R[p].x * inv;
+    if (jm != j) out[(size_t)jm * Nx + p] = R[p].y * inv;
+  }
 }
 
 // Dealiased product of two real rows: pad both to M, multiply, truncate back.
@@ -909,6 +952,8 @@ cudaError_t set_transform_smem_limits(int bytes) {
   if ((e = fftr::xprod_r_set_limits<double2, XProdArgs>(bytes)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(k_x_rfft, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess) return e;
   if ((e = cudaFuncSetAttribute(k_x_irfft, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(k_x_irfft_half, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) != cudaSuccess)
+    return e;
   return cudaFuncSetAttribute(k_x_dealias_mul, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
@@ -947,13 +992,19 @@ void launch_xprod_b(const XProdArgs& a, cudaStream_t st) {
 void launch_x_rfft(const double* grid, double2* spec, int nrows, int Nx, const FftPlan& fp, const double2* tw,
                    cudaStream_t st) {
   size_t smem = 2 * (size_t)Nx * sizeof(double2);
-  k_x_rfft<<<nrows, 256, smem, st>>>(grid, spec, Nx, fp, tw);
+  k_x_rfft<<<(nrows + 1) / 2, 256, smem, st>>>(grid, spec, nrows, Nx, fp, tw);
 }
 
 void launch_x_irfft(const double2* spec, double* grid, int nrows, int Nx, const FftPlan& fp, const double2* tw,
                     cudaStream_t st) {
   size_t smem = 2 * (size_t)Nx * sizeof(double2);
-  k_x_irfft<<<nrows, 256, smem, st>>>(spec, grid, Nx, fp, tw);
+  k_x_irfft<<<(nrows + 1) / 2, 256, smem, st>>>(spec, grid, nrows, Nx, fp, tw);
+}
+
+void launch_x_irfft_half(const double2* half, double* grid, int nfields, int Nz, int Nx, const FftPlan& fp,
+                         const double2* tw, cudaStream_t st) {
+  size_t smem = 2 * (size_t)Nx * sizeof(double2);
+  k_x_irfft_half<<<dim3((Nz + 1) / 2, nfields), 256, smem, st>>>(half, grid, Nz, Nx, fp, tw);
 }
 
 void launch_x_dealias_mul(const double* a, const double* b, double* out, int nrows, int Nx, int M,

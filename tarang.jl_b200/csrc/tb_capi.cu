@@ -194,6 +194,12 @@ ClassDev class_dev(tb_plan* P, int sy, int c, FactorSet* f) {
   return cd;
 }
 
+// Band rows the records hold: padded to whole backward windows with one
+// partition (no rows to share out), else the system's npad.
+int solve_rows(const TauSystem& S) {
+  return S.tau_parts == 1 ? (S.lay.cls[0].n + kBwdWin - 1) / kBwdWin * kBwdWin : S.npad;
+}
+
 TauArgs tau_args(tb_plan* P, int sy, FactorSet* f, const double2* rhsP) {
   TauArgs a{};
   a.cls[0] = class_dev(P, sy, 0, f);
@@ -208,7 +214,8 @@ TauArgs tau_args(tb_plan* P, int sy, FactorSet* f, const double2* rhsP) {
   a.X = P->X.as<double2>();
   a.tau = P->tau.as<double2>();
   a.rhsP = rhsP;
-  a.npad = P->sys[sy].npad;
+  a.npad = solve_rows(P->sys[sy]);
+  a.brec = tau_bwd_rec(P->sys[sy].tau_parts);
   a.PP = f ? f->PP.as<double>() : nullptr;
   a.HR = f ? f->HR.as<double>() : nullptr;
   a.rhs_off = P->sys[sy].rhs_off.as<int>();
@@ -254,22 +261,28 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
   fs->beta = beta;
   const int Nk = P->Nk;
   const size_t groups = (size_t)(Nk + kSolveModes - 1) / kSolveModes;
-  const size_t n = S.npad;
+  const size_t n = solve_rows(S);
   auto fit = [](DevBuf& b, size_t bytes) {
     if (b.bytes != bytes) b.alloc(bytes);
   };
-  fit(fs->FR, groups * n * 2 * kFwdRec * kSolveModes * sizeof(double));
-  fit(fs->BR, groups * n * 2 * kBwdRec * kSolveModes * sizeof(double));
-  fit(fs->SI, groups * 2 * 16 * kSolveModes * sizeof(double));
-  fit(fs->PP, tau_transfer_doubles(Nk, S.tau_parts) * sizeof(double));
-  fit(fs->HR, tau_response_doubles(Nk, (int)n, S.tau_parts) * sizeof(double));
-  TB_CUDA_TRY(cudaMemsetAsync(fs->FR.p, 0, fs->FR.bytes, P->st));
-  TB_CUDA_TRY(cudaMemsetAsync(fs->BR.p, 0, fs->BR.bytes, P->st));
-  TB_CUDA_TRY(cudaMemsetAsync(fs->SI.p, 0, fs->SI.bytes, P->st));
+  const bool banded = !S.helm;
+  if (!S.helm) {
+    fit(fs->FR, groups * n * 2 * kFwdRec * kSolveModes * sizeof(double));
+    fit(fs->BR, groups * n * 2 * tau_bwd_rec(S.tau_parts) * kSolveModes * sizeof(double));
+    fit(fs->SI, groups * 2 * 16 * kSolveModes * sizeof(double));
+    TB_CUDA_TRY(cudaMemsetAsync(fs->FR.p, 0, fs->FR.bytes, P->st));
+    TB_CUDA_TRY(cudaMemsetAsync(fs->BR.p, 0, fs->BR.bytes, P->st));
+    TB_CUDA_TRY(cudaMemsetAsync(fs->SI.p, 0, fs->SI.bytes, P->st));
+  }
+  fit(fs->PP, banded ? tau_transfer_doubles(Nk, S.tau_parts) * sizeof(double) : 0);
+  fit(fs->HR, banded ? tau_response_doubles(Nk, (int)n, S.tau_parts) * sizeof(double) : 0);
+  const int rows = S.lay.cls[0].n;
+  fit(fs->DI, (S.helm ? helm_doubles(Nk, rows) : 0) * sizeof(double));
   int neg = 0x7fffffff;
   TB_CUDA_TRY(cudaMemcpyAsync(P->err_mode.p, &neg, sizeof(int), cudaMemcpyHostToDevice, P->st));
   TauArgs a = tau_args(P, sy, fs.get(), nullptr);
-  for (int b = 0; b < P->B; ++b) {  // one factor launch per stacked instance (its own kappa, nu)
+  if (S.helm) launch_helm_factor(a, fs->DI.as<double>(), P->st);
+  for (int b = 0; b < P->B && !S.helm; ++b) {  // one factor launch per stacked instance (its own kappa, nu)
     TauArgs ab = a;
     ab.mode0 = b * P->Nkm;
     if (P->B > 1)
@@ -279,7 +292,7 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
       }
     launch_tau_factor(ab, S.tau_parts, P->st);
   }
-  launch_tau_transfer(a, S.tau_parts, P->st);
+  if (banded) launch_tau_transfer(a, S.tau_parts, P->st);
   check_launch("tau factor");
   int bad = 0;
   TB_CUDA_TRY(cudaMemcpyAsync(&bad, P->err_mode.p, sizeof(int), cudaMemcpyDeviceToHost, P->st));
@@ -292,6 +305,17 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
   }
   S.factors.push_back(std::move(fs));
   return S.factors.back().get();
+}
+
+// The solve of system sy with factor set fs: a's right-hand side into a's state.
+void tau_solve(tb_plan* P, int sy, const FactorSet* fs, const TauArgs& a) {
+  const TauSystem& S = P->sys[sy];
+  timed(P, sy ? "tau_solve_perp" : "tau_solve", [&] {
+    if (S.helm)
+      launch_helm_solve(a, fs->DI.as<double>(), P->st);
+    else
+      launch_tau_solve(a, S.tau_parts, P->st);
+  });
 }
 
 // F = -(u.grad) f in C^(2) rows (sfwd) or T coefficients (fwd) for f = b, ux, uz.
@@ -549,7 +573,7 @@ void enqueue_rk_step_2d(tb_plan* P, double dt) {
         a.t_dev = P->t_dev.as<double>();
         a.bc_toff = ci * dt;
       }
-      timed(P, "tau_solve", [&] { launch_tau_solve(a, P->sys[0].tau_parts, P->st); });
+      tau_solve(P, 0, fs, a);
       nk += 2;
     }
     // the stage solve (i > 0) has written the FP32 copy of X_i
@@ -607,9 +631,9 @@ void enqueue_rk_step(tb_plan* P, double dt) {
         a.t_dev = P->t_dev.as<double>();
         a.bc_toff = ci * dt;
       }
-      timed(P, "tau_solve", [&] { launch_tau_solve(a, P->sys[0].tau_parts, P->st); });
+      tau_solve(P, 0, fs, a);
       TauArgs a2 = tau_args(P, 1, fs2, P->LXP[i].as<double2>());
-      timed(P, "tau_solve_perp", [&] { launch_tau_solve(a2, P->sys[1].tau_parts, P->st); });
+      tau_solve(P, 1, fs2, a2);
       // L X_i = (rhs - M X_i) / beta on the side stream, beside F(X_i)
       fork_side(P);
       timed(P, "lx_finalize", [&] {
@@ -681,7 +705,7 @@ void enqueue_sbdf_step(tb_plan* P, double dt, int order) {
       a.t_dev = P->t_dev.as<double>();
       a.bc_toff = dt;
     }
-    timed(P, "tau_solve", [&] { launch_tau_solve(a, P->sys[0].tau_parts, P->st); });
+    tau_solve(P, 0, fs, a);
   };
   if (P->ndim == 2) {
     // M X (of the state with Im dropped at the DC / Nyquist modes), the
@@ -733,7 +757,7 @@ void enqueue_sbdf_step(tb_plan* P, double dt, int order) {
     TB_CUDA_TRY(cudaMemcpyAsync(P->MXprev.p, MXcur, sizeof(double2) * cnt, cudaMemcpyDeviceToDevice, side(P)));
     solve();
     TauArgs s2 = tau_args(P, 1, fs2, P->Rsb.as<double2>());
-    timed(P, "tau_solve_perp", [&] { launch_tau_solve(s2, P->sys[1].tau_parts, P->st); });
+    tau_solve(P, 1, fs2, s2);
     join_side(P);
     P->kernels_per_step = (P->mixed ? 6 : 5) + 5;
   }
@@ -899,7 +923,7 @@ void tb::plan_set_variant(tb_plan* P, int tau_parts, int xrows) {
     TB_REQUIRE(plan_tau_parts_ok(P, tau_parts), TB_ENOTSUPPORTED, "tau solve partitions must be 1, 4, 8 or 16 and fit");
     for (int sy = 0; sy < P->nsys; ++sy) {
       TauSystem& S = P->sys[sy];
-      if (S.tau_parts == tau_parts) continue;
+      if (S.helm || S.tau_parts == tau_parts) continue;
       TB_CUDA_TRY(cudaStreamSynchronize(P->st));
       S.tau_parts = tau_parts;
       S.factors.clear();  // record layouts differ between the two forms
@@ -957,7 +981,7 @@ size_t tb::plan_device_bytes(const tb_plan* P) {
                              &t.bord,   &t.c2_z,  &t.c2_nz,   &t.c1_z,  &t.c1_nz,    &t.col_code, &t.left_code};
       for (const DevBuf* d : tb_) b += d->bytes;
     }
-    for (const auto& f : S.factors) b += f->FR.bytes + f->BR.bytes + f->SI.bytes + f->PP.bytes + f->HR.bytes;
+    for (const auto& f : S.factors) b += f->FR.bytes + f->BR.bytes + f->SI.bytes + f->PP.bytes + f->HR.bytes + f->DI.bytes;
   }
   b += rbc3d_device_bytes(P) + P->kappa_m.bytes + P->nu_m.bytes;
   for (const DevBuf& d : P->sys[0].mband) b += d.bytes;
@@ -1042,6 +1066,20 @@ long long rhs_code(const tb_plan* P, int sy, int eq, int k) {
   return 2 * ((long long)4 * P->Nz + k) * P->Nk;
 }
 
+// The shape k_helm_factor eliminates: kl = 1, columns r - 1 .. r + 1 and, in row
+// n - 3 alone, r + 2; one border unknown, whose column starts in row 0.
+void require_helmholtz_shape(const TauLayout& lay) {
+  for (const ClassLayout& L : lay.cls) {
+    bool ok = L.kl == 1 && L.ku <= 2 && L.nb == 1 && L.n >= 4;
+    const int w = L.kl + L.ku + 1;
+    for (int r = 0; ok && L.ku == 2 && r < L.n; ++r) {
+      const Coef& c = L.band[(size_t)r * w + 3];
+      if (r != L.n - 3 && (c.m != 0 || c.l0 != 0 || c.l1 != 0 || c.l2 != 0)) ok = false;
+    }
+    TB_REQUIRE(ok, TB_ENOTSUPPORTED, "unexpected shape of the decoupled velocity system");
+  }
+}
+
 // Pad a class's band template to the compiled (kTauKL, kTauKU) shape.
 void pad_band(ClassLayout& L) {
   TB_REQUIRE(L.kl <= kTauKL && L.ku <= kTauKU && L.nb <= 4, TB_ENOTSUPPORTED, "unexpected tau band shape");
@@ -1112,6 +1150,7 @@ void install_system(tb_plan* P, int sy, TauLayout lay) {
   const int n = lay.cls[0].n;
   S.npad = (n + kTauRowPad - 1) / kTauRowPad * kTauRowPad;
   S.tau_parts = default_tau_parts((P->Nk + kSolveModes - 1) / kSolveModes, S.npad);
+  S.helm = sy == 1;
   TB_REQUIRE(tau_solve_smem_bytes(S.npad, S.tau_parts) <= 227 * 1024, TB_ENOTSUPPORTED,
              "Nz too large for the staged tau solve");
   const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, S.tau_parts) * sizeof(double);
@@ -1393,7 +1432,11 @@ void tb::build_plan(tb_plan* P, tb_context* ctx, const tb_problem_desc* descs, i
       upload(P->kappa_m, km);
       upload(P->nu_m, nm);
     }
-    if (d3) install_system(P, 1, build_helmholtz_layout(P->Nz, desc->Lz, desc->nu));
+    if (d3) {
+      TauLayout hl = build_helmholtz_layout(P->Nz, desc->Lz, desc->nu);
+      require_helmholtz_shape(hl);
+      install_system(P, 1, std::move(hl));
+    }
     P->nsys = d3 ? 2 : 1;
     TB_REQUIRE(rk_final_smem_bytes(P->Nz) <= 227 * 1024, TB_ENOTSUPPORTED, "Nz too large for the final RK update");
     P->err_mode.alloc(sizeof(int));

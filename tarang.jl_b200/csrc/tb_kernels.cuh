@@ -180,6 +180,8 @@ constexpr int kFwdRot = kFwdRec - 1;
 constexpr int kBwdCode = 1 + kTauKL + kTauKU + 4;
 constexpr int kBwdG = kBwdCode + 1;
 constexpr int kBwdRec = kBwdG + 4;
+// (with one partition there are no responses: the record ends with the code)
+__host__ __device__ constexpr int tau_bwd_rec(int parts) { return parts == 1 ? kBwdG : kBwdRec; }
 // per-row backward responses H of the partitioned solve: 12 entries (the
 // rows' store codes come from the per-row table TauArgs::xcode)
 constexpr int kHRec = kTauKL + kTauKU;
@@ -248,7 +250,8 @@ struct ClassDev {
 struct TauArgs {
   ClassDev cls[2];
   int Nz, Nk, Nx;
-  int npad;            // band rows padded to a multiple of kTauRowPad
+  int npad;            // band rows padded to a multiple of kTauRowPad (one partition: of kBwdWin)
+  int brec;            // doubles of a backward record (tau_bwd_rec)
   double k0;           // 2 pi / Lx
   const double* kmag;  // per-mode horizontal wavenumber |k| (3D), or null for k0 * m
   double alpha, beta;  // LHS = alpha M + beta L
@@ -292,6 +295,11 @@ struct TauArgs {
 void launch_tau_factor(const TauArgs& a, int parts, cudaStream_t st);
 void launch_tau_transfer(const TauArgs& a, int parts, cudaStream_t st);
 void launch_tau_solve(const TauArgs& a, int parts, cudaStream_t st);
+// The 3D program's decoupled component (build_helmholtz_layout): tridiagonal
+// records HF (helm_doubles) and solve.
+size_t helm_doubles(int Nk, int n);
+void launch_helm_factor(const TauArgs& a, double* HF, cudaStream_t st);
+void launch_helm_solve(const TauArgs& a, const double* HF, cudaStream_t st);
 cudaError_t set_tau_smem_limits(int bytes);
 size_t tau_solve_smem_bytes(int npad, int parts);
 size_t tau_transfer_doubles(int Nk, int parts);

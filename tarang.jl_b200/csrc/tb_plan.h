@@ -99,6 +99,7 @@ struct FactorSet {
   DevBuf FR, BR, SI;  // solve-layout factor records (see tb_kernels.cuh)
   DevBuf PP;          // partition transfer matrices of the solve
   DevBuf HR;          // per-row backward responses of the partitioned solve
+  DevBuf DI;          // tridiagonal records (TauSystem::helm)
 };
 
 // One family of per-mode banded tau systems: the coupled Boussinesq system
@@ -111,6 +112,7 @@ struct TauSystem {
   std::vector<DevBuf> mband, mbord;  // stacked instances: band / border coefficients [instance][class]
   std::vector<std::unique_ptr<FactorSet>> factors;
   int tau_parts = 1;  // partitions of the solve (kTauParts16, kTauParts8, kTauParts or 1)
+  bool helm = false;   // the 3D program's decoupled component: tridiagonal solve
   int npad = 0;       // band rows padded to a multiple of kTauRowPad
 };
 

@@ -54,9 +54,9 @@ __device__ __forceinline__ double* fwd_record(double* FR, int npad, int m, int j
   const int g = m / kSolveModes, mm = m % kSolveModes;
   return FR + ((((size_t)g * npad + j) * 2 + c) * kSolveModes + mm) * kFwdRec;
 }
-__device__ __forceinline__ double* bwd_record(double* BR, int npad, int m, int j, int c) {
+__device__ __forceinline__ double* bwd_record(double* BR, int npad, int brec, int m, int j, int c) {
   const int g = m / kSolveModes, mm = m % kSolveModes;
-  return BR + ((((size_t)g * npad + j) * 2 + c) * kSolveModes + mm) * kBwdRec;
+  return BR + ((((size_t)g * npad + j) * 2 + c) * kSolveModes + mm) * brec;
 }
 
 // ---------------------------------------------------------------------------
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(32 * kFactorWarps) k_tau_factor(TauArgs a) {
     }
     // records of row j (row j itself is final after the swap)
     double* fr = fwd_record(C.FR, a.npad, m, j, c);
-    double* br = bwd_record(C.BR, a.npad, m, j, c);
+    double* br = bwd_record(C.BR, a.npad, a.brec, m, j, c);
     if (lane == 0) {
       fr[0] = __longlong_as_double((long long)(p - j));  // pivot offset, integer bits
     } else if (lane <= KL) {
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(32 * kFactorWarps) k_tau_factor(TauArgs a) {
   // padding rows n..npad-1: identity rows with no right-hand side and no store
   for (int j = n + lane; j < a.npad; j += 32) {
     double* fr = fwd_record(C.FR, a.npad, m, j, c);
-    double* br = bwd_record(C.BR, a.npad, m, j, c);
+    double* br = bwd_record(C.BR, a.npad, a.brec, m, j, c);
     for (int t = 0; t < kFwdRec; ++t) fr[t] = 0.0;
     br[0] = 1.0;
     for (int t = 1; t < kBwdCode; ++t) br[t] = 0.0;
@@ -371,7 +371,7 @@ template <int P>
 __host__ __device__ constexpr size_t part_stage_doubles() {
   constexpr size_t MP = kSolveModes, R = part_rows<P>(), NL = 4 * MP;
   constexpr size_t F = R * (2 * MP * kFwdRec + 2 * 2 * MP);
-  constexpr size_t B = R * (2 * MP * kBwdRec + (ys_global<P>() ? NL : 0));
+  constexpr size_t B = R * (2 * MP * tau_bwd_rec(P) + (ys_global<P>() ? NL : 0));
   constexpr size_t H = R * (2 * MP * kHRec + (P > kTauParts8 ? NL : 0));
   return F > B ? (F > H ? F : H) : (B > H ? B : H);
 }
@@ -437,10 +437,11 @@ __global__ void __launch_bounds__(32 * P / PPW) k_tau_solve(TauArgs a) {
   constexpr int MP = kSolveModes;
   constexpr int W1 = KL + KU + 1;
   constexpr int FREC = 2 * MP * kFwdRec;  // doubles per forward row (both classes)
-  constexpr int BREC = 2 * MP * kBwdRec;  // doubles per backward row
+  constexpr int BR1 = tau_bwd_rec(P);     // doubles of one backward record (no responses with one partition)
+  constexpr int BREC = 2 * MP * BR1;      // doubles per backward row
   constexpr int HREC = 2 * MP * kHRec;    // doubles per H row
   constexpr int RREC = 2 * MP;            // double2 rhs entries per row (class, mode)
-  constexpr int FV = kFwdRec / 2, BV = kBwdRec / 2, HV = kHRec / 2;  // 16-byte words per record
+  constexpr int FV = kFwdRec / 2, BV = BR1 / 2, HV = kHRec / 2;  // 16-byte words per record
   constexpr int NL = 4 * MP;  // distinct lanes of a partition
   constexpr int TPL = 32 / PPW;  // threads per partition (a warp, or a half-warp)
   constexpr int BSUB = 3;     // backward rows whose records are held in registers at once
@@ -755,7 +756,7 @@ __global__ void __launch_bounds__(32 * P / PPW) k_tau_solve(TauArgs a) {
       issue_bwd(s + NSB - 1);
       cp_async_wait<NSB - 1>();  // stage s is resident
       __syncwarp();
-      const double2* st = reinterpret_cast<const double2*>(ring + (size_t)(s % NSB) * BST + (size_t)slot * kBwdRec);
+      const double2* st = reinterpret_cast<const double2*>(ring + (size_t)(s % NSB) * BST + (size_t)slot * BR1);
 #pragma unroll
       for (int h = 0; h < R / BSUB; ++h) {
         // rows q0 + kBwdWin - 1 - u for u = hs R + h BSUB + w; stage row index R - 1 - (h BSUB + w)
@@ -776,8 +777,10 @@ __global__ void __launch_bounds__(32 * P / PPW) k_tau_solve(TauArgs a) {
           else
             acc0 = *yx;
           double acc1 = 0.0, acc2 = 0.0;
+          if constexpr (P > 1) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) acc2 = fma(rec(kBwdG + i), d[i], acc2);  // y correction G d
+            for (int i = 0; i < 4; ++i) acc2 = fma(rec(kBwdG + i), d[i], acc2);  // y correction G d
+          }
 #pragma unroll
           for (int b = 0; b < NBMAX; ++b) acc1 = fma(-rec(W1 + b), x1[b], acc1);
 #pragma unroll
@@ -1004,7 +1007,7 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
           yj = yt;
         }
       }
-      bwd_record(a.cls[0].BR, np, m, j, c)[kBwdG + i] = yj;
+      bwd_record(a.cls[0].BR, np, a.brec, m, j, c)[kBwdG + i] = yj;
       for (int t = 1; t <= KL; ++t) y[(u + t) % kFwdWin] = fma(-fr[t], yj, y[(u + t) % kFwdWin]);
       for (int b = 0; b < NBMAX; ++b) z[b] = fma(-fr[1 + KL + b], yj, z[b]);
       y[u] = 0.0;
@@ -1018,7 +1021,7 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
   double xw[kBwdWin];
   for (int t = 0; t < kBwdWin; ++t) xw[t] = (t == ib) ? 1.0 : 0.0;
   for (int j = r1 - 1; j >= r0; --j) {
-    const double* br = bwd_record(a.cls[0].BR, np, m, j, c);
+    const double* br = bwd_record(a.cls[0].BR, np, a.brec, m, j, c);
     double acc = 0.0;
     for (int t = 1; t <= KL + KU; ++t) acc = fma(-br[t], xw[(j + t) % kBwdWin], acc);
     xw[j % kBwdWin] = acc * br[0];
@@ -1026,6 +1029,124 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
     hr[ib] = xw[j % kBwdWin];
   }
   for (int o = 0; o < kBwdWin; ++o) tr[kTrPsi + ib * kBwdWin + o] = xw[o];  // Psi^T: row ib
+}
+
+// ---------------------------------------------------------------------------
+// The decoupled velocity component of the 3D program: per (mode, class) a
+// tridiagonal block (plus one entry, the tau column's in row n - 3) with one
+// border unknown and one boundary row, solved without pivoting (a pivot is
+// never smaller than the entry below it; the factorisation checks that and
+// reports the mode otherwise).  Five numbers a row against the 28 of the general
+// band records, and half the rows' padding; thread = mode, so every load is a
+// coalesced row of modes.  Bound by HBM: 169 MB of records and 4 passes over a
+// plane at 256x256x128.
+//   HF[class][field][row][mode]: 0 l (multiplier of row r + 1), 1 cq (of the
+//   boundary row), 2 1 / d, 3 u (column r + 1), 4 e (border column), then
+//   HF + 10 n Nk: [class][0 v (column n - 1 of row n - 3), 1 1 / Schur][mode].
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_helm_factor(TauArgs a, double* __restrict__ HF) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+  if (m >= a.Nk) return;
+  const ClassDev& C = a.cls[c];
+  const int n = C.n, cw = C.kl + C.ku + 1;
+  const size_t Nk = a.Nk, fld = (size_t)n * Nk;
+  const double kx = a.kmag[m];
+  auto A = [&](int r, int col) -> double {
+    return (r < n && col < n) ? coef_val(C.band[(size_t)r * cw + col - r + C.kl], a.alpha, a.beta, kx) : 0.0;
+  };
+  auto bnd = [&](int col) -> double { return col < n ? a.beta * C.c2_nz[col] : 0.0; };
+  double* R = HF + (size_t)c * 5 * fld + m;
+  double d = A(0, 0), u = A(0, 1), v = A(0, 2), e = coef_val(C.bord[0], a.alpha, a.beta, kx);
+  double c0 = bnd(0), c1 = bnd(1), cs = a.beta * C.c1_nz[0];
+  double vk = 0.0;
+  bool bad = false;
+  for (int r = 0; r < n; ++r) {
+    const double below = A(r + 1, r), dinv = 1.0 / d, l = below * dinv, cq = c0 * dinv;
+    bad = bad || !(fabs(d) > 0.0) || !isfinite(d) || fabs(below) > fabs(d);
+    if (r == n - 3) vk = v;
+    R[(size_t)r * Nk] = l;
+    R[fld + (size_t)r * Nk] = cq;
+    R[2 * fld + (size_t)r * Nk] = dinv;
+    R[3 * fld + (size_t)r * Nk] = u;
+    R[4 * fld + (size_t)r * Nk] = e;
+    cs -= cq * e;
+    c0 = c1 - cq * u;
+    c1 = bnd(r + 2) - cq * v;
+    d = A(r + 1, r + 1) - l * u;
+    u = A(r + 1, r + 2) - l * v;
+    v = A(r + 1, r + 3);
+    e = (r + 1 < n ? coef_val(C.bord[r + 1], a.alpha, a.beta, kx) : 0.0) - l * e;
+  }
+  if (bad || !(fabs(cs) > 0.0) || !isfinite(cs)) atomicMin(a.err_mode, m);
+  double* S = HF + 10 * fld + (size_t)c * 2 * Nk + m;
+  S[0] = vk;
+  S[Nk] = 1.0 / cs;
+}
+
+// One solve; right-hand side plane 4 of rhsP (row k of class c: k = c + 2 r),
+// unknowns to X plane 4 (border k = c, band column r: k = c + 2 r + 2) and the
+// tau row of the last column.  y passes through X.  Row loads are issued HU
+// ahead of the recurrence.
+__global__ void __launch_bounds__(128) k_helm_solve(TauArgs a, const double* __restrict__ HF) {
+  constexpr int HU = 4;
+  const int m = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+  if (m >= a.Nk) return;
+  const int n = a.cls[c].n, Nz = a.Nz;
+  const size_t Nk = a.Nk, fld = (size_t)n * Nk;
+  const double* R = HF + (size_t)c * 5 * fld + m;
+  const double* S = HF + 10 * fld + (size_t)c * 2 * Nk + m;
+  const double2* rhs = a.rhsP + ((size_t)4 * Nz + c) * Nk + m;  // row r at rhs + 2 r Nk
+  double2* x = a.X + ((size_t)4 * Nz + c) * Nk + m;             // coefficient c + 2 q at x + 2 q Nk
+  double2* last = a.X + (size_t)(a.cls[c].col_code[n - 1] >> 1) + m;
+  auto slot = [&](int r) -> double2& { return r < n - 1 ? x[2 * (size_t)(r + 1) * Nk] : *last; };
+  double2 y = make_double2(0.0, 0.0), z = y;
+  double lp = 0.0;
+  for (int r0 = 0; r0 < n; r0 += HU) {
+    double2 f[HU];
+    double l[HU], q[HU];
+#pragma unroll
+    for (int i = 0; i < HU; ++i) {
+      const int r = min(r0 + i, n - 1);
+      f[i] = rhs[2 * (size_t)r * Nk];
+      l[i] = R[(size_t)r * Nk];
+      q[i] = R[fld + (size_t)r * Nk];
+    }
+#pragma unroll
+    for (int i = 0; i < HU; ++i)
+      if (r0 + i < n) {
+        y = cfma(-lp, y, f[i]);
+        lp = l[i];
+        z = cfma(-q[i], y, z);
+        slot(r0 + i) = y;
+      }
+  }
+  const double v = S[0], si = S[Nk];
+  const double2 x1 = make_double2(si * z.x, si * z.y);
+  x[0] = x1;
+  double2 xa = make_double2(0.0, 0.0), xb = xa;  // x_{r+1}, x_{r+2}
+  for (int r0 = n - 1; r0 >= 0; r0 -= HU) {
+    double2 f[HU];
+    double di[HU], u[HU], e[HU];
+#pragma unroll
+    for (int i = 0; i < HU; ++i) {
+      const int r = max(r0 - i, 0);
+      f[i] = slot(r);
+      di[i] = R[2 * fld + (size_t)r * Nk];
+      u[i] = R[3 * fld + (size_t)r * Nk];
+      e[i] = R[4 * fld + (size_t)r * Nk];
+    }
+#pragma unroll
+    for (int i = 0; i < HU; ++i)
+      if (r0 - i >= 0) {
+        const int r = r0 - i;
+        double2 acc = cfma(-e[i], x1, f[i]);
+        if (r == n - 3) acc = cfma(-v, xb, acc);
+        acc = cfma(-u[i], xa, acc);
+        xb = xa;
+        xa = make_double2(acc.x * di[i], acc.y * di[i]);
+        slot(r) = xa;
+      }
+  }
 }
 
 template <int N>
@@ -1416,23 +1537,15 @@ void launch_tau_transfer(const TauArgs& a, int parts, cudaStream_t st) {
 }
 void launch_tau_solve(const TauArgs& a, int parts, cudaStream_t st) { solve_impl<kTauKL, kTauKU>(a, parts, st); }
 
-
-void launch_lincomb(const LinComb& lc, double2* out, long long count, cudaStream_t st) {
-  int blocks = (int)((count + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (blocks < 1) blocks = 1;
-#define TB_LINCOMB_CASE(N) \
-  case N:                    \
-    k_lincomb<N><<<blocks, 256, 0, st>>>(lc, out, count); \
-    break;
-  switch (lc.n) {
-    TB_LINCOMB_CASE(1) TB_LINCOMB_CASE(2) TB_LINCOMB_CASE(3) TB_LINCOMB_CASE(4) TB_LINCOMB_CASE(5) TB_LINCOMB_CASE(6)
-    TB_LINCOMB_CASE(7) TB_LINCOMB_CASE(8) TB_LINCOMB_CASE(9) TB_LINCOMB_CASE(10) TB_LINCOMB_CASE(11) TB_LINCOMB_CASE(12)
-    default:
-      throw Error{TB_EINVAL, "linear combination of more than 12 stage vectors"};
-  }
-#undef TB_LINCOMB_CASE
+size_t helm_doubles(int Nk, int n) { return (size_t)Nk * (10 * (size_t)n + 4); }
+void launch_helm_factor(const TauArgs& a, double* HF, cudaStream_t st) {
+  k_helm_factor<<<dim3((a.Nk + 127) / 128, 2), 128, 0, st>>>(a, HF);
 }
+void launch_helm_solve(const TauArgs& a, const double* HF, cudaStream_t st) {
+  k_helm_solve<<<dim3((a.Nk + 127) / 128, 2), 128, 0, st>>>(a, HF);
+}
+
+
 
 void launch_advance_time(double* t, double dt, cudaStream_t st) { k_advance_time<<<1, 1, 0, st>>>(t, dt); }
 

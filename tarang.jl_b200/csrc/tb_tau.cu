@@ -1497,7 +1497,8 @@ cudaError_t set_tau_smem_limits(int bytes) {
   const void* fns[] = {(const void*)k_rk_final<1>,  (const void*)k_rk_final<2>,  (const void*)k_rk_final<3>,
                        (const void*)k_rk_final<4>,  (const void*)k_rk_final<5>,  (const void*)k_rk_final<6>,
                        (const void*)k_rk_final<7>,  (const void*)k_rk_final<8>,  (const void*)k_rk_final<9>,
-                       (const void*)k_rk_final<10>, (const void*)k_rk_final<11>, (const void*)k_rk_final<12>};
+                       (const void*)k_rk_final<10>, (const void*)k_rk_final<11>, (const void*)k_rk_final<12>,
+                       (const void*)k_stage_final};
   for (const void* fn : fns) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;

@@ -265,7 +265,7 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
   auto fit = [](DevBuf& b, size_t bytes) {
     if (b.bytes != bytes) b.alloc(bytes);
   };
-  const bool banded = !S.helm;
+  const bool banded = !S.dense && !S.helm;
   if (!S.helm) {
     fit(fs->FR, groups * n * 2 * kFwdRec * kSolveModes * sizeof(double));
     fit(fs->BR, groups * n * 2 * tau_bwd_rec(S.tau_parts) * kSolveModes * sizeof(double));
@@ -277,7 +277,7 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
   fit(fs->PP, banded ? tau_transfer_doubles(Nk, S.tau_parts) * sizeof(double) : 0);
   fit(fs->HR, banded ? tau_response_doubles(Nk, (int)n, S.tau_parts) * sizeof(double) : 0);
   const int rows = S.lay.cls[0].n;
-  fit(fs->DI, (S.helm ? helm_doubles(Nk, rows) : 0) * sizeof(double));
+  fit(fs->DI, (S.dense ? tau_dense_doubles(Nk, rows) : S.helm ? helm_doubles(Nk, rows) : 0) * sizeof(double));
   int neg = 0x7fffffff;
   TB_CUDA_TRY(cudaMemcpyAsync(P->err_mode.p, &neg, sizeof(int), cudaMemcpyHostToDevice, P->st));
   TauArgs a = tau_args(P, sy, fs.get(), nullptr);
@@ -292,6 +292,7 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
       }
     launch_tau_factor(ab, S.tau_parts, P->st);
   }
+  if (S.dense) launch_tau_dense(a, fs->DI.as<double>(), P->st);
   if (banded) launch_tau_transfer(a, S.tau_parts, P->st);
   check_launch("tau factor");
   int bad = 0;
@@ -313,6 +314,8 @@ void tau_solve(tb_plan* P, int sy, const FactorSet* fs, const TauArgs& a) {
   timed(P, sy ? "tau_solve_perp" : "tau_solve", [&] {
     if (S.helm)
       launch_helm_solve(a, fs->DI.as<double>(), P->st);
+    else if (S.dense)
+      launch_tau_apply(a, fs->DI.as<double>(), P->st);
     else
       launch_tau_solve(a, S.tau_parts, P->st);
   });
@@ -923,9 +926,10 @@ void tb::plan_set_variant(tb_plan* P, int tau_parts, int xrows) {
     TB_REQUIRE(plan_tau_parts_ok(P, tau_parts), TB_ENOTSUPPORTED, "tau solve partitions must be 1, 4, 8 or 16 and fit");
     for (int sy = 0; sy < P->nsys; ++sy) {
       TauSystem& S = P->sys[sy];
-      if (S.helm || S.tau_parts == tau_parts) continue;
+      if (S.helm || (S.tau_parts == tau_parts && !S.dense)) continue;
       TB_CUDA_TRY(cudaStreamSynchronize(P->st));
       S.tau_parts = tau_parts;
+      S.dense = false;
       S.factors.clear();  // record layouts differ between the two forms
       const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, tau_parts) * sizeof(double);
       if (ys > P->solve_scratch.bytes) P->solve_scratch.alloc(ys);
@@ -1116,6 +1120,15 @@ int default_tau_parts(int groups, int npad) {
   return fits(kTauParts16) ? kTauParts16 : 1;
 }
 
+// Whether the systems are solved by their dense inverses: those of all modes
+// have to stay in L2 beside the step's planes.  One solve, event-timed, dense
+// against the best partitioning: 96x24 (2 MB) 8.7 against 16.0 us, 256x64 (34 MB)
+// 14.2 against 22.6, 192x76 (36 MB) 14.8 against 25.0, 512x48 (39 MB) 17.8 against
+// 19.8.
+bool default_tau_dense(int Nk, int n) {
+  return n + 4 <= kDenseMax && tau_dense_doubles(Nk, n) * sizeof(double) <= (size_t)40 << 20;
+}
+
 void install_system(tb_plan* P, int sy, TauLayout lay) {
   TauSystem& S = P->sys[sy];
   auto to_int = [](long long v) {
@@ -1151,6 +1164,7 @@ void install_system(tb_plan* P, int sy, TauLayout lay) {
   S.npad = (n + kTauRowPad - 1) / kTauRowPad * kTauRowPad;
   S.tau_parts = default_tau_parts((P->Nk + kSolveModes - 1) / kSolveModes, S.npad);
   S.helm = sy == 1;
+  S.dense = !S.helm && default_tau_dense(P->Nk, n);
   TB_REQUIRE(tau_solve_smem_bytes(S.npad, S.tau_parts) <= 227 * 1024, TB_ENOTSUPPORTED,
              "Nz too large for the staged tau solve");
   const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, S.tau_parts) * sizeof(double);
@@ -1759,8 +1773,10 @@ tb_status tb_plan_tune(tb_plan* P, double dt, int trial_steps, int* tau_parts, i
     PlanSnapshot snap;
     plan_snapshot(P, &snap);
     std::vector<int> parts_c, rows_c;
+    // (systems solved by their inverses stay so: 0 keeps them)
     for (int p : {kTauParts16, kTauParts8, kTauParts, 1})
-      if (plan_tau_parts_ok(P, p)) parts_c.push_back(p);
+      if (!P->sys[0].dense && plan_tau_parts_ok(P, p)) parts_c.push_back(p);
+    if (parts_c.empty()) parts_c.push_back(0);
     if (P->ndim == 3) {
       for (int r : {1, 2, 4})
         if (rbc3d_xrows_ok(P, r)) rows_c.push_back(r);
@@ -1786,11 +1802,11 @@ tb_status tb_plan_tune(tb_plan* P, double dt, int trial_steps, int* tau_parts, i
         plan_restore(P, snap);
         if (ms < best) {
           best = ms;
-          bp = pc;
+          if (pc > 0) bp = pc;
           br = rc;
         }
       }
-    plan_set_variant(P, bp, br);
+    plan_set_variant(P, P->sys[0].dense ? 0 : bp, br);
     // then, in 3D, the side stream on or off, on a longer trial (the difference
     // is a few percent)
     const int ov_steps = std::max(trial_steps, 10);

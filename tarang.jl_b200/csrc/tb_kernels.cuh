@@ -300,6 +300,13 @@ void launch_tau_solve(const TauArgs& a, int parts, cudaStream_t st);
 size_t helm_doubles(int Nk, int n);
 void launch_helm_factor(const TauArgs& a, double* HF, cudaStream_t st);
 void launch_helm_solve(const TauArgs& a, const double* HF, cudaStream_t st);
+// Dense form of small systems (n + 4 <= kDenseMax): the inverses of all modes
+// from the factor records, and the solve as a product with them.
+constexpr int kDenseMax = 160;
+int tau_dense_ld(int n);
+size_t tau_dense_doubles(int Nk, int n);
+void launch_tau_dense(const TauArgs& a, double* DI, cudaStream_t st);
+void launch_tau_apply(const TauArgs& a, const double* DI, cudaStream_t st);
 cudaError_t set_tau_smem_limits(int bytes);
 size_t tau_solve_smem_bytes(int npad, int parts);
 size_t tau_transfer_doubles(int Nk, int parts);

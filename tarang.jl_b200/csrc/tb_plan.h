@@ -99,7 +99,7 @@ struct FactorSet {
   DevBuf FR, BR, SI;  // solve-layout factor records (see tb_kernels.cuh)
   DevBuf PP;          // partition transfer matrices of the solve
   DevBuf HR;          // per-row backward responses of the partitioned solve
-  DevBuf DI;          // tridiagonal records (TauSystem::helm)
+  DevBuf DI;          // dense inverses (TauSystem::dense) or tridiagonal records (TauSystem::helm)
 };
 
 // One family of per-mode banded tau systems: the coupled Boussinesq system
@@ -113,6 +113,7 @@ struct TauSystem {
   std::vector<std::unique_ptr<FactorSet>> factors;
   int tau_parts = 1;  // partitions of the solve (kTauParts16, kTauParts8, kTauParts or 1)
   bool helm = false;   // the 3D program's decoupled component: tridiagonal solve
+  bool dense = false;  // small systems: solved by their inverses instead (until a partitioning is set)
   int npad = 0;       // band rows padded to a multiple of kTauRowPad
 };
 

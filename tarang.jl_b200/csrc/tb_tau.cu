@@ -1032,6 +1032,167 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
 }
 
 // ---------------------------------------------------------------------------
+// Small systems: the solve as one product with the dense inverse.  The banded
+// sweeps are a chain of about 4 n dependent steps, 14 us at n = 64 whatever the
+// partitions, while the inverses of a small grid's modes fit L2 (4.8 MB at
+// 128x32, 38 MB at 256x64) and their product with the right-hand sides is a
+// sum over n terms in any order.
+//
+// DI[mode][class][output o][input j], j fastest: inputs are the n band rows and
+// the 4 boundary rows, outputs the n band columns and the 4 border unknowns
+// (tau_dense_ld(n) entries a row, the spare ones zero).
+// ---------------------------------------------------------------------------
+
+// Column j of the inverse by one thread, (mode, class) by one block: the sweeps
+// of k_tau_solve on a unit right-hand side.  The block's records (n rows) are
+// staged in shared memory first, where every thread reads the same ones; the
+// column's y and x live in DI, written 32 columns a warp.
+constexpr int kDenseRec = kFwdRec + kBwdCode;  // pivot, multipliers; 1 / d, U, border
+template <int KL, int KU>
+__global__ void k_tau_dense(TauArgs a, double* __restrict__ DI, int ld) {
+  extern __shared__ double drec[];  // [row < npad][kDenseRec], identity rows past n
+  const int m = blockIdx.x, c = blockIdx.y, j = threadIdx.x;
+  const int n = a.cls[c].n, np = a.npad, n_out = n + NBMAX;
+  for (int q = threadIdx.x; q < np * kDenseRec; q += blockDim.x) {
+    const int row = q / kDenseRec, t = q - row * kDenseRec;
+    drec[q] = t < kFwdRec ? fwd_record(a.cls[0].FR, np, m, row, c)[t]
+                          : bwd_record(a.cls[0].BR, np, a.brec, m, row, c)[t - kFwdRec];
+  }
+  __syncthreads();
+  if (j >= ld) return;
+  double* col = DI + ((size_t)m * 2 + c) * n_out * ld + j;
+  double y[kFwdWin], z[NBMAX];
+#pragma unroll
+  for (int t = 0; t < kFwdWin; ++t) y[t] = (t == j) ? 1.0 : 0.0;
+#pragma unroll
+  for (int b = 0; b < NBMAX; ++b) z[b] = (j == n + b) ? 1.0 : 0.0;
+  for (int s = 0; s < np; s += kFwdWin) {
+#pragma unroll
+    for (int u = 0; u < kFwdWin; ++u) {
+      const double* fr = drec + (s + u) * kDenseRec;
+      const int p = __double2loint(fr[0]);
+      double yj = y[u];
+#pragma unroll
+      for (int t = 1; t <= KL; ++t) {
+        const bool sw = (t == p);
+        const double yt = y[(u + t) % kFwdWin];
+        y[(u + t) % kFwdWin] = sw ? yj : yt;
+        yj = sw ? yt : yj;
+      }
+      if (s + u < n) col[(size_t)(s + u) * ld] = yj;
+#pragma unroll
+      for (int t = 1; t <= KL; ++t) y[(u + t) % kFwdWin] = fma(-fr[t], yj, y[(u + t) % kFwdWin]);
+#pragma unroll
+      for (int b = 0; b < NBMAX; ++b) z[b] = fma(-fr[1 + KL + b], yj, z[b]);
+      y[u] = (s + u + kFwdWin == j && j < n) ? 1.0 : 0.0;
+    }
+  }
+  double x1[NBMAX];
+  const double* si = a.cls[0].SI + ((size_t)(m / kSolveModes) * 2 + c) * NBMAX * NBMAX * kSolveModes + m % kSolveModes;
+#pragma unroll
+  for (int q = 0; q < NBMAX; ++q) {
+    double acc = 0.0;
+#pragma unroll
+    for (int b = 0; b < NBMAX; ++b) acc = fma(si[(q * NBMAX + b) * kSolveModes], z[b], acc);
+    x1[q] = acc;
+    col[(size_t)(n + q) * ld] = acc;
+  }
+  double xw[kBwdWin];
+#pragma unroll
+  for (int t = 0; t < kBwdWin; ++t) xw[t] = 0.0;
+  for (int q0 = np - kBwdWin; q0 >= 0; q0 -= kBwdWin) {
+#pragma unroll
+    for (int u = kBwdWin - 1; u >= 0; --u) {
+      const int row = q0 + u;
+      const double* br = drec + row * kDenseRec + kFwdRec;
+      double acc = row < n ? col[(size_t)row * ld] : 0.0;
+#pragma unroll
+      for (int b = 0; b < NBMAX; ++b) acc = fma(-br[KL + KU + 1 + b], x1[b], acc);
+#pragma unroll
+      for (int t = KL + KU; t >= 1; --t) acc = fma(-br[t], xw[(u + t) % kBwdWin], acc);
+      xw[u] = acc * br[0];
+      if (row < n) col[(size_t)row * ld] = xw[u];
+    }
+  }
+}
+
+// The product, one block per (mode, class): lane l holds the right-hand sides
+// l, l + 32, ... (real and imaginary column) in registers and walks four rows of
+// the inverse at a time (4 NQ coalesced loads in flight); the eight sums meet
+// by shuffles.  Bound by the latency of two dependent loads and the L2 rate.
+template <int NQ>
+__global__ void __launch_bounds__(256) k_tau_apply(TauArgs a, const double* __restrict__ DI, int ld) {
+  const int m = blockIdx.x, c = blockIdx.y, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int n = a.cls[c].n, nb = a.cls[c].nb, n_out = n + NBMAX, Nk = a.Nk;
+  const double* M = DI + ((size_t)m * 2 + c) * n_out * ld;
+  double re[NQ], im[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) {
+    const int j = lane + 32 * q;
+    re[q] = im[q] = 0.0;
+    if (j < n) {
+      const int code = a.rhs_off[2 * j + c];
+      if (code >= 0) {
+        const double2 v = a.rhsP[(size_t)(code >> 1) + m];
+        re[q] = (code & 1) ? v.y : v.x;  // -i v on the u_x momentum rows
+        im[q] = (code & 1) ? -v.x : v.y;
+      }
+    } else if (j - n < nb) {
+      const int b = j - n;
+      if (m % a.Nkm == 0) re[q] = a.beta * a.cls[c].bc_rhs[b];
+      if (b == 0 && a.bcdyn != nullptr) {  // the parity combination of the walls, as in k_tau_solve
+        const double t = *a.t_dev + a.bc_toff;
+        const double2 v0b = a.bcdyn[m], v1b = a.bcdyn[Nk + m], v0t = a.bcdyn[2 * (size_t)Nk + m],
+                      v1t = a.bcdyn[3 * (size_t)Nk + m];
+        const double2 bot = cfma(t, v1b, v0b), top = cfma(t, v1t, v0t);
+        re[q] = a.beta * 0.5 * (c == 0 ? top.x + bot.x : top.x - bot.x);
+        im[q] = a.beta * 0.5 * (c == 0 ? top.y + bot.y : top.y - bot.y);
+      }
+    }
+  }
+  double* Xd = reinterpret_cast<double*>(a.X);
+  for (int o0 = 4 * warp; o0 < n_out; o0 += 32) {
+    double w[4][NQ];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q)
+        w[r][q] = (o0 + r < n_out && lane + 32 * q < ld) ? M[(size_t)(o0 + r) * ld + lane + 32 * q] : 0.0;
+    double s[8];  // row r, column p at 2 r + p
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      s[2 * r] = s[2 * r + 1] = 0.0;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        s[2 * r] = fma(w[r][q], re[q], s[2 * r]);
+        s[2 * r + 1] = fma(w[r][q], im[q], s[2 * r + 1]);
+      }
+    }
+    // halving exchange: after the three steps lane l holds the sum number
+    // (l >> 2) & 7 over the lanes that share its two low bits
+#pragma unroll
+    for (int h = 4, bit = 16; h >= 1; h /= 2, bit /= 2) {
+      const bool up = lane & bit;
+#pragma unroll
+      for (int i = 0; i < h; ++i) {
+        const double keep = up ? s[i + h] : s[i], give = up ? s[i] : s[i + h];
+        s[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+      }
+    }
+    double v = s[0];
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    if ((lane & 3) == 0) {
+      const int id = lane >> 2, o = o0 + (id >> 1), part = id & 1;
+      if (o < n)
+        store_unknown(Xd, a.cls[c].col_code[o], m, part, v, true, a.X32, a.x32_lim);
+      else if (o - n < nb)
+        store_unknown(Xd, a.cls[c].left_code[o - n], m, part, v, true, a.X32, a.x32_lim);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // The decoupled velocity component of the 3D program: per (mode, class) a
 // tridiagonal block (plus one entry, the tau column's in row n - 3) with one
 // border unknown and one boundary row, solved without pivoting (a pivot is
@@ -1498,7 +1659,7 @@ cudaError_t set_tau_smem_limits(int bytes) {
                        (const void*)k_rk_final<4>,  (const void*)k_rk_final<5>,  (const void*)k_rk_final<6>,
                        (const void*)k_rk_final<7>,  (const void*)k_rk_final<8>,  (const void*)k_rk_final<9>,
                        (const void*)k_rk_final<10>, (const void*)k_rk_final<11>, (const void*)k_rk_final<12>,
-                       (const void*)k_stage_final};
+                       (const void*)k_stage_final,  (const void*)k_tau_dense<kTauKL, kTauKU>};
   for (const void* fn : fns) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
@@ -1546,7 +1707,45 @@ void launch_helm_solve(const TauArgs& a, const double* HF, cudaStream_t st) {
   k_helm_solve<<<dim3((a.Nk + 127) / 128, 2), 128, 0, st>>>(a, HF);
 }
 
+int tau_dense_ld(int n) { return (n + NBMAX + 3) / 4 * 4; }
+size_t tau_dense_doubles(int Nk, int n) { return (size_t)Nk * 2 * (n + NBMAX) * tau_dense_ld(n); }
 
+void launch_tau_dense(const TauArgs& a, double* DI, cudaStream_t st) {
+  const int ld = tau_dense_ld(a.cls[0].n);
+  const size_t smem = (size_t)a.npad * kDenseRec * sizeof(double);
+  k_tau_dense<kTauKL, kTauKU><<<dim3(a.Nk, 2), (ld + 31) / 32 * 32, smem, st>>>(a, DI, ld);
+}
+
+void launch_tau_apply(const TauArgs& a, const double* DI, cudaStream_t st) {
+  const int ld = tau_dense_ld(a.cls[0].n);
+  const dim3 grid(a.Nk, 2);
+  switch ((ld + 31) / 32) {
+    case 1: k_tau_apply<1><<<grid, 256, 0, st>>>(a, DI, ld); break;
+    case 2: k_tau_apply<2><<<grid, 256, 0, st>>>(a, DI, ld); break;
+    case 3: k_tau_apply<3><<<grid, 256, 0, st>>>(a, DI, ld); break;
+    case 4: k_tau_apply<4><<<grid, 256, 0, st>>>(a, DI, ld); break;
+    case 5: k_tau_apply<5><<<grid, 256, 0, st>>>(a, DI, ld); break;
+    default: throw Error{TB_EINVAL, "system too large for the dense solve"};
+  }
+}
+
+
+void launch_lincomb(const LinComb& lc, double2* out, long long count, cudaStream_t st) {
+  int blocks = (int)((count + 255) / 256);
+  if (blocks > 148 * 16) blocks = 148 * 16;
+  if (blocks < 1) blocks = 1;
+#define TB_LINCOMB_CASE(N) \
+  case N:                    \
+    k_lincomb<N><<<blocks, 256, 0, st>>>(lc, out, count); \
+    break;
+  switch (lc.n) {
+    TB_LINCOMB_CASE(1) TB_LINCOMB_CASE(2) TB_LINCOMB_CASE(3) TB_LINCOMB_CASE(4) TB_LINCOMB_CASE(5) TB_LINCOMB_CASE(6)
+    TB_LINCOMB_CASE(7) TB_LINCOMB_CASE(8) TB_LINCOMB_CASE(9) TB_LINCOMB_CASE(10) TB_LINCOMB_CASE(11) TB_LINCOMB_CASE(12)
+    default:
+      throw Error{TB_EINVAL, "linear combination of more than 12 stage vectors"};
+  }
+#undef TB_LINCOMB_CASE
+}
 
 void launch_advance_time(double* t, double dt, cudaStream_t st) { k_advance_time<<<1, 1, 0, st>>>(t, dt); }
 

@@ -1863,6 +1863,7 @@ tb_status tb_plan_tune(tb_plan* P, double dt, int trial_steps, int* tau_parts, i
       }
     }
     plan_restore(P, snap);
+    plan_prepare(P, dt, 1);  // factors and step graph of the choice: the next step only launches
     if (tau_parts) *tau_parts = bp;
     if (xrows) *xrows = br;
   });

@@ -24,6 +24,7 @@
 
 #include <cuda_runtime.h>
 
+#include "tb_chain.cuh"
 #include "tb_fft.cuh"
 #include "tb_internal.h"
 
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(NT, CTAS) k_xprod_r(Args a) {
   C* A = reinterpret_cast<C*>(xr_raw);
   C* tw = A + 4 * Ms;
   for (int t = threadIdx.x; t < a.rp.ntw; t += NT) tw[t] = a.iptw[t];
+  grid_wait();
   const int z = blockIdx.x, zm = a.Nz - 1 - z;
   const bool lower = z <= zm;
   const size_t ld = a.ld > 0 ? (size_t)a.ld : (size_t)Nk, col0 = (size_t)blockIdx.y * Nk;
@@ -383,9 +385,9 @@ inline void launch_xprod_r_t(const Args& a, cudaStream_t st) {
   const size_t smem = xprod_r_smem_bytes<C>(a.M, a.rp.ntw);
   const dim3 grid(a.Nz, a.instances > 0 ? a.instances : 1);
   if (2 * smem <= 227 * 1024)
-    k_xprod_r<256, 2, C, Args><<<grid, 256, smem, st>>>(a);
+    launch_chained(k_xprod_r<256, 2, C, Args>, grid, 256, smem, st, a);
   else
-    k_xprod_r<512, 1, C, Args><<<grid, 512, smem, st>>>(a);
+    launch_chained(k_xprod_r<512, 1, C, Args>, grid, 512, smem, st, a);
 }
 
 template <class C, class Args>

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include "tb_chain.cuh"
 #include "tb_internal.h"
 
 namespace tb {

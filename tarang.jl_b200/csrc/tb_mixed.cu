@@ -23,6 +23,7 @@ namespace {
 namespace F = tb::fftg;
 
 __global__ void k_round_f32(const double2* __restrict__ in, float2* __restrict__ out, long long n) {
+  grid_wait(in);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const double2 v = in[i];
     out[i] = make_float2((float)v.x, (float)v.y);
@@ -39,6 +40,7 @@ constexpr int SBM = 64, SBN = 64, SBK = 16, STH = 256;
 
 template <class OutT>
 __global__ void __launch_bounds__(STH) k_gemm_f32(GemmBatch32 bt, int ncol, int ldb, int ldc, int Nrows) {
+  grid_wait();
   __shared__ __align__(16) float As[2][SBK][SBM];  // transposed A tile
   __shared__ __align__(16) float Bs[2][SBK][SBN];
   const GemmItem32& it = bt.item[blockIdx.z];
@@ -375,7 +377,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_xprod32_b(XProdArgs32
 void launch_round_f32(const double2* in, float2* out, long long n, cudaStream_t st) {
   int blocks = (int)((n + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
-  k_round_f32<<<blocks, 256, 0, st>>>(in, out, n);
+  launch_chained(k_round_f32, blocks, 256, 0, st, in, out, n);
 }
 
 void launch_gemm_f32(const GemmBatch32& bt, int nbatch, int ncol, int ldb, int ldc, int Nrows, bool out_f64,
@@ -384,9 +386,9 @@ void launch_gemm_f32(const GemmBatch32& bt, int nbatch, int ncol, int ldb, int l
   for (int b = 0; b < nbatch; ++b) mmax = bt.item[b].M > mmax ? bt.item[b].M : mmax;
   dim3 grid((ncol + SBN - 1) / SBN, (mmax + SBM - 1) / SBM, nbatch);
   if (out_f64)
-    k_gemm_f32<double><<<grid, STH, 0, st>>>(bt, ncol, ldb, ldc, Nrows);
+    launch_chained(k_gemm_f32<double>, grid, STH, 0, st, bt, ncol, ldb, ldc, Nrows);
   else
-    k_gemm_f32<float><<<grid, STH, 0, st>>>(bt, ncol, ldb, ldc, Nrows);
+    launch_chained(k_gemm_f32<float>, grid, STH, 0, st, bt, ncol, ldb, ldc, Nrows);
 }
 
 size_t xprod32_smem_bytes(int M, int nptw) {

@@ -426,6 +426,7 @@ __device__ __forceinline__ void store_unknown(double* Xd, int code, int m, int p
 
 template <int KL, int KU, int P, int PPW>
 __global__ void __launch_bounds__(32 * P / PPW) k_tau_solve(TauArgs a) {
+  grid_wait();
   static_assert(KL + 2 == kFwdWin && KL + KU == kBwdWin, "window sizes follow the band shape");
   constexpr int R = part_rows<P>();  // rows per ring stage
   static_assert(kFwdWin % R == 0 && kBwdWin % R == 0, "whole stages per forward window and per backward block");
@@ -1122,6 +1123,7 @@ __global__ void k_tau_dense(TauArgs a, double* __restrict__ DI, int ld) {
 // by shuffles.  Bound by the latency of two dependent loads and the L2 rate.
 template <int NQ>
 __global__ void __launch_bounds__(256) k_tau_apply(TauArgs a, const double* __restrict__ DI, int ld) {
+  grid_wait();
   const int m = blockIdx.x, c = blockIdx.y, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int n = a.cls[c].n, nb = a.cls[c].nb, n_out = n + NBMAX, Nk = a.Nk;
   const double* M = DI + ((size_t)m * 2 + c) * n_out * ld;
@@ -1476,6 +1478,7 @@ __device__ __forceinline__ double2 stage_sum(const StageTerms& a, int e, int k, 
 // terms are zero outside the DC / Nyquist modes (F, M X and the first right-hand
 // side have none), by the threads of plane 1 there.
 __global__ void __launch_bounds__(128) k_stage_rhs(StageTerms a, double2* __restrict__ out) {
+  grid_wait();
   const int m = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y, e = 1 + blockIdx.z;
   if (m >= a.Nk) return;
   StageLoads L;
@@ -1517,6 +1520,7 @@ __device__ __forceinline__ void s_solve(double2* ys, const double* sk, int K, in
 // the taus zeroed here too.
 __global__ void __launch_bounds__(256, 2) k_stage_final(StageTerms a, double2* __restrict__ Xo, double2* __restrict__ tau,
                                                      int ntau) {
+  grid_wait();
   extern __shared__ double2 ys[];  // as in k_rk_final
   constexpr int MB = kFinalModes, RG = 256 / MB;
   const int f = blockIdx.y >> 1, par = blockIdx.y & 1, Nz = a.Nz, Nk = a.Nk;
@@ -1628,13 +1632,14 @@ template <int KL, int KU>
 void solve_impl(const TauArgs& a, int parts, cudaStream_t st) {
   const int groups = (a.Nk + kSolveModes - 1) / kSolveModes;
   if (parts == kTauParts16)
-    k_tau_solve<KL, KU, kTauParts16, kTau8PerWarp>
-        <<<groups, 32 * kTauParts16 / kTau8PerWarp, solve_smem_bytes<kTauParts16>(a.npad), st>>>(a);
+    launch_chained(k_tau_solve<KL, KU, kTauParts16, kTau8PerWarp>, groups, 32 * kTauParts16 / kTau8PerWarp,
+                   solve_smem_bytes<kTauParts16>(a.npad), st, a);
   else if (parts == kTauParts8)
-    k_tau_solve<KL, KU, kTauParts8, kTau8PerWarp>
-        <<<groups, 32 * kTauParts8 / kTau8PerWarp, solve_smem_bytes<kTauParts8>(a.npad), st>>>(a);
+    launch_chained(k_tau_solve<KL, KU, kTauParts8, kTau8PerWarp>, groups, 32 * kTauParts8 / kTau8PerWarp,
+                   solve_smem_bytes<kTauParts8>(a.npad), st, a);
   else if (parts == kTauParts)
-    k_tau_solve<KL, KU, kTauParts, 1><<<groups, 32 * kTauParts, solve_smem_bytes<kTauParts>(a.npad), st>>>(a);
+    launch_chained(k_tau_solve<KL, KU, kTauParts, 1>, groups, 32 * kTauParts,
+                   solve_smem_bytes<kTauParts>(a.npad), st, a);
   else
     k_tau_solve<KL, KU, 1, 1><<<groups, 32, solve_smem_bytes<1>(a.npad), st>>>(a);
 }
@@ -1720,11 +1725,11 @@ void launch_tau_apply(const TauArgs& a, const double* DI, cudaStream_t st) {
   const int ld = tau_dense_ld(a.cls[0].n);
   const dim3 grid(a.Nk, 2);
   switch ((ld + 31) / 32) {
-    case 1: k_tau_apply<1><<<grid, 256, 0, st>>>(a, DI, ld); break;
-    case 2: k_tau_apply<2><<<grid, 256, 0, st>>>(a, DI, ld); break;
-    case 3: k_tau_apply<3><<<grid, 256, 0, st>>>(a, DI, ld); break;
-    case 4: k_tau_apply<4><<<grid, 256, 0, st>>>(a, DI, ld); break;
-    case 5: k_tau_apply<5><<<grid, 256, 0, st>>>(a, DI, ld); break;
+    case 1: launch_chained(k_tau_apply<1>, grid, 256, 0, st, a, DI, ld); break;
+    case 2: launch_chained(k_tau_apply<2>, grid, 256, 0, st, a, DI, ld); break;
+    case 3: launch_chained(k_tau_apply<3>, grid, 256, 0, st, a, DI, ld); break;
+    case 4: launch_chained(k_tau_apply<4>, grid, 256, 0, st, a, DI, ld); break;
+    case 5: launch_chained(k_tau_apply<5>, grid, 256, 0, st, a, DI, ld); break;
     default: throw Error{TB_EINVAL, "system too large for the dense solve"};
   }
 }
@@ -1778,12 +1783,12 @@ void launch_rk_final(const LinComb& lc, double2* X, double2* tau, const double* 
 }
 
 void launch_stage_rhs(const StageTerms& a, double2* out, cudaStream_t st) {
-  k_stage_rhs<<<dim3((a.Nk + 127) / 128, a.Nz, 3), 128, 0, st>>>(a, out);
+  launch_chained(k_stage_rhs, dim3((a.Nk + 127) / 128, a.Nz, 3), 128, 0, st, a, out);
 }
 
 void launch_stage_final(const StageTerms& a, double2* Xout, double2* tau, int ntau, cudaStream_t st) {
-  k_stage_final<<<dim3((a.Nk + kFinalModes - 1) / kFinalModes, 6), 256, rk_final_smem_bytes(a.Nz), st>>>(a, Xout, tau,
-                                                                                                        ntau);
+  launch_chained(k_stage_final, dim3((a.Nk + kFinalModes - 1) / kFinalModes, 6), 256, rk_final_smem_bytes(a.Nz), st, a, Xout,
+                 tau, ntau);
 }
 
 size_t rk_final_smem_bytes(int Nz) {

@@ -831,6 +831,7 @@ __global__ void __launch_bounds__(kTcThreads) k_tc32p_image(const float* __restr
 template <bool BWD>
 __global__ void __launch_bounds__(kPThreads, 1) k_tc32p(const float* __restrict__ in, const float* __restrict__ images,
                                                         void* out, int nfields, int N, int ncol) {
+  grid_wait(in);
   extern __shared__ uint8_t tc_smem_raw[];
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(tc_smem_raw);
   const uint32_t pad = (1024u - (raw & 1023u)) & 1023u;
@@ -1248,9 +1249,9 @@ void launch_tc32p(bool backward, const float* in, const float* images, void* out
   const int ntask = nfields * ((ncol + kPN - 1) / kPN);
   const int grid = sms < Q * ntask ? sms : Q * ntask;
   if (backward)
-    k_tc32p<true><<<grid, kPThreads, kPSmem, st>>>(in, images, out, nfields, N, ncol);
+    launch_chained(k_tc32p<true>, grid, kPThreads, kPSmem, st, in, images, out, nfields, N, ncol);
   else
-    k_tc32p<false><<<grid, kPThreads, kPSmem, st>>>(in, images, out, nfields, N, ncol);
+    launch_chained(k_tc32p<false>, grid, kPThreads, kPSmem, st, in, images, out, nfields, N, ncol);
 }
 
 int tc32_status() {

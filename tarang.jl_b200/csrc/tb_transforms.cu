@@ -57,6 +57,7 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 //                 16-deep slice; the two k halves are summed through shared memory.
 template <bool SPLITK>
 __global__ void __launch_bounds__(GTH) k_gemm_f64(GemmBatch bt, int ncol, int ldb, int ldc, int Nrows) {
+  grid_wait();
   constexpr int TM = SPLITK ? GBM / 2 : GBM;  // CTA tile rows
   extern __shared__ __align__(16) double gsm[];
   double (*As)[GBM * ASTR] = reinterpret_cast<double (*)[GBM * ASTR]>(gsm);
@@ -205,10 +206,10 @@ void launch_gemm_f64(const GemmBatch& bt, int nbatch, int ncol, int ldb, int ldc
   if (ctas < 2LL * 148) {
     // too few 64-row tiles to fill the SMs: halve the tile rows and split K inside the CTA
     dim3 grid(ncx, (mmax + GBM / 2 - 1) / (GBM / 2), nbatch);
-    k_gemm_f64<true><<<grid, GTH, kGemmSmem, st>>>(bt, ncol, ldb, ldc, Nrows);
+    launch_chained(k_gemm_f64<true>, grid, GTH, kGemmSmem, st, bt, ncol, ldb, ldc, Nrows);
   } else {
     dim3 grid(ncx, (mmax + GBM - 1) / GBM, nbatch);
-    k_gemm_f64<false><<<grid, GTH, kGemmSmem, st>>>(bt, ncol, ldb, ldc, Nrows);
+    launch_chained(k_gemm_f64<false>, grid, GTH, kGemmSmem, st, bt, ncol, ldb, ldc, Nrows);
   }
 }
 
@@ -792,6 +793,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_xprod_b(XProdArgs a) 
 // transforms are half the work.  An odd last row goes with zeros.
 __global__ void __launch_bounds__(256) k_x_rfft(const double* __restrict__ grid, double2* __restrict__ spec, int nrows,
                                                 int Nx, FftPlan fp, const double2* __restrict__ tw) {
+  grid_wait(grid);
   extern __shared__ double2 sm[];
   double2* A = sm;
   double2* B = sm + Nx;
@@ -849,6 +851,7 @@ __global__ void __launch_bounds__(256) k_x_irfft(const double2* __restrict__ spe
 // so one read of a half row and one FFT give both.  Grid (ceil(Nz/2), fields).
 __global__ void __launch_bounds__(256) k_x_irfft_half(const double2* __restrict__ half, double* __restrict__ grid, int Nz,
                                                       int Nx, FftPlan fp, const double2* __restrict__ tw) {
+  grid_wait(half);
   extern __shared__ double2 sm[];
   double2* A = sm;
   double2* B = sm + Nx;
@@ -992,7 +995,7 @@ void launch_xprod_b(const XProdArgs& a, cudaStream_t st) {
 void launch_x_rfft(const double* grid, double2* spec, int nrows, int Nx, const FftPlan& fp, const double2* tw,
                    cudaStream_t st) {
   size_t smem = 2 * (size_t)Nx * sizeof(double2);
-  k_x_rfft<<<(nrows + 1) / 2, 256, smem, st>>>(grid, spec, nrows, Nx, fp, tw);
+  launch_chained(k_x_rfft, (nrows + 1) / 2, 256, smem, st, grid, spec, nrows, Nx, fp, tw);
 }
 
 void launch_x_irfft(const double2* spec, double* grid, int nrows, int Nx, const FftPlan& fp, const double2* tw,
@@ -1004,7 +1007,7 @@ void launch_x_irfft(const double2* spec, double* grid, int nrows, int Nx, const 
 void launch_x_irfft_half(const double2* half, double* grid, int nfields, int Nz, int Nx, const FftPlan& fp,
                          const double2* tw, cudaStream_t st) {
   size_t smem = 2 * (size_t)Nx * sizeof(double2);
-  k_x_irfft_half<<<dim3((Nz + 1) / 2, nfields), 256, smem, st>>>(half, grid, Nz, Nx, fp, tw);
+  launch_chained(k_x_irfft_half, dim3((Nz + 1) / 2, nfields), 256, smem, st, half, grid, Nz, Nx, fp, tw);
 }
 
 void launch_x_dealias_mul(const double* a, const double* b, double* out, int nrows, int Nx, int M,

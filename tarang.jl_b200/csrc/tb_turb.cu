@@ -141,8 +141,8 @@ __host__ __device__ inline int ystride(int My) { return Rp::rpad<float2>(My) + 4
 // FFT along y; out: mix[f][y][kx].  The columns of a group share the passes'
 // barriers and their rows are stored together (32 bytes at CW = 4), which
 // replaces a separate transpose: bound by shared-memory traffic.
-template <int CW>
-__global__ void __launch_bounds__(kTurbThreads, 3) k_turb_yinv(TurbArgs a, const float2* __restrict__ q,
+template <int CW, int BL>
+__global__ void __launch_bounds__(kTurbThreads, BL) k_turb_yinv(TurbArgs a, const float2* __restrict__ q,
                                                                float2* __restrict__ mix) {
   extern __shared__ __align__(16) float2 sm[];
   const int My = a.My, Ny = a.Ny, kx0 = blockIdx.x * CW, f = blockIdx.y;
@@ -228,7 +228,8 @@ __device__ __forceinline__ void xmiddle(float2* __restrict__ A, int Ms, int n) {
   }
 }
 
-__global__ void __launch_bounds__(kTurbThreads, 3) k_turb_xpass(TurbArgs a, const float2* __restrict__ mix,
+template <int BL>
+__global__ void __launch_bounds__(kTurbThreads, BL) k_turb_xpass(TurbArgs a, const float2* __restrict__ mix,
                                                                 float2* __restrict__ pm) {
   extern __shared__ __align__(16) float2 sm[];
   const int Mx = a.Mx, hN = a.Nx / 2, y0 = 2 * blockIdx.x;
@@ -393,6 +394,17 @@ int columns_per_block(int Kx, int factors) {
   return 1;
 }
 
+// Whether a kernel runs its build for four blocks of kTurbThreads an SM (64
+// registers, 28 to 72 bytes of spills) instead of three (78): where the grid is
+// more than three blocks an SM can hold at once and shared memory has room for
+// four. At 1024x1024 the 516 blocks of the inverse y transforms are then one
+// wave and not one and a sixth (10 RK443 steps 4452 -> 4115 us; the forward kernel,
+// whose blocks all fit at once, has the one build); at 256x256, where a wave
+// holds every block, the spills cost 4 %.
+bool four_blocks(int blocks, int threads, size_t smem) {
+  return (long long)blocks * threads > 3LL * 148 * kTurbThreads && 4 * (smem + 1024) <= 228 * 1024;
+}
+
 TurbArgs args_of(const tb_turb* T) {
   TurbArgs a{};
   a.Nx = T->Nx;
@@ -421,10 +433,15 @@ void enqueue_rhs(tb_turb* T, const float2* q, float2* qo, float2* Fp, double dt,
   // about one butterfly of radix 8 a thread
   auto threads = [](int arrays, int n) { return arrays * n <= 1024 ? kTurbThreads / 2 : kTurbThreads; };
   const int ci = columns_per_block(T->Kx, 4), cf = columns_per_block(T->Kx, 1);
-  auto yinv = ci == 4 ? k_turb_yinv<4> : ci == 2 ? k_turb_yinv<2> : k_turb_yinv<1>;
+  const int bi = (T->Kx + ci - 1) / ci * 4, bx = T->My / 2, ti = threads(ci, T->My), tx = threads(4, T->Mx);
+  const bool i4 = four_blocks(bi, ti, y_smem(T, ci)), x4 = four_blocks(bx, tx, x_smem(T));
+  auto yinv = ci == 4   ? (i4 ? k_turb_yinv<4, 4> : k_turb_yinv<4, 3>)
+              : ci == 2 ? (i4 ? k_turb_yinv<2, 4> : k_turb_yinv<2, 3>)
+                        : (i4 ? k_turb_yinv<1, 4> : k_turb_yinv<1, 3>);
+  auto xpass = x4 ? k_turb_xpass<4> : k_turb_xpass<3>;
   auto yfwd = cf == 4 ? k_turb_yfwd<4> : cf == 2 ? k_turb_yfwd<2> : k_turb_yfwd<1>;
-  yinv<<<dim3((T->Kx + ci - 1) / ci, 4), threads(ci, T->My), y_smem(T, ci), T->st>>>(a, q, mix);
-  k_turb_xpass<<<T->My / 2, threads(4, T->Mx), x_smem(T), T->st>>>(a, mix, pm);
+  yinv<<<dim3(bi / 4, 4), ti, y_smem(T, ci), T->st>>>(a, q, mix);
+  xpass<<<bx, tx, x_smem(T), T->st>>>(a, mix, pm);
   yfwd<<<(T->Kx + cf - 1) / cf, threads(cf, T->My), y_smem(T, cf), T->st>>>(a, pm, q, qo, Fp, (float)dt, mode, c,
                                                                             (float)wF);
 }
@@ -584,9 +601,10 @@ tb_turb* tb::turb_create(tb_context* ctx, const tb_problem_desc& d, const double
   upload(T->posy, rplan_positions(T->ry));
   TB_REQUIRE(x_smem(T.get()) <= 227 * 1024 && y_smem(T.get(), 4) <= 227 * 1024, TB_ENOTSUPPORTED,
              "turbulence grid too large for the shared-memory transforms");
-  for (const void* k : {(const void*)k_turb_yinv<1>, (const void*)k_turb_yinv<2>, (const void*)k_turb_yinv<4>,
-                        (const void*)k_turb_xpass, (const void*)k_turb_yfwd<1>, (const void*)k_turb_yfwd<2>,
-                        (const void*)k_turb_yfwd<4>})
+  for (const void* k : {(const void*)k_turb_yinv<1, 3>, (const void*)k_turb_yinv<2, 3>, (const void*)k_turb_yinv<4, 3>,
+                        (const void*)k_turb_yinv<1, 4>, (const void*)k_turb_yinv<2, 4>, (const void*)k_turb_yinv<4, 4>,
+                        (const void*)k_turb_xpass<3>, (const void*)k_turb_xpass<4>, (const void*)k_turb_yfwd<1>,
+                        (const void*)k_turb_yfwd<2>, (const void*)k_turb_yfwd<4>})
     TB_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
   turb_set(T.get(), q0);
   return T.release();

@@ -10,9 +10,10 @@ from oracle.tarang_oracle import (RBC3D, TABLEAUS, RBC3Params, rbc3_initial_b, r
 pytestmark = pytest.mark.gpu
 
 
-# kx columns 5 .. 1025 against 1, 2 and 4 a block; padded lengths 12 .. 3072
+# kx columns 5 .. 1025 against 1, 2 and 4 a block; padded lengths 12 .. 3072; the
+# last two exceed three blocks an SM in the y and in the x transforms
 @pytest.mark.parametrize("Nx,Ny", [(8, 8), (8, 64), (12, 16), (108, 72), (256, 48), (512, 32), (1024, 16), (2048, 8),
-                                   (16, 2048), (972, 12)])
+                                   (16, 2048), (972, 12), (2048, 256), (512, 1152)])
 @pytest.mark.parametrize("scheme", ["SBDF2", "RK222", "RK443"])
 def test_turbulence_sizes_match_oracle(tb, scheme, Nx, Ny):
     ts = {"RK222": tb._lib.TB_RK222, "RK443": tb._lib.TB_RK443, "SBDF2": tb._lib.TB_SBDF2}[scheme]

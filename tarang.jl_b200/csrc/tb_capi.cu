@@ -1962,7 +1962,7 @@ void planes_of_grids_2d(tb_plan* P, const double* grid, double2* coeff, int nfie
   double2* spec = P->G.as<double2>();  // 12 half planes: room for six planes
   for (int f0 = 0; f0 < nfields; f0 += kFieldsPerLaunch) {
     const int nf = std::min(kFieldsPerLaunch, nfields - f0);
-    launch_x_rfft(grid + f0 * g, spec, nf * P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st);
+    launch_x_rfft(grid + f0 * g, spec, P->Nz, P->Nx, P->fpN, P->twN.as<double2>(), P->st, nf);
     GemmBatch bt{};
     int nb = 0;
     for (int f = 0; f < nf; ++f) {

@@ -152,7 +152,7 @@ cudaError_t set_transform_smem_limits(int bytes);
 // Standalone x transforms on rows: forward rfft (grid rows -> half spectra) and
 // backward irfft (half spectra -> grid rows), unnormalised / 1/N like FFTW.
 void launch_x_rfft(const double* grid, double2* spec, int nrows, int Nx, const FftPlan& fp, const double2* tw,
-                   cudaStream_t st);
+                   cudaStream_t st, int nfields = 1);  // nfields fields of nrows rows, back to back
 void launch_x_irfft(const double2* spec, double* grid, int nrows, int Nx, const FftPlan& fp, const double2* tw,
                     cudaStream_t st);
 // Grid fields (Nz x Nx each, back to back) from their even / odd Chebyshev half

@@ -790,7 +790,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_xprod_b(XProdArgs a) 
 // rfft of real rows (unnormalised), two rows to a complex FFT: rows 2 i and 2 i + 1
 // as real and imaginary part, the spectra separated by conjugate symmetry.  The
 // kernel is bound by the passes' shared-memory round trips, so half the
-// transforms are half the work.  An odd last row goes with zeros.
+// transforms are half the work.  Pairs stay inside a field (blockIdx.y, nrows
+// rows each), whose rows the other transforms mix anyway: one field's size and
+// infinities do not reach another's coefficients.  An odd last row goes with
+// zeros.
 __global__ void __launch_bounds__(256) k_x_rfft(const double* __restrict__ grid, double2* __restrict__ spec, int nrows,
                                                 int Nx, FftPlan fp, const double2* __restrict__ tw) {
   grid_wait(grid);
@@ -800,11 +803,12 @@ __global__ void __launch_bounds__(256) k_x_rfft(const double* __restrict__ grid,
   const int row = 2 * blockIdx.x;
   const bool two = row + 1 < nrows;
   const int Nk = Nx / 2 + 1;
-  const double* g = grid + (size_t)row * Nx;
+  const size_t first = (size_t)blockIdx.y * nrows + row;
+  const double* g = grid + first * Nx;
   for (int p = threadIdx.x; p < Nx; p += blockDim.x) A[p] = make_double2(g[p], two ? g[Nx + p] : 0.0);
   __syncthreads();
   const double2* R = fft_cta(A, B, fp, tw, -1);
-  double2* out = spec + (size_t)row * Nk;
+  double2* out = spec + first * Nk;
   for (int k = threadIdx.x; k < Nk; k += blockDim.x) {
     const double2 c = R[k], w = R[k ? Nx - k : 0];
     const bool edge = k == 0 || 2 * k == Nx;
@@ -993,9 +997,9 @@ void launch_xprod_b(const XProdArgs& a, cudaStream_t st) {
 }
 
 void launch_x_rfft(const double* grid, double2* spec, int nrows, int Nx, const FftPlan& fp, const double2* tw,
-                   cudaStream_t st) {
+                   cudaStream_t st, int nfields) {
   size_t smem = 2 * (size_t)Nx * sizeof(double2);
-  launch_chained(k_x_rfft, (nrows + 1) / 2, 256, smem, st, grid, spec, nrows, Nx, fp, tw);
+  launch_chained(k_x_rfft, dim3((nrows + 1) / 2, nfields), 256, smem, st, grid, spec, nrows, Nx, fp, tw);
 }
 
 void launch_x_irfft(const double2* spec, double* grid, int nrows, int Nx, const FftPlan& fp, const double2* tw,

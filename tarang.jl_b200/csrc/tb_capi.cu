@@ -270,9 +270,13 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
     fit(fs->FR, groups * n * 2 * kFwdRec * kSolveModes * sizeof(double));
     fit(fs->BR, groups * n * 2 * tau_bwd_rec(S.tau_parts) * kSolveModes * sizeof(double));
     fit(fs->SI, groups * 2 * 16 * kSolveModes * sizeof(double));
-    TB_CUDA_TRY(cudaMemsetAsync(fs->FR.p, 0, fs->FR.bytes, P->st));
-    TB_CUDA_TRY(cudaMemsetAsync(fs->BR.p, 0, fs->BR.bytes, P->st));
-    TB_CUDA_TRY(cudaMemsetAsync(fs->SI.p, 0, fs->SI.bytes, P->st));
+    // (the factorisation writes every record of a mode; the solves also read the
+    // last group's spare modes)
+    if (Nk % kSolveModes)
+      for (DevBuf* b : {&fs->FR, &fs->BR, &fs->SI}) {
+        const size_t g = b->bytes / groups;
+        TB_CUDA_TRY(cudaMemsetAsync(static_cast<char*>(b->p) + (groups - 1) * g, 0, g, P->st));
+      }
   }
   fit(fs->PP, banded ? tau_transfer_doubles(Nk, S.tau_parts) * sizeof(double) : 0);
   fit(fs->HR, banded ? tau_response_doubles(Nk, (int)n, S.tau_parts) * sizeof(double) : 0);

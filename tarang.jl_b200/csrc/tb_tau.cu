@@ -74,8 +74,11 @@ __device__ __forceinline__ double* bwd_record(double* BR, int npad, int brec, in
 // columns: lane t < KL+KU updates column j+1+t of the KL rows below and of
 // the boundary rows, lanes KL+KU.. the border entries.  Every element gets the
 // same operations in the same order as a sequential elimination, so the
-// factors do not depend on the lane split; the pivot scan (KL+1 candidates)
-// and the Schur inverse run on lane 0.
+// factors do not depend on the lane split; the Schur inverse runs on lane 0.
+// Bound by the latency of a step's chain (a warp an SM sub-partition): the
+// coefficients of the row and column that enter are read a step ahead, the ring
+// slots advance instead of being divided for, and a record leaves in one store
+// (1024x256 1240 -> 737 us, 1536x384 1905 -> 1181).
 // ---------------------------------------------------------------------------
 constexpr int kFactorWarps = 4;  // systems (warps) per CTA of the factorisation
 
@@ -92,7 +95,7 @@ __host__ __device__ constexpr size_t factor_smem_bytes() {
 
 template <int KL, int KU>
 __global__ void __launch_bounds__(32 * kFactorWarps) k_tau_factor(TauArgs a) {
-  static_assert(KL + KU + NBMAX <= 32 && kFwdRec <= 32 && kBwdCode < 32, "one lane per column and record slot");
+  static_assert(KL + KU + NBMAX <= 32 && kFwdRec <= 32 && kBwdRec <= 32, "one lane per column and record slot");
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int ml = blockIdx.x * kFactorWarps + warp;  // mode within this instance
   const int c = blockIdx.y;
@@ -112,136 +115,152 @@ __global__ void __launch_bounds__(32 * kFactorWarps) k_tau_factor(TauArgs a) {
   auto Cr = [&](int q, int col) -> double& { return win[RR * (WW + NBMAX) + q * CW + col % CW]; };
   auto C1 = [&](int q, int b) -> double& { return win[RR * (WW + NBMAX) + NBMAX * CW + q * NBMAX + b]; };
   const int cw = C.kl + C.ku + 1;
-  // row r enters: lane s < WW fills band slot s, lanes < nb the border
-  auto init_row = [&](int r) {
-    if (lane < WW) {
-      double v = 0.0;
-      const int d = lane + C.kl - KL;  // band-table entry of slot lane
-      const int col = r + lane - KL;
-      if (d >= 0 && d < cw && col >= 0 && col < n) v = coef_val(C.band[(size_t)r * cw + d], a.alpha, a.beta, kx);
-      Wr(r, lane) = v;
-    }
-    if (lane < nb) Bd(r, lane) = coef_val(C.bord[(size_t)r * nb + lane], a.alpha, a.beta, kx);
+  // row r enters: lane s < WW fills band slot s, lanes < nb the border; its
+  // coefficients (fetch) are read a step before the window takes them (put)
+  Coef rowc{}, bordc{};
+  double wallc = 0.0;
+  auto fetch_row = [&](int r) {
+    const int d = lane + C.kl - KL;  // band-table entry of slot lane
+    const int col = r + lane - KL;
+    rowc = Coef{};
+    if (lane < WW && d >= 0 && d < cw && col >= 0 && col < n) rowc = C.band[(size_t)r * cw + d];
+    if (lane < nb) bordc = C.bord[(size_t)r * nb + lane];
   };
-  auto init_col = [&](int col) {
-    if (lane < nb) Cr(lane, col) = a.beta * (zmode ? C.c2_z : C.c2_nz)[(size_t)lane * n + col];
+  auto put_row = [&](int r) {
+    if (lane < WW) Wr(r, lane) = coef_val(rowc, a.alpha, a.beta, kx);
+    if (lane < nb) Bd(r, lane) = coef_val(bordc, a.alpha, a.beta, kx);
   };
-  for (int r = 0; r <= KL && r < n; ++r) init_row(r);
-  for (int col = 0; col < CW && col < n; ++col) init_col(col);
+  auto fetch_col = [&](int col) {
+    if (lane < nb) wallc = (zmode ? C.c2_z : C.c2_nz)[(size_t)lane * n + col];
+  };
+  auto put_col = [&](int col) {
+    if (lane < nb) Cr(lane, col) = a.beta * wallc;
+  };
+  for (int r = 0; r <= KL && r < n; ++r) {
+    fetch_row(r);
+    put_row(r);
+  }
+  for (int col = 0; col < CW && col < n; ++col) {
+    fetch_col(col);
+    put_col(col);
+  }
+  if (KL + 1 < n) fetch_row(KL + 1);
+  if (CW < n) fetch_col(CW);
   if (lane < nb * nb) {
     const int q = lane / nb, b = lane % nb;
     C1(q, b) = a.beta * (zmode ? C.c1_z : C.c1_nz)[q * nb + b];
   }
   __syncwarp();
+  // rows j + t in slot ro[t], column j in slot cj (rows at i % RR, columns at c % CW)
+  int ro[KL + 1], cj = 0;
+#pragma unroll
+  for (int t = 0; t <= KL; ++t) ro[t] = t;
+  double* const bord = win + RR * WW;
+  double* const walls = bord + RR * NBMAX;
+  // store target (element offset of its row * 2 + the i flag) of band column j,
+  // and whether the row entering the forward window there is a u_x momentum
+  // row, scaled by -i on load
+  auto column_code = [&](int j) { return j < n ? (long long)C.col_code[j] : 0LL; };
+  auto rotation = [&](int j) { return j + kFwdWin < n && C.row_eq[j + kFwdWin] == EQ_MX ? 1LL : 0LL; };
+  long long tail = lane == kBwdCode ? column_code(0) : lane == kFwdRot ? rotation(0) : 0LL;
   for (int j = 0; j < n; ++j) {
     // rows / columns entering the window at this step (their slots held row /
     // column j-1, finished at the previous step)
-    if (j >= 1 && j + KL < n) init_row(j + KL);
-    if (j >= 1 && j + CW - 1 < n) init_col(j + CW - 1);
+    const long long tail_j = tail;
+    if (j >= 1) {
+      if (j + KL < n) put_row(j + KL);
+      if (j + CW - 1 < n) put_col(j + CW - 1);
+      if (j + KL + 1 < n) fetch_row(j + KL + 1);
+      if (j + CW < n) fetch_col(j + CW);
+    }
+    if (lane == kBwdCode) tail = column_code(j + 1);
+    if (lane == kFwdRot) tail = rotation(j + 1);
     __syncwarp();
     const int ilast = min(j + KL, n - 1);
     const int clast = min(j + KL + KU, n - 1);
-    // pivot: the first largest |entry| of column j among rows j..ilast
-    int p = j;
-    bool bad = false;
-    if (lane == 0) {
-      double best = fabs(Wr(j, KL));
-      for (int i = j + 1; i <= ilast; ++i) {
-        double v = fabs(Wr(i, j - i + KL));
-        if (v > best) {
-          best = v;
-          p = i;
-        }
+    // pivot: the first largest |entry| of column j among rows j..ilast (every
+    // lane scans the same entries)
+    int p = 0, po = ro[0];
+    double best = fabs(win[ro[0] * WW + KL]);
+#pragma unroll
+    for (int t = 1; t <= KL; ++t) {
+      const double v = j + t <= ilast ? fabs(win[ro[t] * WW + KL - t]) : 0.0;
+      if (v > best) {
+        best = v;
+        p = t;
+        po = ro[t];
       }
-      bad = !(best > 0.0) || !isfinite(best);
     }
-    p = __shfl_sync(0xffffffffu, p, 0);
-    if (__shfl_sync(0xffffffffu, (int)bad, 0)) {
+    if (!(best > 0.0) || !isfinite(best)) {
       if (lane == 0) atomicMin(a.err_mode, m);
       return;
     }
-    if (p != j) {
-      const int cc = j + lane;
-      if (cc <= clast) {
-        double t = Wr(j, cc - j + KL);
-        Wr(j, cc - j + KL) = Wr(p, cc - p + KL);
-        Wr(p, cc - p + KL) = t;
+    if (p != 0) {
+      __syncwarp();  // the column is read
+      if (j + lane <= clast) {
+        double* const wj = win + ro[0] * WW + KL + lane;
+        double* const wp = win + po * WW + KL + lane - p;
+        const double t = *wj;
+        *wj = *wp;
+        *wp = t;
       }
       if (lane < nb) {
-        double t = Bd(j, lane);
-        Bd(j, lane) = Bd(p, lane);
-        Bd(p, lane) = t;
+        const double t = bord[ro[0] * NBMAX + lane];
+        bord[ro[0] * NBMAX + lane] = bord[po * NBMAX + lane];
+        bord[po * NBMAX + lane] = t;
       }
       __syncwarp();
     }
-    const double dinv = 1.0 / Wr(j, KL);
-    // multipliers of the rows below and of the boundary rows, read by every
-    // lane before lane 0 clears their column-j entries
+    const double dinv = 1.0 / win[ro[0] * WW + KL];
+    // multipliers of the rows below and of the boundary rows (the entries of
+    // column j stay in the window, where nothing reads them again)
     double l[KL], cqv[NBMAX];
 #pragma unroll
-    for (int t = 0; t < KL; ++t) {
-      const int i = j + 1 + t;
-      l[t] = (i <= ilast) ? Wr(i, j - i + KL) * dinv : 0.0;
-    }
+    for (int t = 0; t < KL; ++t) l[t] = (j + 1 + t <= ilast) ? win[ro[t + 1] * WW + KL - 1 - t] * dinv : 0.0;
 #pragma unroll
-    for (int q = 0; q < NBMAX; ++q) cqv[q] = (q < nb) ? Cr(q, j) * dinv : 0.0;
-    __syncwarp();
-    if (lane == 0) {
-      for (int t = 0; t < KL; ++t)
-        if (j + 1 + t <= ilast) Wr(j + 1 + t, j - (j + 1 + t) + KL) = 0.0;
-      for (int q = 0; q < nb; ++q) Cr(q, j) = 0.0;
-    }
+    for (int q = 0; q < NBMAX; ++q) cqv[q] = (q < nb) ? walls[q * CW + cj] * dinv : 0.0;
     if (lane < KL + KU) {
-      const int cc = j + 1 + lane;
-      if (cc <= clast) {
-        const double wj = Wr(j, cc - j + KL);
+      if (j + 1 + lane <= clast) {
+        const double wj = win[ro[0] * WW + KL + 1 + lane];
+        const int cc = cj + 1 + lane >= CW ? cj + 1 + lane - CW : cj + 1 + lane;
 #pragma unroll
-        for (int t = 0; t < KL; ++t) {
-          const int i = j + 1 + t;
-          if (i <= ilast) Wr(i, cc - i + KL) -= l[t] * wj;
-        }
+        for (int t = 0; t < KL; ++t)
+          if (j + 1 + t <= ilast) win[ro[t + 1] * WW + KL + lane - t] -= l[t] * wj;
 #pragma unroll
         for (int q = 0; q < NBMAX; ++q)
-          if (q < nb) Cr(q, cc) -= cqv[q] * wj;
+          if (q < nb) walls[q * CW + cc] -= cqv[q] * wj;
       }
     } else if (lane - (KL + KU) < nb) {
       const int b = lane - (KL + KU);
-      const double bj = Bd(j, b);
+      const double bj = bord[ro[0] * NBMAX + b];
 #pragma unroll
-      for (int t = 0; t < KL; ++t) {
-        const int i = j + 1 + t;
-        if (i <= ilast) Bd(i, b) -= l[t] * bj;
-      }
+      for (int t = 0; t < KL; ++t)
+        if (j + 1 + t <= ilast) bord[ro[t + 1] * NBMAX + b] -= l[t] * bj;
 #pragma unroll
       for (int q = 0; q < NBMAX; ++q)
         if (q < nb) C1(q, b) -= cqv[q] * bj;
     }
-    // records of row j (row j itself is final after the swap)
-    double* fr = fwd_record(C.FR, a.npad, m, j, c);
-    double* br = bwd_record(C.BR, a.npad, a.brec, m, j, c);
-    if (lane == 0) {
-      fr[0] = __longlong_as_double((long long)(p - j));  // pivot offset, integer bits
-    } else if (lane <= KL) {
-      fr[lane] = l[lane - 1];
-    } else if (lane <= KL + NBMAX) {
-      fr[lane] = cqv[lane - 1 - KL];  // 0 past nb
-    } else if (lane == kFwdRot) {
-      // 1 when the right-hand side of row j + kFwdWin (the row entering the
-      // forward window at this row) is a u_x momentum row, scaled by -i on load
-      const int jn = j + kFwdWin;
-      fr[kFwdRot] = __longlong_as_double((jn < n && C.row_eq[jn] == EQ_MX) ? 1LL : 0LL);
-    }
-    if (lane == 0) {
-      br[0] = dinv;
-    } else if (lane < W1) {
-      br[lane] = (j + lane < n) ? Wr(j, KL + lane) : 0.0;
+    // records of row j (row j itself is final after the swap), a value a lane
+    double fv = __longlong_as_double(lane == 0 ? (long long)p : tail_j);  // pivot offset; rotation flag
+#pragma unroll
+    for (int t = 0; t < KL; ++t) fv = lane == 1 + t ? l[t] : fv;
+#pragma unroll
+    for (int q = 0; q < NBMAX; ++q) fv = lane == 1 + KL + q ? cqv[q] : fv;  // 0 past nb
+    if (lane < kFwdRec) fwd_record(C.FR, a.npad, m, j, c)[lane] = fv;
+    double bv = 0.0;  // (slots from kBwdG on: the first partition's responses; k_tau_transfer writes the others')
+    if (lane < W1) {
+      if (j + lane < n) bv = win[ro[0] * WW + KL + lane];
     } else if (lane < W1 + NBMAX) {
-      const int b = lane - W1;
-      br[lane] = (b < nb) ? Bd(j, b) : 0.0;
-    } else if (lane == kBwdCode) {
-      // store target of this band column (element offset of its row * 2 + the i flag), bit-cast
-      br[kBwdCode] = __longlong_as_double((long long)C.col_code[j]);
+      if (lane - W1 < nb) bv = bord[ro[0] * NBMAX + lane - W1];
     }
+    if (lane == 0) bv = dinv;
+    if (lane == kBwdCode) bv = __longlong_as_double(tail_j);
+    if (lane < a.brec) bwd_record(C.BR, a.npad, a.brec, m, j, c)[lane] = bv;
+    const int r0 = ro[0];
+#pragma unroll
+    for (int t = 0; t < KL; ++t) ro[t] = ro[t + 1];
+    ro[KL] = r0;
+    cj = cj + 1 == CW ? 0 : cj + 1;
     __syncwarp();  // row j's slot is refilled at the next step
   }
   // padding rows n..npad-1: identity rows with no right-hand side and no store
@@ -250,7 +269,7 @@ __global__ void __launch_bounds__(32 * kFactorWarps) k_tau_factor(TauArgs a) {
     double* br = bwd_record(C.BR, a.npad, a.brec, m, j, c);
     for (int t = 0; t < kFwdRec; ++t) fr[t] = 0.0;
     br[0] = 1.0;
-    for (int t = 1; t < kBwdCode; ++t) br[t] = 0.0;
+    for (int t = 1; t < a.brec; ++t) br[t] = 0.0;
     br[kBwdCode] = __longlong_as_double(-1LL);
   }
   if (lane != 0) return;
@@ -978,57 +997,88 @@ __global__ void __launch_bounds__(32 * P / PPW) k_tau_solve(TauArgs a) {
 // y and border unknowns):
 //   H of row j (H record) = x_j,  Psi_k[o][i] = x of row r0 + o (stored
 //   transposed, [i][o], so the carry reads it by input).
+//
+// A block takes one partition of one mode group: warp 0 the four forward units,
+// warps 1..3 four backward units each, lane = (class, mode, unit), so that a
+// warp's loads of a row are one contiguous run of records.  The windows are
+// unrolled and stay in registers.  Bound by memory: at 1536x384 (16
+// partitions) 0.45 GB of records read and responses written; with a thread's
+// windows indexed at run time (local memory) and one mode's record per lane it
+// took 780 us, now 156; at 1024x256 (8 partitions) 350, now 72.
 // ---------------------------------------------------------------------------
 template <int KL, int KU, int P, int PPW>
 __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
-  // one thread per (mode, class, partition, unit): forward unit i < 4,
-  // backward unit i - 4 < 12
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y & 1, k = blockIdx.y >> 1;
-  const int i = blockIdx.z;
-  if (m >= a.Nk) return;
-  const int np = a.npad;
-  const int g = m / kSolveModes, mm = m % kSolveModes;
-  // Phi, Gz, Psi exist only for P > 1 (a.PP is null otherwise)
-  double* tr = P > 1 ? a.PP + ((((size_t)g * P + k) * 2 + c) * kSolveModes + mm) * kTransfer : nullptr;
+  static_assert(P > 1 && KL == 4 && kBwdWin == 12 && kSolveModes == 4, "warp 0 forward, three backward; 32 lanes");
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int i = lane % 4, mm = lane / 4 % 4, c = lane / 16;
+  const int g = blockIdx.x, k = blockIdx.y, np = a.npad;
   const int r0 = tau_part_row0(np, P, k, PPW), r1 = tau_part_row0(np, P, k + 1, PPW);
-  if (i < 4) {
+  double* tr = a.PP + ((((size_t)g * P + k) * 2 + c) * kSolveModes + mm) * kTransfer;
+  double* BR = bwd_record(a.cls[0].BR, np, kBwdRec, g * kSolveModes + mm, 0, c);
+  constexpr size_t FROW = 2 * kSolveModes * kFwdRec, BROW = 2 * kSolveModes * kBwdRec;
+  if (warp == 0) {
     if (k < 1) return;
+    const double* FR = fwd_record(a.cls[0].FR, np, g * kSolveModes + mm, 0, c);
     double y[kFwdWin], z[NBMAX] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
     for (int t = 0; t < kFwdWin; ++t) y[t] = (t == i) ? 1.0 : 0.0;
-    for (int j = r0; j < r1; ++j) {
-      const double* fr = fwd_record(a.cls[0].FR, np, m, j, c);
-      const int u = (j - r0) % kFwdWin;
-      const int p = __double2loint(fr[0]);
-      double yj = y[u];
-      for (int t = 1; t <= KL; ++t) {
-        if (t == p) {
-          const double yt = y[(u + t) % kFwdWin];
-          y[(u + t) % kFwdWin] = yj;
-          yj = yt;
+    for (int j0 = r0; j0 < r1; j0 += kFwdWin) {
+#pragma unroll
+      for (int u = 0; u < kFwdWin; ++u) {
+        double fr[kFwdRec];
+#pragma unroll
+        for (int v = 0; v < kFwdRec / 2; ++v) {
+          const double2 d = __ldg(reinterpret_cast<const double2*>(FR + (size_t)(j0 + u) * FROW) + v);
+          fr[2 * v] = d.x;
+          fr[2 * v + 1] = d.y;
         }
+        const int p = __double2loint(fr[0]);
+        double yj = y[u];
+#pragma unroll
+        for (int t = 1; t <= KL; ++t) {
+          const bool sw = (t == p);
+          const double yt = y[(u + t) % kFwdWin];
+          y[(u + t) % kFwdWin] = sw ? yj : yt;
+          yj = sw ? yt : yj;
+        }
+        BR[(size_t)(j0 + u) * BROW + kBwdG + i] = yj;
+#pragma unroll
+        for (int t = 1; t <= KL; ++t) y[(u + t) % kFwdWin] = fma(-fr[t], yj, y[(u + t) % kFwdWin]);
+#pragma unroll
+        for (int b = 0; b < NBMAX; ++b) z[b] = fma(-fr[1 + KL + b], yj, z[b]);
+        y[u] = 0.0;
       }
-      bwd_record(a.cls[0].BR, np, a.brec, m, j, c)[kBwdG + i] = yj;
-      for (int t = 1; t <= KL; ++t) y[(u + t) % kFwdWin] = fma(-fr[t], yj, y[(u + t) % kFwdWin]);
-      for (int b = 0; b < NBMAX; ++b) z[b] = fma(-fr[1 + KL + b], yj, z[b]);
-      y[u] = 0.0;
     }
+#pragma unroll
     for (int o = 0; o < 4; ++o) tr[kTrPhi + o * 4 + i] = y[o];
+#pragma unroll
     for (int b = 0; b < NBMAX; ++b) tr[kTrGz + b * 4 + i] = z[b];
     return;
   }
-  const int ib = i - 4;
   if (k == P - 1) return;  // the last partition's unknowns need no correction (stored by its backward sweep)
+  const int ib = 4 * (warp - 1) + i;
+  double* HR = a.HR + (((size_t)g * np * 2 + c) * kSolveModes + mm) * kHRec + ib;
   double xw[kBwdWin];
+#pragma unroll
   for (int t = 0; t < kBwdWin; ++t) xw[t] = (t == ib) ? 1.0 : 0.0;
-  for (int j = r1 - 1; j >= r0; --j) {
-    const double* br = bwd_record(a.cls[0].BR, np, a.brec, m, j, c);
-    double acc = 0.0;
-    for (int t = 1; t <= KL + KU; ++t) acc = fma(-br[t], xw[(j + t) % kBwdWin], acc);
-    xw[j % kBwdWin] = acc * br[0];
-    double* hr = a.HR + ((((size_t)g * np + j) * 2 + c) * kSolveModes + mm) * kHRec;
-    hr[ib] = xw[j % kBwdWin];
+  for (int j0 = r1 - kBwdWin; j0 >= r0; j0 -= kBwdWin) {
+#pragma unroll
+    for (int u = kBwdWin - 1; u >= 0; --u) {
+      double br[KL + KU + 2];
+#pragma unroll
+      for (int v = 0; v < (KL + KU + 2) / 2; ++v) {
+        const double2 d = __ldg(reinterpret_cast<const double2*>(BR + (size_t)(j0 + u) * BROW) + v);
+        br[2 * v] = d.x;
+        br[2 * v + 1] = d.y;
+      }
+      double acc = 0.0;
+#pragma unroll
+      for (int t = 1; t <= KL + KU; ++t) acc = fma(-br[t], xw[(u + t) % kBwdWin], acc);
+      xw[u] = acc * br[0];
+      HR[(size_t)(j0 + u) * 2 * kSolveModes * kHRec] = xw[u];
+    }
   }
+#pragma unroll
   for (int o = 0; o < kBwdWin; ++o) tr[kTrPsi + ib * kBwdWin + o] = xw[o];  // Psi^T: row ib
 }
 
@@ -1612,12 +1662,10 @@ void factor_impl(const TauArgs& a, int parts, cudaStream_t st) {
 template <int KL, int KU>
 void transfer_impl(const TauArgs& a, int parts, cudaStream_t st) {
   // one partition: the sweeps need no transfer responses (B1 stores x directly)
-  const int tgx = (a.Nk + 127) / 128;
-  if (parts == kTauParts) k_tau_transfer<KL, KU, kTauParts, 1><<<dim3(tgx, 2 * kTauParts, 16), 128, 0, st>>>(a);
-  if (parts == kTauParts8)
-    k_tau_transfer<KL, KU, kTauParts8, kTau8PerWarp><<<dim3(tgx, 2 * kTauParts8, 16), 128, 0, st>>>(a);
-  if (parts == kTauParts16)
-    k_tau_transfer<KL, KU, kTauParts16, kTau8PerWarp><<<dim3(tgx, 2 * kTauParts16, 16), 128, 0, st>>>(a);
+  const dim3 grid((a.Nk + kSolveModes - 1) / kSolveModes, parts);
+  if (parts == kTauParts) k_tau_transfer<KL, KU, kTauParts, 1><<<grid, 128, 0, st>>>(a);
+  if (parts == kTauParts8) k_tau_transfer<KL, KU, kTauParts8, kTau8PerWarp><<<grid, 128, 0, st>>>(a);
+  if (parts == kTauParts16) k_tau_transfer<KL, KU, kTauParts16, kTau8PerWarp><<<grid, 128, 0, st>>>(a);
 }
 
 template <int P>

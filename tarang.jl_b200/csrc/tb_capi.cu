@@ -186,6 +186,7 @@ ClassDev class_dev(tb_plan* P, int sy, int c, FactorSet* f) {
   cd.c1_nz = T.c1_nz.as<double>();
   cd.col_code = T.col_code.as<int>();
   cd.left_code = T.left_code.as<int>();
+  cd.nonzero = T.nonzero.as<int>();
   if (f) {
     cd.FR = f->FR.as<double>();
     cd.BR = f->BR.as<double>();
@@ -282,6 +283,7 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
   fit(fs->HR, banded ? tau_response_doubles(Nk, (int)n, S.tau_parts) * sizeof(double) : 0);
   const int rows = S.lay.cls[0].n;
   fit(fs->DI, (S.dense ? tau_dense_doubles(Nk, rows) : S.helm ? helm_doubles(Nk, rows) : 0) * sizeof(double));
+  if (S.dense && fs->DI.bytes / 2 > P->dense_work.bytes) P->dense_work.alloc(fs->DI.bytes / 2);
   int neg = 0x7fffffff;
   TB_CUDA_TRY(cudaMemcpyAsync(P->err_mode.p, &neg, sizeof(int), cudaMemcpyHostToDevice, P->st));
   TauArgs a = tau_args(P, sy, fs.get(), nullptr);
@@ -295,8 +297,8 @@ FactorSet* get_factors(tb_plan* P, int sy, double alpha, double beta) {
         ab.cls[c].bord = S.mbord[2 * b + c].as<Coef>();
       }
     launch_tau_factor(ab, S.tau_parts, P->st);
+    if (S.dense) launch_tau_dense(ab, fs->DI.as<double>(), P->dense_work.as<float>(), P->st);
   }
-  if (S.dense) launch_tau_dense(a, fs->DI.as<double>(), P->st);
   if (banded) launch_tau_transfer(a, S.tau_parts, P->st);
   check_launch("tau factor");
   int bad = 0;
@@ -977,7 +979,7 @@ size_t tb::plan_device_bytes(const tb_plan* P) {
   const DevBuf* bufs[] = {&P->X,   &P->X2,  &P->G,   &P->H,    &P->MX0,  &P->Fprev, &P->MXprev, &P->Rsb,
                           &P->bwd, &P->fwd, &P->s3,   &P->twM,  &P->twN,   &P->ptwM,   &P->bEv, &P->bOv,
                           &P->bEd, &P->bOd, &P->fE,   &P->fO,   &P->sfE,   &P->sfO,    &P->err_mode,
-                          &P->solve_scratch, &P->bcdyn,  &P->t_dev};
+                          &P->solve_scratch, &P->dense_work, &P->bcdyn,  &P->t_dev};
   for (const DevBuf* d : bufs) b += d->bytes;
   for (int i = 0; i < 4; ++i) b += P->FP[i].bytes + P->LXP[i].bytes;
   for (int sy = 0; sy < P->nsys; ++sy) {
@@ -986,7 +988,7 @@ size_t tb::plan_device_bytes(const tb_plan* P) {
     for (int c = 0; c < 2; ++c) {
       const ClassTables& t = S.ct[c];
       const DevBuf* tb_[] = {&t.row_eq, &t.row_k, &t.col_unk, &t.col_k, &t.left_unk, &t.left_k, &t.bc_rhs, &t.band,
-                             &t.bord,   &t.c2_z,  &t.c2_nz,   &t.c1_z,  &t.c1_nz,    &t.col_code, &t.left_code};
+                             &t.bord,   &t.c2_z,  &t.c2_nz,   &t.c1_z,  &t.c1_nz,    &t.col_code, &t.left_code, &t.nonzero};
       for (const DevBuf* d : tb_) b += d->bytes;
     }
     for (const auto& f : S.factors) b += f->FR.bytes + f->BR.bytes + f->SI.bytes + f->PP.bytes + f->HR.bytes + f->DI.bytes;
@@ -1133,6 +1135,35 @@ bool default_tau_dense(int Nk, int n) {
   return n + 4 <= kDenseMax && tau_dense_doubles(Nk, n) * sizeof(double) <= (size_t)40 << 20;
 }
 
+// The columns of a class's nonzeros (ClassDev::nonzero), empty where a row or a
+// wall has more than the list's room.
+std::vector<int> nonzero_columns(const ClassLayout& L) {
+  const int n = L.n, w = L.kl + L.ku + 1, nw = dense_wall_entries(n);
+  auto any = [](const Coef& c) { return c.m != 0 || c.l0 != 0 || c.l1 != 0 || c.l2 != 0; };
+  std::vector<int> t(dense_nonzeros(n), -1);
+  for (int r = 0; r < n; ++r) {
+    int k = 0;
+    auto put = [&](int col) {
+      if (k < kDenseNz) t[(size_t)r * kDenseNz + k] = col;
+      ++k;
+    };
+    for (int d = 0; d < w; ++d)
+      if (any(L.band[(size_t)r * w + d])) put(r + d - L.kl);
+    for (int b = 0; b < L.nb; ++b)
+      if (any(L.bord[(size_t)r * L.nb + b])) put(n + b);
+    if (k > kDenseNz) return {};
+  }
+  for (int q = 0; q < L.nb; ++q) {
+    int k = 0;
+    for (int j = 0; j < n; ++j)
+      if (L.c2_z[(size_t)q * n + j] != 0 || L.c2_nz[(size_t)q * n + j] != 0) {
+        if (k == nw) return {};
+        t[(size_t)n * kDenseNz + q * nw + k++] = j;
+      }
+  }
+  return t;
+}
+
 void install_system(tb_plan* P, int sy, TauLayout lay) {
   TauSystem& S = P->sys[sy];
   auto to_int = [](long long v) {
@@ -1162,6 +1193,11 @@ void install_system(tb_plan* P, int sy, TauLayout lay) {
     upload(T.c1_nz, L.c1_nz);
     upload(T.col_code, cc);
     upload(T.left_code, lc);
+    if (sy == 0 && L.n + 4 <= kDenseMax) {
+      const std::vector<int> nz = nonzero_columns(L);
+      TB_REQUIRE(!nz.empty(), TB_ENOTSUPPORTED, "unexpected shape of the tau system");
+      upload(T.nonzero, nz);
+    }
   }
   TB_REQUIRE(lay.cls[0].n == lay.cls[1].n, TB_ENOTSUPPORTED, "parity classes of unequal size");
   const int n = lay.cls[0].n;

@@ -220,6 +220,14 @@ __host__ __device__ inline int tau_part_row0(int np, int P, int k, int ppw = 1) 
 // global scratch (prefetched with the records), so that 16 rings fit one SM.
 constexpr int kTau8PerWarp = 2;
 constexpr int kTauParts16 = 16;
+// Nonzeros of a system, listed for the residuals of its dense inverse (systems
+// with n + 4 <= kDenseMax): kDenseNz entries a band row, the row's columns (band
+// column j < n, border unknown n + b) in ascending order, then -1; then, for each of
+// four boundary rows, dense_wall_entries(n) band columns, then -1.
+constexpr int kDenseMax = 160;
+constexpr int kDenseNz = 10;
+__host__ __device__ constexpr int dense_wall_entries(int n) { return n / 4 + 2; }
+__host__ __device__ constexpr int dense_nonzeros(int n) { return n * kDenseNz + 4 * dense_wall_entries(n); }
 struct ClassDev {
   int n, nb, kl, ku;
   const short* row_eq;
@@ -240,6 +248,7 @@ struct ClassDev {
   // j -> col_code[j], border unknown b -> left_code[b]
   const int* col_code;
   const int* left_code;
+  const int* nonzero;  // the list of dense_nonzeros(n) columns, or null
   // factors, shared by both classes (set on cls[0]):
   //   FR[group][row][class][kSolveModes][kFwdRec], BR[group][row][class][kSolveModes][kBwdRec],
   //   SI[group][class][4][4][kSolveModes]
@@ -302,11 +311,12 @@ size_t helm_doubles(int Nk, int n);
 void launch_helm_factor(const TauArgs& a, double* HF, cudaStream_t st);
 void launch_helm_solve(const TauArgs& a, const double* HF, cudaStream_t st);
 // Dense form of small systems (n + 4 <= kDenseMax): the inverses of all modes
-// from the factor records, and the solve as a product with them.
-constexpr int kDenseMax = 160;
+// from the factor records, one refinement included (W: as many floats of work
+// space; one launch per stacked instance, as launch_tau_factor), and the solve
+// as a product with them.
 int tau_dense_ld(int n);
 size_t tau_dense_doubles(int Nk, int n);
-void launch_tau_dense(const TauArgs& a, double* DI, cudaStream_t st);
+void launch_tau_dense(const TauArgs& a, double* DI, float* W, cudaStream_t st);
 void launch_tau_apply(const TauArgs& a, const double* DI, cudaStream_t st);
 cudaError_t set_tau_smem_limits(int bytes);
 size_t tau_solve_smem_bytes(int npad, int parts);

@@ -92,6 +92,7 @@ void upload(DevBuf& d, const std::vector<T>& h) {
 struct ClassTables {
   DevBuf row_eq, row_k, col_unk, col_k, left_unk, left_k, bc_rhs, band, bord, c2_z, c2_nz, c1_z, c1_nz;
   DevBuf col_code, left_code;  // store targets of the band columns / border unknowns
+  DevBuf nonzero;              // columns of the system's nonzeros (ClassDev::nonzero)
 };
 
 struct FactorSet {
@@ -200,6 +201,7 @@ struct tb_plan {
   int nsys = 1;
   DevBuf err_mode;
   DevBuf solve_scratch;  // y columns of one-partition tau solves (shared by the systems)
+  DevBuf dense_work;     // residuals and corrections while dense inverses are formed
   // dynamic wall values of b (tb_set_wall_values): [bottom value, bottom rate,
   // top value, top rate][mode] on the device, and the time since they were
   // set (advanced on the device at the end of each step, so graphs replay)

@@ -1085,8 +1085,8 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
 // ---------------------------------------------------------------------------
 // Small systems: the solve as one product with the dense inverse.  The banded
 // sweeps are a chain of about 4 n dependent steps, 14 us at n = 64 whatever the
-// partitions, while the inverses of a small grid's modes fit L2 (4.8 MB at
-// 128x32, 38 MB at 256x64) and their product with the right-hand sides is a
+// partitions, while the inverses of a small grid's modes fit L2 (4.6 MB at
+// 128x32, 36 MB at 256x64) and their product with the right-hand sides is a
 // sum over n terms in any order.
 //
 // DI[mode][class][output o][input j], j fastest: inputs are the n band rows and
@@ -1094,77 +1094,233 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
 // (tau_dense_ld(n) entries a row, the spare ones zero).
 // ---------------------------------------------------------------------------
 
-// Column j of the inverse by one thread, (mode, class) by one block: the sweeps
-// of k_tau_solve on a unit right-hand side.  The block's records (n rows) are
-// staged in shared memory first, where every thread reads the same ones; the
-// column's y and x live in DI, written 32 columns a warp.
-constexpr int kDenseRec = kFwdRec + kBwdCode;  // pivot, multipliers; 1 / d, U, border
-template <int KL, int KU>
-__global__ void k_tau_dense(TauArgs a, double* __restrict__ DI, int ld) {
-  extern __shared__ double drec[];  // [row < npad][kDenseRec], identity rows past n
-  const int m = blockIdx.x, c = blockIdx.y, j = threadIdx.x;
-  const int n = a.cls[c].n, np = a.npad, n_out = n + NBMAX;
-  for (int q = threadIdx.x; q < np * kDenseRec; q += blockDim.x) {
-    const int row = q / kDenseRec, t = q - row * kDenseRec;
-    drec[q] = t < kFwdRec ? fwd_record(a.cls[0].FR, np, m, row, c)[t]
-                          : bwd_record(a.cls[0].BR, np, a.brec, m, row, c)[t - kFwdRec];
-  }
-  __syncthreads();
-  if (j >= ld) return;
-  double* col = DI + ((size_t)m * 2 + c) * n_out * ld + j;
-  double y[kFwdWin], z[NBMAX];
+// The (mode, class) systems' inverses, one block each, column j by thread j, to
+// within a rounding or two of the exact inverse, in three launches.  The sweeps
+// of k_tau_solve on a unit right-hand side give a first inverse whose columns
+// err by the condition of the system, each in its own direction, so that a
+// solution made from it errs more than the banded solve of the same system (u_x
+// of ten 512x48 RK222 steps: 4e-14 against 7e-15).  So every column is refined
+// once: its residual is accumulated in pairs of doubles (k_dense_residual) and
+// solved for with the same records.
+//
+// The block's records are staged in shared memory, where every thread reads the
+// same ones; a column's x lives in DI, the residual and the correction's y in W
+// (laid out as DI), both written 32 columns a warp.  The sweeps are bound by the
+// latency of their rows (about two warps an SM sub-partition), so a window's
+// global loads are issued a window ahead of the recurrence, and the products of
+// a backward row run in three chains of which only two links wait for the row
+// below.  The residuals of all rows are independent and take the nonzeros from
+// a list instead of testing the whole band.  W needs a few digits only: FP32,
+// scaled by a power of two to stay in range.  256x64: 46 + 42 + 53 us (the
+// sweeps alone, without these loads ahead, took 74), 128x32 20 + 9 + 22.
+constexpr int kDenseRec = kFwdRec + kBwdCode + 1;  // pivot, multipliers; 1 / d, U, border; one spare (16-byte rows)
+constexpr double kResScale = 1099511627776.0;       // 2^40
+
+// Sum of two doubles and its rounding error.
+__device__ __forceinline__ void two_sum(double& hi, double& err, double a, double b) {
+  hi = a + b;
+  const double t = hi - a;
+  err = (a - (hi - t)) + (b - t);
+}
+// s + c -= a x, the product exact, the sum in two doubles
+__device__ __forceinline__ void sub_product(double& s, double& c, double a, double x) {
+  const double p = a * x, pe = fma(a, x, -p);
+  double e;
+  two_sum(s, e, s, -p);
+  c += e - pe;
+}
+
+// Forward sweep of one column over np rows: row r's right-hand side is rhs(r)
+// (zero from n on), y goes to put(r, y); z: the boundary rows' right-hand
+// sides, on exit the border accumulators.
+template <int KL, class Rhs, class Put>
+__device__ __forceinline__ void dense_forward(const double* drec, int n, int np, double (&z)[NBMAX], Rhs rhs, Put put) {
+  double y[kFwdWin], next[kFwdWin];
 #pragma unroll
-  for (int t = 0; t < kFwdWin; ++t) y[t] = (t == j) ? 1.0 : 0.0;
+  for (int t = 0; t < kFwdWin; ++t) y[t] = rhs(t);
 #pragma unroll
-  for (int b = 0; b < NBMAX; ++b) z[b] = (j == n + b) ? 1.0 : 0.0;
+  for (int t = 0; t < kFwdWin; ++t) next[t] = rhs(t + kFwdWin);
   for (int s = 0; s < np; s += kFwdWin) {
+    double in[kFwdWin];
+#pragma unroll
+    for (int u = 0; u < kFwdWin; ++u) in[u] = next[u];
+#pragma unroll
+    for (int u = 0; u < kFwdWin; ++u) next[u] = rhs(s + u + 2 * kFwdWin);
 #pragma unroll
     for (int u = 0; u < kFwdWin; ++u) {
       const double* fr = drec + (s + u) * kDenseRec;
       const int p = __double2loint(fr[0]);
-      double yj = y[u];
+      const double y0 = y[u];
+      double yj = y0;
+#pragma unroll
+      for (int t = 1; t <= KL; ++t) yj = t == p ? y[(u + t) % kFwdWin] : yj;
 #pragma unroll
       for (int t = 1; t <= KL; ++t) {
-        const bool sw = (t == p);
-        const double yt = y[(u + t) % kFwdWin];
-        y[(u + t) % kFwdWin] = sw ? yj : yt;
-        yj = sw ? yt : yj;
+        const double yt = t == p ? y0 : y[(u + t) % kFwdWin];
+        y[(u + t) % kFwdWin] = fma(-fr[t], yj, yt);
       }
-      if (s + u < n) col[(size_t)(s + u) * ld] = yj;
-#pragma unroll
-      for (int t = 1; t <= KL; ++t) y[(u + t) % kFwdWin] = fma(-fr[t], yj, y[(u + t) % kFwdWin]);
 #pragma unroll
       for (int b = 0; b < NBMAX; ++b) z[b] = fma(-fr[1 + KL + b], yj, z[b]);
-      y[u] = (s + u + kFwdWin == j && j < n) ? 1.0 : 0.0;
+      if (s + u < n) put(s + u, yj);
+      y[u] = in[u];
     }
   }
-  double x1[NBMAX];
-  const double* si = a.cls[0].SI + ((size_t)(m / kSolveModes) * 2 + c) * NBMAX * NBMAX * kSolveModes + m % kSolveModes;
+}
+
+// Border unknowns x1 = SI z, then the backward sweep: y(r) and base(r) in,
+// put(r, x, base) out.
+template <int KL, int KU, class Y, class Base, class Put>
+__device__ __forceinline__ void dense_backward(const double* drec, const double* si, int n, int np,
+                                               const double (&z)[NBMAX], double (&x1)[NBMAX], Y y, Base base, Put put) {
 #pragma unroll
   for (int q = 0; q < NBMAX; ++q) {
     double acc = 0.0;
 #pragma unroll
     for (int b = 0; b < NBMAX; ++b) acc = fma(si[(q * NBMAX + b) * kSolveModes], z[b], acc);
     x1[q] = acc;
-    col[(size_t)(n + q) * ld] = acc;
   }
   double xw[kBwdWin];
 #pragma unroll
   for (int t = 0; t < kBwdWin; ++t) xw[t] = 0.0;
+  using Ty = decltype(y(0));
+  using Tb = decltype(base(0));
+  Ty ynext[kBwdWin];
+  Tb bnext[kBwdWin];
+  auto fetch = [&](int q0) {
+#pragma unroll
+    for (int u = 0; u < kBwdWin; ++u) {
+      const bool in = q0 >= 0 && q0 + u < n;
+      ynext[u] = in ? y(q0 + u) : Ty(0);
+      bnext[u] = in ? base(q0 + u) : Tb(0);
+    }
+  };
+  fetch(np - kBwdWin);
   for (int q0 = np - kBwdWin; q0 >= 0; q0 -= kBwdWin) {
+    Ty yv[kBwdWin];
+    Tb bv[kBwdWin];
+#pragma unroll
+    for (int u = 0; u < kBwdWin; ++u) {
+      yv[u] = ynext[u];
+      bv[u] = bnext[u];
+    }
+    fetch(q0 - kBwdWin);
 #pragma unroll
     for (int u = kBwdWin - 1; u >= 0; --u) {
-      const int row = q0 + u;
-      const double* br = drec + row * kDenseRec + kFwdRec;
-      double acc = row < n ? col[(size_t)row * ld] : 0.0;
+      const double* br = drec + (q0 + u) * kDenseRec + kFwdRec;
+      double a0 = yv[u], a1 = 0.0, a2 = 0.0;
 #pragma unroll
-      for (int b = 0; b < NBMAX; ++b) acc = fma(-br[KL + KU + 1 + b], x1[b], acc);
+      for (int b = 0; b < NBMAX; ++b) a0 = fma(-br[KL + KU + 1 + b], x1[b], a0);
 #pragma unroll
-      for (int t = KL + KU; t >= 1; --t) acc = fma(-br[t], xw[(u + t) % kBwdWin], acc);
-      xw[u] = acc * br[0];
-      if (row < n) col[(size_t)row * ld] = xw[u];
+      for (int t = KL + KU; t >= 8; --t) a1 = fma(-br[t], xw[(u + t) % kBwdWin], a1);
+#pragma unroll
+      for (int t = 7; t >= 3; --t) a2 = fma(-br[t], xw[(u + t) % kBwdWin], a2);
+      a0 += a1 + a2;
+      a0 = fma(-br[2], xw[(u + 2) % kBwdWin], a0);
+      a0 = fma(-br[1], xw[(u + 1) % kBwdWin], a0);
+      xw[u] = a0 * br[0];
+      if (q0 + u < n) put(q0 + u, xw[u], bv[u]);
     }
   }
+}
+
+// REFINE false: the columns from unit right-hand sides; true: the corrections
+// from the residuals in W, added.
+template <int KL, int KU, bool REFINE>
+__global__ void __launch_bounds__(kDenseMax) k_tau_dense(TauArgs a, double* __restrict__ DI, float* __restrict__ W,
+                                                         int ld) {
+  extern __shared__ __align__(16) double drec[];  // [row < np][kDenseRec], identity rows past n
+  const int m = a.mode0 + blockIdx.x, c = blockIdx.y, j = threadIdx.x;
+  const int n = a.cls[c].n, np = (n + kBwdWin - 1) / kBwdWin * kBwdWin;
+  for (int q = threadIdx.x; q < np * (kDenseRec - 1); q += blockDim.x) {
+    const int row = q / (kDenseRec - 1), t = q - row * (kDenseRec - 1);
+    drec[row * kDenseRec + t] = t < kFwdRec ? fwd_record(a.cls[0].FR, a.npad, m, row, c)[t]
+                                            : bwd_record(a.cls[0].BR, a.npad, a.brec, m, row, c)[t - kFwdRec];
+  }
+  __syncthreads();
+  if (j >= ld) return;
+  const size_t sys = ((size_t)m * 2 + c) * (n + NBMAX) * ld + j;
+  double* x = DI + sys;
+  const double* si = a.cls[0].SI + ((size_t)(m / kSolveModes) * 2 + c) * NBMAX * NBMAX * kSolveModes + m % kSolveModes;
+  double z[NBMAX], x1[NBMAX];
+  if constexpr (REFINE) {
+    float* w = W + sys;
+#pragma unroll
+    for (int b = 0; b < NBMAX; ++b) z[b] = w[(size_t)(n + b) * ld];
+    dense_forward<KL>(
+        drec, n, np, z, [&](int r) { return r < n ? (double)w[(size_t)r * ld] : 0.0; },
+        [&](int r, double v) { w[(size_t)r * ld] = (float)v; });
+    dense_backward<KL, KU>(
+        drec, si, n, np, z, x1, [&](int r) { return w[(size_t)r * ld]; }, [&](int r) { return x[(size_t)r * ld]; },
+        [&](int r, double v, double old) { x[(size_t)r * ld] = fma(1.0 / kResScale, v, old); });
+#pragma unroll
+    for (int q = 0; q < NBMAX; ++q) x[(size_t)(n + q) * ld] = fma(1.0 / kResScale, x1[q], x[(size_t)(n + q) * ld]);
+  } else {
+#pragma unroll
+    for (int b = 0; b < NBMAX; ++b) z[b] = (j == n + b) ? 1.0 : 0.0;
+    dense_forward<KL>(
+        drec, n, np, z, [&](int r) { return r == j && r < n ? 1.0 : 0.0; },
+        [&](int r, double v) { x[(size_t)r * ld] = v; });
+    dense_backward<KL, KU>(
+        drec, si, n, np, z, x1, [&](int r) { return x[(size_t)r * ld]; }, [](int) { return 0; },
+        [&](int r, double v, int) { x[(size_t)r * ld] = v; });
+#pragma unroll
+    for (int q = 0; q < NBMAX; ++q) x[(size_t)(n + q) * ld] = x1[q];
+  }
+}
+
+// The residuals of the first inverse's columns: kResRows band rows a block
+// (blockIdx.z), then a boundary row each.  The system's entries are evaluated as
+// k_tau_factor evaluates them.  Half bound by its FP64 operations, ten a product
+// (256x64: 42 us for 0.3 GFMA; one block a system, whose rows wait for one
+// another's loads, 56).
+constexpr int kResRows = 16;
+__global__ void __launch_bounds__(kDenseMax) k_dense_residual(TauArgs a, const double* __restrict__ DI,
+                                                              float* __restrict__ W, int ld) {
+  __shared__ double co[kResRows * kDenseNz];
+  __shared__ int at[kResRows * kDenseNz];  // the entry's unknown in a column; -1: no more in the row
+  static_assert(dense_wall_entries(kDenseMax) <= kResRows * kDenseNz, "a boundary row's entries fit");
+  const int ml = blockIdx.x, m = a.mode0 + ml, c = blockIdx.y, j = threadIdx.x;
+  const ClassDev& C = a.cls[c];
+  const int n = C.n, nb = C.nb, cw = C.kl + C.ku + 1, nw = dense_wall_entries(n);
+  const int chunks = (n + kResRows - 1) / kResRows, r0 = blockIdx.z * kResRows, wall = blockIdx.z - chunks;
+  const double kx = a.kmag ? a.kmag[m] : a.k0 * ml;
+  const int count = wall < 0 ? min(kResRows, n - r0) * kDenseNz : nw;
+  const int* list = C.nonzero + (wall < 0 ? r0 * kDenseNz : n * kDenseNz + wall * nw);
+  for (int q = threadIdx.x; q < count; q += blockDim.x) {
+    const int col = list[q], row = r0 + q / kDenseNz;
+    double v = 0.0;
+    if (col >= 0)
+      v = wall >= 0 ? a.beta * (ml == 0 ? C.c2_z : C.c2_nz)[(size_t)wall * n + col]
+                    : coef_val(col < n ? C.band[(size_t)row * cw + col - row + C.kl] : C.bord[(size_t)row * nb + col - n],
+                               a.alpha, a.beta, kx);
+    co[q] = v;
+    at[q] = col >= 0 ? col * ld : -1;
+  }
+  __syncthreads();
+  if (j >= ld) return;
+  const size_t sys = ((size_t)m * 2 + c) * (n + NBMAX) * ld + j;
+  const double* x = DI + sys;
+  float* w = W + sys;
+  if (wall < 0) {
+    for (int r = 0; r < kResRows && r0 + r < n; ++r) {
+      double s = (j == r0 + r) ? 1.0 : 0.0, e = 0.0;
+#pragma unroll
+      for (int t = 0; t < kDenseNz; ++t) {
+        const int p = at[r * kDenseNz + t];
+        if (p < 0) break;
+        sub_product(s, e, co[r * kDenseNz + t], x[p]);
+      }
+      w[(size_t)(r0 + r) * ld] = (float)(kResScale * (s + e));
+    }
+    return;
+  }
+  double s = (j == n + wall) ? 1.0 : 0.0, e = 0.0;
+  if (wall < nb)
+    for (int q = 0; q < nb; ++q)
+      sub_product(s, e, a.beta * (ml == 0 ? C.c1_z : C.c1_nz)[wall * nb + q], x[(size_t)(n + q) * ld]);
+#pragma unroll 4
+  for (int i = 0; i < nw; ++i) sub_product(s, e, co[i], x[max(at[i], 0)]);
+  w[(size_t)(n + wall) * ld] = (float)(kResScale * (s + e));
 }
 
 // The product, one block per (mode, class): lane l holds the right-hand sides
@@ -1712,7 +1868,8 @@ cudaError_t set_tau_smem_limits(int bytes) {
                        (const void*)k_rk_final<4>,  (const void*)k_rk_final<5>,  (const void*)k_rk_final<6>,
                        (const void*)k_rk_final<7>,  (const void*)k_rk_final<8>,  (const void*)k_rk_final<9>,
                        (const void*)k_rk_final<10>, (const void*)k_rk_final<11>, (const void*)k_rk_final<12>,
-                       (const void*)k_stage_final,  (const void*)k_tau_dense<kTauKL, kTauKU>};
+                       (const void*)k_stage_final,  (const void*)k_tau_dense<kTauKL, kTauKU, false>,
+                       (const void*)k_tau_dense<kTauKL, kTauKU, true>};
   for (const void* fn : fns) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
@@ -1763,10 +1920,13 @@ void launch_helm_solve(const TauArgs& a, const double* HF, cudaStream_t st) {
 int tau_dense_ld(int n) { return (n + NBMAX + 3) / 4 * 4; }
 size_t tau_dense_doubles(int Nk, int n) { return (size_t)Nk * 2 * (n + NBMAX) * tau_dense_ld(n); }
 
-void launch_tau_dense(const TauArgs& a, double* DI, cudaStream_t st) {
-  const int ld = tau_dense_ld(a.cls[0].n);
-  const size_t smem = (size_t)a.npad * kDenseRec * sizeof(double);
-  k_tau_dense<kTauKL, kTauKU><<<dim3(a.Nk, 2), (ld + 31) / 32 * 32, smem, st>>>(a, DI, ld);
+void launch_tau_dense(const TauArgs& a, double* DI, float* W, cudaStream_t st) {
+  const int n = a.cls[0].n, ld = tau_dense_ld(n), threads = (ld + 31) / 32 * 32;
+  const size_t smem = (size_t)((n + kBwdWin - 1) / kBwdWin * kBwdWin) * kDenseRec * sizeof(double);
+  const dim3 grid(a.Nkm, 2);
+  k_tau_dense<kTauKL, kTauKU, false><<<grid, threads, smem, st>>>(a, DI, W, ld);
+  k_dense_residual<<<dim3(a.Nkm, 2, (n + kResRows - 1) / kResRows + NBMAX), threads, 0, st>>>(a, DI, W, ld);
+  k_tau_dense<kTauKL, kTauKU, true><<<grid, threads, smem, st>>>(a, DI, W, ld);
 }
 
 void launch_tau_apply(const TauArgs& a, const double* DI, cudaStream_t st) {

@@ -27,13 +27,14 @@ struct DevBuf {
   void alloc(size_t b) {
     if (p) cudaFree(p);
     p = nullptr;
-    bytes = b;
+    bytes = 0;  // (and stays so where the allocation fails: callers compare it before they allocate)
     if (b == 0) return;
     cudaError_t e = cudaMalloc(&p, b);
     if (e != cudaSuccess) {
       p = nullptr;
       throw Error{TB_ENOMEM, std::string("cudaMalloc(") + std::to_string(b) + "): " + cudaGetErrorString(e)};
     }
+    bytes = b;
   }
   template <class T>
   T* as() const {

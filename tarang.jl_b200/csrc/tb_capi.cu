@@ -919,11 +919,9 @@ static bool xprod2d_form_fits(const tb_plan* P, int form) {
 
 bool tb::plan_tau_parts_ok(const tb_plan* P, int parts) {
   if (parts != 1 && parts != kTauParts && parts != kTauParts8 && parts != kTauParts16) return false;
-  for (int sy = 0; sy < P->nsys; ++sy) {
-    if (tau_solve_smem_bytes(P->sys[sy].npad, parts) > 227 * 1024) return false;
-    if (P->sys[sy].npad / kBwdWin < parts) return false;  // every partition at least one window
-  }
-  return true;
+  // (the 3D program's decoupled component is not partitioned)
+  const int npad = P->sys[0].npad;
+  return tau_solve_smem_bytes(npad, parts) <= 227 * 1024 && npad / kBwdWin >= parts;  // at least one window each
 }
 
 void tb::plan_set_variant(tb_plan* P, int tau_parts, int xrows) {
@@ -1202,13 +1200,15 @@ void install_system(tb_plan* P, int sy, TauLayout lay) {
   TB_REQUIRE(lay.cls[0].n == lay.cls[1].n, TB_ENOTSUPPORTED, "parity classes of unequal size");
   const int n = lay.cls[0].n;
   S.npad = (n + kTauRowPad - 1) / kTauRowPad * kTauRowPad;
-  S.tau_parts = default_tau_parts((P->Nk + kSolveModes - 1) / kSolveModes, S.npad);
   S.helm = sy == 1;
-  S.dense = !S.helm && default_tau_dense(P->Nk, n);
-  TB_REQUIRE(tau_solve_smem_bytes(S.npad, S.tau_parts) <= 227 * 1024, TB_ENOTSUPPORTED,
-             "Nz too large for the staged tau solve");
-  const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, S.tau_parts) * sizeof(double);
-  if (ys > P->solve_scratch.bytes) P->solve_scratch.alloc(ys);
+  if (!S.helm) {
+    S.tau_parts = default_tau_parts((P->Nk + kSolveModes - 1) / kSolveModes, S.npad);
+    S.dense = default_tau_dense(P->Nk, n);
+    TB_REQUIRE(tau_solve_smem_bytes(S.npad, S.tau_parts) <= 227 * 1024, TB_ENOTSUPPORTED,
+               "Nz too large for the staged tau solve");
+    const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, S.tau_parts) * sizeof(double);
+    if (ys > P->solve_scratch.bytes) P->solve_scratch.alloc(ys);
+  }
   // per (band row, class) right-hand-side code, -1 for the padding rows
   std::vector<int> ro((size_t)2 * S.npad, -1);
   for (int j = 0; j < n; ++j)

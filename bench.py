@@ -418,6 +418,8 @@ def run_ours(args, cfg, scheme, dist):
     # then the plan's kernel shapes are tuned on a few steps (state restored)
     if args.tau_parts or args.x_form:
         plan.set_variant(tau_parts=args.tau_parts, xrows=args.x_form)
+        if args.tau_parts and plan.solve_form():
+            plan.set_solve_form(False)  # the partitions asked for, not the dense inverses
     plan.step(cfg.dt, args.warmup)
     tuned = plan.variant() if (args.tau_parts or args.x_form) else plan.tune(cfg.dt, trial_steps=3)
     if args.tensor_cores:

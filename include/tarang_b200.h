@@ -205,6 +205,13 @@ tb_status tb_checkpoint_load(tb_plan* plan, const double* grid, int where, const
  *              3 = batched and in place (decimation in frequency for the
  *              inverse, in time for the forward transforms; half the shared
  *              memory of 2).
+ * The tau systems of small grids (2 Nz + 4 <= 160 rows a parity class, inverses of
+ * all modes up to 40 MB) start in the dense form instead: solved by their
+ * inverses, with tau_parts standing by.  tb_plan_set_solve_form chooses between
+ * the dense form (1; TB_ENOTSUPPORTED for more rows) and the partitions (0).  In
+ * tb_plan_set_variant the value of tau_parts that the plan reports changes
+ * nothing, the form included, so that a plan's variant set on another of its
+ * size gives the same solves; any other value selects the partitioned form.
  * 0 keeps a setting.  A change drops the plan's factors and step graphs; the
  * next step rebuilds them.  tb_plan_tune times trial_steps steps of every
  * feasible combination from the current state (the state is restored after
@@ -212,11 +219,14 @@ tb_status tb_checkpoint_load(tb_plan* plan, const double* grid, int where, const
  * the choice (2D: the in-place x-products wherever they fit).  In 3D it then
  * times at least 10 steps with and without the step's independent kernels
  * (M X, L X, the SBDF history copies) overlapped on a second stream beside the
- * right-hand side and keeps the faster; untuned plans run them in line.  Mixed plans with a tensor-core form of their
+ * right-hand side and keeps the faster; untuned plans run them in line.  Plans
+ * in the dense form stay in it.  Mixed plans with a tensor-core form of their
  * transform GEMMs (tb_plan_set_gemm_path) get the faster GEMM path the same
  * way. */
 tb_status tb_plan_set_variant(tb_plan* plan, int tau_parts, int xrows);
 tb_status tb_plan_get_variant(const tb_plan* plan, int* tau_parts, int* xrows);
+tb_status tb_plan_set_solve_form(tb_plan* plan, int dense);
+tb_status tb_plan_get_solve_form(const tb_plan* plan, int* dense);
 tb_status tb_plan_tune(tb_plan* plan, double dt, int trial_steps, int* tau_parts, int* xrows);
 /* FP32 Chebyshev transform GEMMs of a mixed-precision plan: tensor_cores = 1
  * runs them on the tcgen05 tensor cores in TF32 with three products per term
@@ -309,8 +319,10 @@ tb_status tb_plan_device_bytes(const tb_plan* plan, size_t* bytes);
  * over worker streams.  tb_ensemble_tune times candidate (streams, steps per
  * graph, tau-solve partitions of the members) settings on the members from a
  * snapshot of their state, restores the state and keeps the fastest setting
- * (the partitioning is applied to the member plans: tb_plan_get_variant).  member_ms[i]: time from the run's start
- * until member i finished (device clock); total_ms: the run.
+ * (the partitioning is applied to the member plans: tb_plan_get_variant; members
+ * with small systems keep their dense inverses, tb_plan_get_solve_form, unless
+ * the partitioning is faster for them too).  member_ms[i]: time from the run's
+ * start until member i finished (device clock); total_ms: the run.
  * ---------------------------------------------------------------------- */
 typedef struct tb_ensemble tb_ensemble;
 tb_status tb_ensemble_create(tb_context* ctx, int n, tb_plan* const* members, tb_ensemble** out);

@@ -102,6 +102,8 @@ SIGNATURES = {
     "tb_checkpoint_wait": (c_int, [c_void_p]),
     "tb_checkpoint_load": (c_int, [c_void_p, c_void_p, c_int, c_void_p]),
     "tb_plan_get_variant": (c_int, [c_void_p, POINTER(c_int), POINTER(c_int)]),
+    "tb_plan_set_solve_form": (c_int, [c_void_p, c_int]),
+    "tb_plan_get_solve_form": (c_int, [c_void_p, POINTER(c_int)]),
     "tb_plan_set_gemm_path": (c_int, [c_void_p, c_int]),
     "tb_plan_get_gemm_path": (c_int, [c_void_p, POINTER(c_int)]),
     "tb_plan_tune": (c_int, [c_void_p, c_double, c_int, POINTER(c_int), POINTER(c_int)]),

@@ -379,6 +379,16 @@ class Plan:
     def set_variant(self, tau_parts: int = 0, xrows: int = 0) -> None:
         check(lib.tb_plan_set_variant(self.ptr, int(tau_parts), int(xrows)), self.ctx)
 
+    def set_solve_form(self, dense: bool) -> None:
+        """Small systems: the tau solves by their dense inverses (True, the
+        default where they fit) or partitioned (False)."""
+        check(lib.tb_plan_set_solve_form(self.ptr, 1 if dense else 0), self.ctx)
+
+    def solve_form(self) -> bool:
+        v = c_int()
+        check(lib.tb_plan_get_solve_form(self.ptr, byref(v)), self.ctx)
+        return bool(v.value)
+
     def set_gemm_path(self, tensor_cores: bool) -> None:
         """Mixed precision: FP32 transform GEMMs on the tcgen05 tensor cores
         (True) or on the SIMT FP32 kernel (False).  The default is the SIMT

@@ -924,22 +924,35 @@ bool tb::plan_tau_parts_ok(const tb_plan* P, int parts) {
   return tau_solve_smem_bytes(npad, parts) <= 227 * 1024 && npad / kBwdWin >= parts;  // at least one window each
 }
 
+namespace {
+bool default_tau_dense(int Nk, int n);
+}
+
+bool tb::plan_dense_ok(const tb_plan* P) { return P->sys[0].ct[0].nonzero.p != nullptr; }
+
+bool tb::plan_dense_default(const tb_plan* P) { return default_tau_dense(P->Nk, P->sys[0].lay.cls[0].n); }
+
+// The solves of the coupled systems: tau_parts partitions (0 keeps them), or
+// the dense inverses (tau_parts then stands by).  The 3D program's decoupled
+// component has one form.
+void tb::plan_set_solve(tb_plan* P, int tau_parts, bool dense) {
+  TauSystem& S = P->sys[0];
+  if (tau_parts <= 0) tau_parts = S.tau_parts;
+  TB_REQUIRE(plan_tau_parts_ok(P, tau_parts), TB_ENOTSUPPORTED, "tau solve partitions must be 1, 4, 8 or 16 and fit");
+  TB_REQUIRE(!dense || plan_dense_ok(P), TB_ENOTSUPPORTED, "tau systems too large for their dense inverses");
+  if (S.tau_parts == tau_parts && S.dense == dense) return;
+  TB_CUDA_TRY(cudaStreamSynchronize(P->st));
+  drop_step_graphs(P);
+  S.factors.clear();  // record layouts differ between the forms
+  if (!dense) P->dense_work.alloc(0);
+  S.tau_parts = tau_parts;
+  S.dense = dense;
+  const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, tau_parts) * sizeof(double);
+  if (ys > P->solve_scratch.bytes) P->solve_scratch.alloc(ys);
+}
+
 void tb::plan_set_variant(tb_plan* P, int tau_parts, int xrows) {
-  bool changed = false;
-  if (tau_parts > 0) {
-    TB_REQUIRE(plan_tau_parts_ok(P, tau_parts), TB_ENOTSUPPORTED, "tau solve partitions must be 1, 4, 8 or 16 and fit");
-    for (int sy = 0; sy < P->nsys; ++sy) {
-      TauSystem& S = P->sys[sy];
-      if (S.helm || (S.tau_parts == tau_parts && !S.dense)) continue;
-      TB_CUDA_TRY(cudaStreamSynchronize(P->st));
-      S.tau_parts = tau_parts;
-      S.dense = false;
-      S.factors.clear();  // record layouts differ between the two forms
-      const size_t ys = tau_solve_scratch_doubles(P->Nk, S.npad, tau_parts) * sizeof(double);
-      if (ys > P->solve_scratch.bytes) P->solve_scratch.alloc(ys);
-      changed = true;
-    }
-  }
+  if (tau_parts > 0 && tau_parts != P->sys[0].tau_parts) plan_set_solve(P, tau_parts, false);
   if (xrows > 0 && xrows != P->xrows) {
     if (P->ndim == 3)
       TB_REQUIRE(rbc3d_xrows_ok(P, xrows), TB_ENOTSUPPORTED, "x-pass rows must be 1, 2 or 4 and fit");
@@ -948,9 +961,8 @@ void tb::plan_set_variant(tb_plan* P, int tau_parts, int xrows) {
                  "2D x-products form must be 1 (per field), 2 (batched) or 3 (batched in place) and fit");
     TB_CUDA_TRY(cudaStreamSynchronize(P->st));
     P->xrows = xrows;
-    changed = true;
+    drop_step_graphs(P);
   }
-  if (changed) drop_step_graphs(P);
 }
 
 void tb::plan_prepare(tb_plan* P, double dt, int graph_steps) {
@@ -1779,6 +1791,20 @@ tb_status tb_plan_set_variant(tb_plan* P, int tau_parts, int xrows) {
   });
 }
 
+tb_status tb_plan_set_solve_form(tb_plan* P, int dense) {
+  if (!P) return TB_EINVAL;
+  return guard(P->ctx, [&] {
+    TB_CUDA_TRY(cudaSetDevice(P->ctx->device));
+    plan_set_solve(P, 0, dense != 0);
+  });
+}
+
+tb_status tb_plan_get_solve_form(const tb_plan* P, int* dense) {
+  if (!P || !dense) return TB_EINVAL;
+  *dense = P->sys[0].dense ? 1 : 0;
+  return TB_OK;
+}
+
 tb_status tb_plan_set_gemm_path(tb_plan* P, int tensor_cores) {
   if (!P || (tensor_cores != 0 && tensor_cores != 1)) return TB_EINVAL;
   return guard(P->ctx, [&] {
@@ -1813,7 +1839,7 @@ tb_status tb_plan_tune(tb_plan* P, double dt, int trial_steps, int* tau_parts, i
     PlanSnapshot snap;
     plan_snapshot(P, &snap);
     std::vector<int> parts_c, rows_c;
-    // (systems solved by their inverses stay so: 0 keeps them)
+    // (systems solved by their inverses stay so)
     for (int p : {kTauParts16, kTauParts8, kTauParts, 1})
       if (!P->sys[0].dense && plan_tau_parts_ok(P, p)) parts_c.push_back(p);
     if (parts_c.empty()) parts_c.push_back(0);
@@ -1846,7 +1872,7 @@ tb_status tb_plan_tune(tb_plan* P, double dt, int trial_steps, int* tau_parts, i
           br = rc;
         }
       }
-    plan_set_variant(P, P->sys[0].dense ? 0 : bp, br);
+    plan_set_variant(P, bp, br);
     // then, in 3D, the side stream on or off, on a longer trial (the difference
     // is a few percent)
     const int ov_steps = std::max(trial_steps, 10);

@@ -337,7 +337,9 @@ tb_status tb_ensemble_tune(tb_ensemble* E, const double* dt, int trial_steps, in
     };
     // tau-solve partitioning of the members: the partitioned solve has the
     // shortest latency for one plan, the one-warp solve the least work when
-    // many plans share the GPU; both are tried when every member can run them
+    // many plans share the GPU; both are tried when every member can run them.
+    // Plans whose systems are small keep their dense inverses meanwhile, which
+    // are weighed against the partitionings once the rest is chosen.
     // forms: per member, and fused (same-shape members stacked) when some
     // shape has two or more fusible members
     std::vector<bool> cand_f = {false};
@@ -352,20 +354,33 @@ tb_status tb_ensemble_tune(tb_ensemble* E, const double* dt, int trial_steps, in
     float best = 1e30f;
     int bs = E->streams, bg = E->graph_steps, bp = E->members[0]->sys[0].tau_parts;
     bool bf = E->fused;
+    auto shaped = [&](bool fz) {
+      std::vector<tb_plan*> v(E->members.begin(), E->members.end());
+      if (fz)
+        for (auto& G : E->groups) v.push_back(G.plan.get());
+      return v;
+    };
+    auto partitionings = [](const std::vector<tb_plan*>& plans) {
+      std::vector<int> c;
+      for (int pc : {kTauParts8, kTauParts, 1}) {
+        bool ok = true;
+        for (auto* m : plans) ok = ok && plan_tau_parts_ok(m, pc);
+        if (ok) c.push_back(pc);
+      }
+      return c;
+    };
+    auto set_solves = [](const std::vector<tb_plan*>& plans, int pc, bool dense) {
+      for (auto* m : plans) plan_set_solve(m, pc, dense && plan_dense_default(m));
+    };
     for (bool fz : cand_f) {
       E->fused = fz;
       if (fz) build_groups(E);
-      std::vector<tb_plan*> shaped(E->members.begin(), E->members.end());
-      if (fz)
-        for (auto& G : E->groups) shaped.push_back(G.plan.get());
-      std::vector<int> cand_p;
-      for (int pc : {kTauParts8, kTauParts, 1}) {
-        bool ok = true;
-        for (auto* m : shaped) ok = ok && plan_tau_parts_ok(m, pc);
-        if (ok) cand_p.push_back(pc);
-      }
+      const std::vector<tb_plan*> plans = shaped(fz);
+      const bool banded = std::any_of(plans.begin(), plans.end(), [](tb_plan* m) { return !plan_dense_default(m); });
+      std::vector<int> cand_p = partitionings(plans);
+      if (!banded && cand_p.size() > 1) cand_p.resize(1);  // none in use yet
       for (int pc : cand_p) {
-        for (auto* m : shaped) plan_set_variant(m, pc, 0);
+        set_solves(plans, pc, true);
         // warm-up: factors and graphs of every member / group at this dt
         run(E, dt, std::min(trial_steps, 2), std::min(n, 8), 1, nullptr, nullptr);
         restore();
@@ -390,17 +405,34 @@ tb_status tb_ensemble_tune(tb_ensemble* E, const double* dt, int trial_steps, in
       }
     }
     E->fused = bf;
-    for (auto* m : E->members) plan_set_variant(m, bp, 0);
-    if (bf)
-      for (auto& G : E->groups) plan_set_variant(G.plan.get(), bp, 0);
+    const std::vector<tb_plan*> all = shaped(bf);
+    const std::vector<int> cand_p = partitionings(all);
+    if (!cand_p.empty()) {
+      // (0: the dense inverses where a new plan has them, bp elsewhere) against
+      // every system partitioned alike, best of two alternating trials each
+      std::vector<int> form = {0};
+      if (std::any_of(all.begin(), all.end(), [](tb_plan* m) { return plan_dense_default(m); }))
+        form.insert(form.end(), cand_p.begin(), cand_p.end());
+      std::vector<float> ms(form.size(), 1e30f);
+      for (int t = 0; t < 2 && form.size() > 1; ++t)
+        for (size_t f = 0; f < form.size(); ++f) {
+          set_solves(all, form[f] ? form[f] : bp, form[f] == 0);
+          run(E, dt, trial_steps, bs, bg, nullptr, nullptr);  // factors and graphs of this form
+          restore();
+          float tot = 0.f;
+          run(E, dt, trial_steps, bs, bg, nullptr, &tot);
+          restore();
+          ms[f] = std::min(ms[f], tot);
+        }
+      const int f = form[std::min_element(ms.begin(), ms.end()) - ms.begin()];
+      if (f) bp = f;
+      set_solves(all, bp, f == 0);
+    }
     E->streams = bs;
     E->graph_steps = bg;
     // mixed members with a tensor-core form of their transform GEMMs: that
     // form or the SIMT kernel, timed on the chosen configuration (best of two
     // alternating trials each)
-    std::vector<tb_plan*> all(E->members.begin(), E->members.end());
-    if (bf)
-      for (auto& G : E->groups) all.push_back(G.plan.get());
     bool any_tc = false;
     for (auto* m : all) any_tc = any_tc || (m->mixed && (m->tc2img.p != nullptr || m->tc3));
     if (any_tc) {

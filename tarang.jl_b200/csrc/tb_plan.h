@@ -351,6 +351,9 @@ bool rbc3d_xrows_ok(const tb_plan* P, int rows);
 // drops the plan's factors and step graphs (rebuilt on the next step).
 bool plan_tau_parts_ok(const tb_plan* P, int parts);
 void plan_set_variant(tb_plan* P, int tau_parts, int xrows);
+bool plan_dense_ok(const tb_plan* P);       // the systems have a dense form
+bool plan_dense_default(const tb_plan* P);  // and a new plan takes it
+void plan_set_solve(tb_plan* P, int tau_parts, bool dense);
 void rbc3d_lx_project(tb_plan* P, double2* LX, double beta, cudaStream_t st = nullptr);  // null: the plan's stream
 void rbc3d_mx_project(tb_plan* P, double2* MX, cudaStream_t st = nullptr);
 size_t rbc3d_device_bytes(const tb_plan* P);

@@ -228,7 +228,7 @@ std::unique_ptr<Job> make_cohort_job(tb_context* ctx, const std::vector<Request*
   j->P = std::make_unique<tb_plan>();
   build_plan(j->P.get(), ctx, descs.data(), (int)descs.size());
   tb_plan* P = j->P.get();
-  if (plan_tau_parts_ok(P, 1)) plan_set_variant(P, 1, 0);  // the one-warp solve, as for single requests
+  if (plan_tau_parts_ok(P, 1)) plan_set_solve(P, 1, false);  // the one-warp solve, as for single requests
   StreamBuf grid;
   grid.alloc((size_t)P->Nz * P->Nx * sizeof(double), P->st);
   TB_CUDA_TRY(cudaMemsetAsync(P->X.p, 0, P->X.bytes, P->st));
@@ -265,7 +265,7 @@ std::unique_ptr<Job> make_job(tb_context* ctx, const Request& r) {
   // form: its blocks need a fifth of the shared memory of the partitioned
   // form's, so several requests' solves share an SM instead of queueing for
   // whole SMs (the throughput choice the ensemble tuner also makes).
-  if (plan_tau_parts_ok(P, 1)) plan_set_variant(P, 1, 0);
+  if (plan_tau_parts_ok(P, 1)) plan_set_solve(P, 1, false);
   // initial state: b from the grid field, u = 0
   StreamBuf grid, coeff;  // staging released in stream order: no device-wide wait
   grid.alloc(r.init.size() * sizeof(double), P->st);

@@ -487,11 +487,8 @@ void enqueue_rk_step(tb_turb* T, double dt) {
     if (!T->f_used[i]) {  // no weight anywhere: the next combination stands alone
       launch_combine(T, combination(i + 1, &w));
     } else {
-      // F_i is kept only where a combination after the next one reads it
-      bool later = i + 1 < s && std::fabs(T->bE[i]) > 1e-14;
-      for (int k = i + 2; k < s; ++k) later = later || std::fabs(T->AE[k][i]) > 1e-14;
       const TurbComb c = combination(i + 1, &w);
-      enqueue_rhs(T, Y[i], nullptr, later ? T->Fs[i].as<float2>() : nullptr, dt, 2, c, w);
+      enqueue_rhs(T, Y[i], nullptr, T->Fs[i].as<float2>(), dt, 2, c, w);  // (null: not kept)
     }
     if (i + 1 < s) Y[i + 1] = T->Ys[i + 1].as<float2>();
   }
@@ -536,7 +533,7 @@ cudaGraphExec_t capture(tb_turb* T, double dt) {
 size_t tb::turb_estimate_bytes(int Nx, int Ny, int timestepper) {
   const size_t Kx = Nx / 2 + 1, Kp = (Kx + 3) / 4 * 4, My = padded_len(Ny);
   // SBDF2: q_n, q_{n-1}, F_{n-1}; RK: q_n, q_{n+1} and up to 3 stage states
-  // and 3 stage right-hand sides (4 stages, the first state and RHS not kept)
+  // and 3 stage right-hand sides (4 stages, the first state and the last RHS not kept)
   const size_t specs = timestepper == TB_SBDF2 ? 3 : (timestepper == TB_RK222 ? 6 : 8);
   return sizeof(float2) * (specs * Kx * Ny + 5 * Kp * My) + (4u << 20);
 }
@@ -588,8 +585,12 @@ tb_turb* tb::turb_create(tb_context* ctx, const tb_problem_desc& d, const double
   for (auto& b : T->Q) b.alloc(spec);
   if (T->rk) {
     for (int i = 1; i < T->stages; ++i) T->Ys[i].alloc(spec);
-    for (int i = 0; i < T->stages; ++i)
-      if (T->f_used[i]) T->Fs[i].alloc(spec);
+    // F_i is kept only where a combination after the next one reads it
+    for (int i = 0; i < T->stages; ++i) {
+      bool later = i + 1 < T->stages && std::fabs(T->bE[i]) > 1e-14;
+      for (int k = i + 2; k < T->stages; ++k) later = later || std::fabs(T->AE[k][i]) > 1e-14;
+      if (later) T->Fs[i].alloc(spec);
+    }
   } else {
     T->Fb.alloc(spec);
   }

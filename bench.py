@@ -468,10 +468,12 @@ def run_ours(args, cfg, scheme, dist):
     # DRAM traffic per launch (average over a step's launches of each kernel
     # name) from the committed ncu capture of this workload
     tpath = os.path.join(ROOT, "profiles", f"traffic_{cfg.Nx}x{cfg.Nz}_{scheme.lower()}.json")
-    tr = {}
+    tr, tr_launches = {}, 0
     if os.path.exists(tpath):
         with open(tpath) as f:
-            tr = {k: v for k, v in json.load(f).items() if not k.startswith("_")}
+            cap = json.load(f)
+        tr = {k: v for k, v in cap.items() if not k.startswith("_")}
+        tr_launches = cap.get("_launches_per_step", 0)
     if roof is not None and top in tr:
         roof["traffic"] = tr[top]
         roof["traffic_source"] = tpath.replace(ROOT + os.sep, "")
@@ -480,7 +482,7 @@ def run_ours(args, cfg, scheme, dist):
     step_roof = {"bytes_per_step_model": model, "achieved_gbs": model / step_s / 1e9,
                  "peak_gbs": peaks.get("hbm_gbs")}
     step_roof["frac"] = step_roof["achieved_gbs"] / step_roof["peak_gbs"]
-    if tr and all(k in tr for k in prof):
+    if set(tr) == set(prof) and tr_launches * nprof == sum(v[1] for v in prof.values()):
         # what the step really moves: measured DRAM bytes of every kernel
         # launch of one step (ncu), over the device time of a step
         meas = sum(tr[k] * prof[k][1] / nprof for k in prof)

@@ -206,7 +206,7 @@ tb_status tb_checkpoint_load(tb_plan* plan, const double* grid, int where, const
  *              inverse, in time for the forward transforms; half the shared
  *              memory of 2).
  * The tau systems of small grids (2 Nz + 4 <= 160 rows a parity class, inverses of
- * all modes up to 40 MB) start in the dense form instead: solved by their
+ * all modes up to 40 MiB) start in the dense form instead: solved by their
  * inverses, with tau_parts standing by.  tb_plan_set_solve_form chooses between
  * the dense form (1; TB_ENOTSUPPORTED for more rows) and the partitions (0).  In
  * tb_plan_set_variant the value of tau_parts that the plan reports changes

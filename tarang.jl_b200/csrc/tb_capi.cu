@@ -1138,8 +1138,8 @@ int default_tau_parts(int groups, int npad) {
 
 // Whether the systems are solved by their dense inverses: those of all modes
 // have to stay in L2 beside the step's planes.  One solve, event-timed, dense
-// against the best partitioning: 96x24 (2 MB) 8.7 against 16.0 us, 256x64 (34 MB)
-// 14.2 against 22.6, 192x76 (36 MB) 14.8 against 25.0, 512x48 (39 MB) 17.8 against
+// against the best partitioning: 96x24 (2 MiB) 8.7 against 16.0 us, 256x64 (34 MiB)
+// 14.2 against 22.6, 192x76 (36 MiB) 14.8 against 25.0, 512x48 (39 MiB) 17.8 against
 // 19.8.
 bool default_tau_dense(int Nk, int n) {
   return n + 4 <= kDenseMax && tau_dense_doubles(Nk, n) * sizeof(double) <= (size_t)40 << 20;

@@ -12,8 +12,9 @@
 // kernel take the last inverse pass, the product and the first forward pass
 // in registers (no shared-memory round trip between them).
 //
-// Why these radices: the transforms are bound by shared-memory traffic and by
-// the barrier and latency of each pass, and both go with the number of passes.
+// Why these radices: the transforms are bound by the instructions, the barrier
+// and the shared-memory round trip of each pass (no unit is above 65 % of its
+// peak), and all go with the number of passes.
 // 1536 points are 3 passes of 12, 16 and 8 here, where radices of at most 8
 // take 4.  make_rplan picks the sequence with the fewest shared-memory
 // wavefronts (bank conflicts counted), plus a fixed charge per pass.
@@ -247,7 +248,9 @@ __device__ __forceinline__ void pass_any(C* buf, int NA, int Ms, const RPlan& p,
 // arrays, the last inverse pass with the products and the first forward pass
 // in registers, dit passes over the two product arrays, truncation.
 //
-// Bound by shared-memory traffic and pass latency.  Against the radix-8 form
+// Bound by the latency of the passes (1024x256 FP64: 16 warps an SM, a third of
+// the issue slots and of the shared-memory peak; barriers and loads first among
+// the waits).  Against the radix-8 form
 // of the same transforms (4 + 4 passes and a product sweep between them) the
 // 1536-point row makes 36 instead of 60 shared-memory accesses an entry.
 // Args: XProdArgs-like (ev, ov, ed, od, out, iptw, rp, Nx, Nk, M, Nz, k0, ld,

@@ -100,7 +100,9 @@ __host__ __device__ inline int ystride(int My) {
 // odd values, 2 even d_z, 3 odd d_z, element (j, m).  Output mix[z][q][y][kx],
 // q = 3 f + kind (value, d_y, d_z).  The 6 CW transforms (both levels) share the
 // passes; rows leave in groups of CW neighbours (32 bytes at the widest), so
-// the x pass reads whole rows.  Bound by shared-memory traffic.
+// the x pass reads whole rows.  Bound by instruction issue (64 % of the slots at
+// 128x128x64 FP32; shared-memory wavefronts 48 % of their peak, a fifth of them
+// bank conflicts).
 template <class C, int CW>
 __global__ void __launch_bounds__(kR3Threads, sizeof(C) == 8 ? 3 : 2)
     k3_yinv(R3Args a, const C* __restrict__ G, const C* __restrict__ twy, const unsigned short* __restrict__ posy,
@@ -236,9 +238,11 @@ __device__ __forceinline__ void xmiddle3(C* __restrict__ A, int Ms, int n) {
 // Per (RR consecutive padded y rows, z level).  mix[z][q][y][kx] ->
 // pm[z][f][y][kx] (f = b, u_x, u_y, u_z; kx < Kx, Nyquist folded): the packed
 // spectra of the 15 factors straight from the rows, dif passes over 8 RR
-// arrays in one buffer, xmiddle3, dit passes over 2 RR arrays.  Bound by
-// shared-memory traffic; at 384 points an entry makes 5 accesses a factor
-// where the two-buffer Stockham form with staged spectra made 9.
+// arrays in one buffer, xmiddle3, dit passes over 2 RR arrays.  Bound by issue
+// and shared memory together (64 % of the issue slots, wavefronts 57 % of their
+// peak at 128x128x64 FP32, barriers first among the waits); at 384 points an
+// entry makes 5 shared-memory accesses a factor where the two-buffer Stockham
+// form with staged spectra made 9.
 template <class C, int RR>
 __global__ void __launch_bounds__(kR3Threads, sizeof(C) == 8 ? 3 : 2)
     k3_xpass(R3Args a, const C* __restrict__ mix, const C* __restrict__ twx, C* __restrict__ pm) {

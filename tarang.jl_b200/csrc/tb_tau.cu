@@ -1085,8 +1085,8 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
 // ---------------------------------------------------------------------------
 // Small systems: the solve as one product with the dense inverse.  The banded
 // sweeps are a chain of about 4 n dependent steps, 14 us at n = 64 whatever the
-// partitions, while the inverses of a small grid's modes fit L2 (4.6 MB at
-// 128x32, 36 MB at 256x64) and their product with the right-hand sides is a
+// partitions, while the inverses of a small grid's modes fit L2 (4.6 MiB at
+// 128x32, 34 MiB at 256x64) and their product with the right-hand sides is a
 // sum over n terms in any order.
 //
 // DI[mode][class][output o][input j], j fastest: inputs are the n band rows and

@@ -789,8 +789,8 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1) k_xprod_b(XProdArgs a) 
 
 // rfft of real rows (unnormalised), two rows to a complex FFT: rows 2 i and 2 i + 1
 // as real and imaginary part, the spectra separated by conjugate symmetry.  The
-// kernel is bound by the passes' shared-memory round trips, so half the
-// transforms are half the work.  Pairs stay inside a field (blockIdx.y, nrows
+// kernel is a chain of passes, each a shared-memory round trip and a barrier, so
+// half the transforms are half the work.  Pairs stay inside a field (blockIdx.y, nrows
 // rows each), whose rows the other transforms mix anyway: one field's size and
 // infinities do not reach another's coefficients.  An odd last row goes with
 // zeros.

@@ -140,7 +140,9 @@ __host__ __device__ inline int ystride(int My) { return Rp::rpad<float2>(My) + 4
 // grid round trip's projection, the x Nyquist split and the y padding, inverse
 // FFT along y; out: mix[f][y][kx].  The columns of a group share the passes'
 // barriers and their rows are stored together (32 bytes at CW = 4), which
-// replaces a separate transpose: bound by shared-memory traffic.
+// replaces a separate transpose.  At 1024x1024 bound by issue and latency (58 %
+// of the issue slots, shared-memory wavefronts 25 % of their peak; most waits
+// are for global loads).
 template <int CW, int BL>
 __global__ void __launch_bounds__(kTurbThreads, BL) k_turb_yinv(TurbArgs a, const float2* __restrict__ q,
                                                                float2* __restrict__ mix) {

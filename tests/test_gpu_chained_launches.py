@@ -31,7 +31,7 @@ def test_chained_steps_match_separated_kernels(tb, Nx, Nz, ts, precision):
         assert np.isfinite(a).all() and np.array_equal(a, b)
 
 
-# 442, 444 and 446 blocks of the row transforms (two rows a block)
+# 444 and 448 blocks of the row transforms (two rows of a field a block, four fields)
 @pytest.mark.parametrize("Nz", [221, 222, 223])
 def test_field_transforms_around_the_limit(tb, Nz):
     import torch

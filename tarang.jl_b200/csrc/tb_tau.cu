@@ -1111,7 +1111,8 @@ __global__ void __launch_bounds__(128) k_tau_transfer(TauArgs a) {
 // a backward row run in three chains of which only two links wait for the row
 // below.  The residuals of all rows are independent and take the nonzeros from
 // a list instead of testing the whole band.  W needs a few digits only: FP32,
-// scaled by a power of two to stay in range.  256x64: 46 + 42 + 53 us (the
+// scaled by a power of two (its entries are in units of the right-hand side,
+// roundings of 1, so they stay in range whatever the system's scale).  256x64: 46 + 42 + 53 us (the
 // sweeps alone, without these loads ahead, took 74), 128x32 20 + 9 + 22.
 constexpr int kDenseRec = kFwdRec + kBwdCode + 1;  // pivot, multipliers; 1 / d, U, border; one spare (16-byte rows)
 constexpr double kResScale = 1099511627776.0;       // 2^40
